@@ -587,9 +587,6 @@ __global__ void k_dot_final(const double *partial, int nb, double *out) {
     }
 }
 
-// residuals of one component, LNORM=2, VELOCITY=0 (src/calc_res.c:137-281):
-// per trace, running float sums times DT, time-reversed difference; the
-// misfit and energy partial sums per trace in double
 // The time window of src/time_window.c:135-210 on one sample: v at 1-based
 // sample j (j >= 2) of trace i, picks [np][ntr]; returns the windowed value
 // and the taper bits (1/2 late/early of the first window, 4/8 of the second).
@@ -654,37 +651,103 @@ struct KWindow {
     int tw_ind;
     float gamma, twl_plus, twl_minus;
 };
-__global__ void k_calc_res(const float *obs, const float *syn, float *diff, int ntr, int ns, float dt,
-                           double *l2_tr, double *en_tr, const int *kill = nullptr, KWindow win = KWindow{}) {
-    const int tr = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tr >= ntr) return;
-    if (kill && kill[tr]) {  // a killed trace keeps a zero residual and adds nothing (src/calc_res.c:196-197)
-        l2_tr[tr] = 0.0;
-        en_tr[tr] = 0.0;
-        return;
-    }
-    const float *s = syn + (long long)tr * ns, *d = obs + (long long)tr * ns;
-    float *df = diff + (long long)tr * ns;
+// Residuals, LNORM=2, VELOCITY=0 (src/calc_res.c:137-281): per trace, running
+// float sums times DT, time-reversed difference; the misfit and energy
+// partial sums per trace in double.
+// One residual launch: traces of up to three components of every slot.  A
+// slot's component k reads obs + slot * obs_slot + k * comp and syn + slot *
+// syn_slot + plane[k] * comp, writes diff + slot * obs_slot + k * comp and
+// the trace sums at tr + (slot * 3 + k) * 2 * mr (misfit, then energy).
+struct KRes {
+    const float *obs, *syn;
+    float *diff;
+    double *tr;
+    long long obs_slot, syn_slot, comp;
+    int plane[3];     // seismogram plane of component k (-1: unused)
+    int first;        // component of blockIdx.y == 0
+    const int *ntr;   // traces of every slot (NULL: mr)
+    int mr, ns;
+    float dt;
+    const int *kill;  // slot * mr (NULL: none)
+    KWindow win;      // picks of slot 0
+    long long win_slot;
+};
+// A warp takes 32 traces, one per lane: the running sums are sequential in a
+// trace (the reference's float order), so a trace is one dependence chain and
+// the kernel is bound by it.  The samples pass through shared memory in 32 x
+// 32 blocks, so that the loads and the reversed stores run along the traces
+// (one 128-byte line each) and the next block is in flight while this one is
+// summed.  All traces, components and slots go in one launch: 2000 samples
+// of 100 traces and two components took 1.1 ms as one thread per trace with
+// strided loads and one launch per slot and component.
+__global__ void __launch_bounds__(32) k_calc_res(KRes a) {
+    constexpr int B = 32;
+    __shared__ float ts[B][B + 1], td[B][B + 1];
+    const int lane = threadIdx.x, slot = blockIdx.z, k = a.first + blockIdx.y, t0 = blockIdx.x * B;
+    const int ntr = a.ntr ? a.ntr[slot] : a.mr;
+    if (a.plane[k] < 0 || t0 >= ntr) return;
+    const int nt = min(B, ntr - t0), tr = t0 + lane;
+    const float *s = a.syn + slot * a.syn_slot + a.plane[k] * a.comp + (long long)t0 * a.ns;
+    const float *d = a.obs + slot * a.obs_slot + k * a.comp + (long long)t0 * a.ns;
+    float *df = a.diff + slot * a.obs_slot + k * a.comp + (long long)t0 * a.ns;
+    KWindow win = a.win;
+    if (win.picks) win.picks += slot * a.win_slot;
+    // a killed trace keeps a zero residual and adds nothing (src/calc_res.c:196-197)
+    const bool mine = lane < nt && !(a.kill && a.kill[(long long)slot * a.mr + tr]);
+    const unsigned live = __ballot_sync(0xffffffffu, mine);
+    float vs[B], vd[B];
+    auto load = [&](int j0) {
+        const int j = j0 + lane;
+#pragma unroll
+        for (int r = 0; r < B; r++) {
+            const bool ok = r < nt && j < a.ns;
+            vs[r] = ok ? s[(long long)r * a.ns + j] : 0.0f;
+            vd[r] = ok ? d[(long long)r * a.ns + j] : 0.0f;
+        }
+    };
     float rs = 0.0f, rd = 0.0f;
     double l2 = 0.0, en = 0.0;
-    for (int j = 0; j < ns; j++) {
-        rs += s[j];
-        rd += d[j];
-        float is = rs * dt, id = rd * dt;
-        if (win.picks && j >= 1) {  // windowed after the integration (src/calc_res.c:157-160)
-            unsigned char m;
-            is = tw_sample(is, j + 1, tr, win.stride, win.tw_ind, win.picks, dt, win.gamma, win.twl_plus,
-                           win.twl_minus, m);
-            id = tw_sample(id, j + 1, tr, win.stride, win.tw_ind, win.picks, dt, win.gamma, win.twl_plus,
-                           win.twl_minus, m);
+    load(0);
+    for (int j0 = 0; j0 < a.ns; j0 += B) {
+#pragma unroll
+        for (int r = 0; r < B; r++) {
+            ts[r][lane] = vs[r];
+            td[r][lane] = vd[r];
         }
-        const float r = is - id;
-        df[ns - 1 - j] = r;
-        l2 += (double)r * (double)r;
-        en += (double)id * (double)id;
+        __syncwarp();
+        if (j0 + B < a.ns) load(j0 + B);
+        const int nj = min(B, a.ns - j0);
+        if (mine) {
+#pragma unroll 4
+            for (int jj = 0; jj < nj; jj++) {
+                rs += ts[lane][jj];
+                rd += td[lane][jj];
+                float is = rs * a.dt, id = rd * a.dt;
+                const int j = j0 + jj;
+                if (win.picks && j >= 1) {  // windowed after the integration (src/calc_res.c:157-160)
+                    unsigned char m;
+                    is = tw_sample(is, j + 1, tr, win.stride, win.tw_ind, win.picks, a.dt, win.gamma, win.twl_plus,
+                                   win.twl_minus, m);
+                    id = tw_sample(id, j + 1, tr, win.stride, win.tw_ind, win.picks, a.dt, win.gamma, win.twl_plus,
+                                   win.twl_minus, m);
+                }
+                const float r = is - id;
+                ts[lane][jj] = r;
+                l2 += (double)r * (double)r;
+                en += (double)id * (double)id;
+            }
+        }
+        __syncwarp();
+        if (lane < nj)
+            for (int r = 0; r < nt; r++)
+                if ((live >> r) & 1) df[(long long)r * a.ns + a.ns - 1 - (j0 + lane)] = ts[r][lane];
+        __syncwarp();
     }
-    l2_tr[tr] = l2;
-    en_tr[tr] = en;
+    if (lane < nt) {
+        double *o = a.tr + ((long long)slot * 3 + k) * 2 * a.mr + tr;
+        o[0] = l2;
+        o[a.mr] = en;
+    }
 }
 
 // Offset-based trace kill (src/create_trkill_table.c:35-46): killtable[r][s]

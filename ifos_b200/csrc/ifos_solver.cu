@@ -1397,7 +1397,16 @@ extern "C" int ifos_calc_res(ifos_ctx *c, int ntr, const float *obs, const float
     float *d_obs = (float *)((char *)scr + tb), *d_syn = d_obs + (size_t)ntr * ns, *d_diff = d_syn + (size_t)ntr * ns;
     CK(cudaMemcpyAsync(d_obs, obs, bytes, cudaMemcpyHostToDevice, c->st));
     CK(cudaMemcpyAsync(d_syn, syn, bytes, cudaMemcpyHostToDevice, c->st));
-    k_calc_res<<<(ntr + 127) / 128, 128, 0, c->st>>>(d_obs, d_syn, d_diff, ntr, ns, c->p.dt, tr, tr + ntr);
+    KRes kr{};
+    kr.obs = d_obs;
+    kr.syn = d_syn;
+    kr.diff = d_diff;
+    kr.tr = tr;
+    kr.mr = ntr;
+    kr.ns = ns;
+    kr.dt = c->p.dt;
+    kr.plane[1] = kr.plane[2] = -1;
+    k_calc_res<<<dim3((ntr + 31) / 32, 1, 1), 32, 0, c->st>>>(kr);
     c->launches++;
     std::vector<double> h((size_t)2 * ntr);
     if (diff) CK(cudaMemcpyAsync(diff, d_diff, bytes, cudaMemcpyDeviceToHost, c->st));
@@ -1450,35 +1459,50 @@ extern "C" int ifos_residual_adjoint(ifos_ctx *c, int nshots, const float *obs, 
     int *d_kill = kill ? (int *)((char *)scr + tb) : nullptr;
     float *d_picks = win ? (float *)((char *)scr + tb + kb) : nullptr;
     float *d_obs = (float *)((char *)scr + tb + kb + pb);
-    CK(cudaMemcpyAsync(d_obs, obs, obs_bytes, cudaMemcpyHostToDevice, c->st));
+    // the observed components in use lie between k0 and k1: the others are not copied
+    int k0 = 3, k1 = -1;
+    for (int k = 0; k < 3; k++)
+        if (plane[k] >= 0) {
+            k0 = std::min(k0, k);
+            k1 = k;
+        }
+    for (int s = 0; s < nshots && k1 >= k0; s++) {
+        const size_t o = ((size_t)s * 3 + k0) * comp;
+        CK(cudaMemcpyAsync(d_obs + o, obs + o, (k1 - k0 + 1) * comp * 4, cudaMemcpyHostToDevice, c->st));
+    }
     if (kill) CK(cudaMemcpyAsync(d_kill, kill, (size_t)nshots * mr * sizeof(int), cudaMemcpyHostToDevice, c->st));
     if (win)
         CK(cudaMemcpyAsync(d_picks, win->picks, (size_t)nshots * np * mr * sizeof(float), cudaMemcpyHostToDevice,
                            c->st));
     CK(cudaMemsetAsync(c->adj.p, 0, obs_bytes, c->st));
     CK(cudaMemsetAsync(tr, 0, tb, c->st));
-    for (int s = 0; s < nshots; s++) {
-        const int ntr = c->ntr_h[s];
-        if (ntr < 1) continue;
-        for (int k = 0; k < 3; k++) {
-            if (plane[k] < 0) continue;
-            const float *syn = (const float *)c->sec.p + ((size_t)s * IFOS_NS + plane[k]) * comp;
-            float *adj = (float *)c->adj.p + ((size_t)s * 3 + k) * comp;
-            double *t = tr + ((size_t)s * 3 + k) * mr * 2;
-            KWindow kw{};
-            if (win) {
-                kw.picks = d_picks + (size_t)s * np * mr;
-                kw.stride = mr;
-                kw.tw_ind = win->tw_ind;
-                kw.gamma = win->gamma;
-                kw.twl_plus = win->twl_plus;
-                kw.twl_minus = win->twl_minus;
-            }
-            k_calc_res<<<(ntr + 127) / 128, 128, 0, c->st>>>(d_obs + ((size_t)s * 3 + k) * comp, syn, adj, ntr, ns,
-                                                             p.dt, t, t + mr, d_kill ? d_kill + (size_t)s * mr : nullptr,
-                                                             kw);
-            c->launches++;
-        }
+    KRes kr{};
+    kr.obs = d_obs;
+    kr.syn = (const float *)c->sec.p;
+    kr.diff = (float *)c->adj.p;
+    kr.tr = tr;
+    kr.comp = (long long)comp;
+    kr.obs_slot = 3 * kr.comp;
+    kr.syn_slot = IFOS_NS * kr.comp;
+    for (int k = 0; k < 3; k++) kr.plane[k] = plane[k];
+    kr.first = k0;
+    kr.ntr = (const int *)c->rec_n.p;
+    kr.mr = mr;
+    kr.ns = ns;
+    kr.dt = p.dt;
+    kr.kill = d_kill;
+    if (win) {
+        kr.win.picks = d_picks;
+        kr.win.stride = mr;
+        kr.win.tw_ind = win->tw_ind;
+        kr.win.gamma = win->gamma;
+        kr.win.twl_plus = win->twl_plus;
+        kr.win.twl_minus = win->twl_minus;
+        kr.win_slot = (long long)np * mr;
+    }
+    if (k1 >= k0) {
+        k_calc_res<<<dim3((mr + 31) / 32, k1 - k0 + 1, nshots), 32, 0, c->st>>>(kr);
+        c->launches++;
     }
     std::vector<double> h(tb / sizeof(double));
     CK(cudaMemcpyAsync(h.data(), tr, tb, cudaMemcpyDeviceToHost, c->st));
