@@ -256,10 +256,40 @@ __global__ void k_correlate(KGrid g, KState<T> S, KModel<T> M, KSnap sn, KGrad g
     }
 }
 
-// Zero-lag correlation for fp32 state and fp32 snapshots: the arithmetic of
-// k_correlate per cell, two adjacent cells of a row per thread with 8-byte
-// loads and stores (rows of NX cells, NX even; the pitched state planes are
-// always pair-aligned).  Grid: x over pairs of a row, y = row, z = slot.
+// 1/b and x/b in double for float b and x, rounded to nearest as the divisions
+// of the reference's expressions.  From an approximate float reciprocal
+// (relative error below 2^-22) one Newton step leaves a residual 1 - b*r of at
+// most 2^-43, which a double holds exactly (b has 24 bits); the second step
+// then rounds r*(1 + residual), whose relative error of 2^-86 is far below
+// the distance of a quotient of 24-bit numbers from a rounding boundary
+// (2^-78), so it rounds as 1/b does.  The same holds for the quotient after
+// one exact-remainder correction (Markstein, IBM J. Res. Dev. 34, 1990).
+// Outside the exponent range where every step is exact the division itself
+// runs.  A correlated cell has three such divisions; as divisions they were
+// most of its 344 instructions.
+struct Recip {
+    float b;
+    double r;
+    bool ok;
+    __device__ __forceinline__ explicit Recip(float d) : b(d) {
+        ok = d >= 0x1p-100f && d <= 0x1p100f;
+        float y;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(ok ? d : 1.0f));
+        const double bd = (double)(ok ? d : 1.0f);
+        r = (double)y;
+        r = __fma_rn(r, __fma_rn(-bd, r, 1.0), r);
+        r = __fma_rn(r, __fma_rn(-bd, r, 1.0), r);
+        if (!ok) r = 1.0 / (double)d;
+    }
+    // x/4 over b (the quarter is exact)
+    __device__ __forceinline__ double quarter_over(float x) const {
+        const double xq = .25 * (double)x;
+        if (!(ok && fabsf(x) <= 0x1p120f)) return xq / (double)b;
+        const double q = xq * r;
+        return __fma_rn(__fma_rn(-q, (double)b, xq), r, q);
+    }
+};
+
 struct CorrCell {
     float vxp1, vyp1, sxx, syy, sxy, sp, vzp1, sxz, syz;  // adjoint state
     float f[8];                                           // stored forward components
@@ -269,144 +299,176 @@ struct CorrCell {
 // rounded, exactly as src/IFOS2D.c:2379-2419 writes it), or double for the
 // grad_acc64 sums (the same terms added in double, rounded once at the end)
 template <int PSV, int SH, int AC, typename W = float>
-__device__ __forceinline__ void correlate_cell(const CorrCell &a, float mm, float ll, float rho, float u, W *w0,
-                                               W *w1, W *w2, W *w3, W *w4, bool mufix = false) {
+__device__ __forceinline__ void correlate_cell(const CorrCell &a, float mm, float ll, float rho, float u, W &w0,
+                                               W &w1, W &w2, W &w3, W &w4, bool mufix) {
     constexpr int KS = PSV ? (AC ? 3 : 5) : 0;  // first SH component
     if (PSV) {
         const float frx = a.f[0], fry = a.f[1];
-        *w2 += (W)(float)((a.vxp1 * frx) + (a.vyp1 * fry));
+        w2 += (W)(float)((a.vxp1 * frx) + (a.vyp1 * fry));
         if (!AC) {
             const float fx = a.f[2], fy = a.f[3], fu = a.f[4];
-            *w0 += (W)(float)((fx + fy) * (a.sxx + a.syy));
+            w0 += (W)(float)((fx + fy) * (a.sxx + a.syy));
             if (mm != 0.0f) {
-                const double t1 = (1.0 / (double)mm) * (double)(fu * a.sxy);
+                const Recip rm(mm), rl(ll);
+                const double t1 = rm.r * (double)(fu * a.sxy);
                 // mufix: the grouping the mu gradient needs (sums of forward times adjoint stresses)
-                const double t2 = (.25 * (double)(mufix ? (fx + fy) * (a.sxx + a.syy) : fx + fy * (a.sxx + a.syy))) /
-                                  (double)ll;
-                const double t3 = (.25 * (double)(mufix ? (fx - fy) * (a.sxx - a.syy) : fx - fy * (a.sxx - a.syy))) /
-                                  (double)mm;
-                *w1 = (W)((double)*w1 + ((t1 + t2) + t3));
+                const double t2 = rl.quarter_over(mufix ? (fx + fy) * (a.sxx + a.syy) : fx + fy * (a.sxx + a.syy));
+                const double t3 = rm.quarter_over(mufix ? (fx - fy) * (a.sxx - a.syy) : fx - fy * (a.sxx - a.syy));
+                w1 = (W)((double)w1 + ((t1 + t2) + t3));
             }
         } else {
             const float fp = a.f[2];
-            *w0 += (W)(float)((fp) * (a.sp));
+            w0 += (W)(float)((fp) * (a.sp));
         }
     }
     if (SH) {
         const float frz = a.f[KS], fxz = a.f[KS + 1], fyz = a.f[KS + 2];
-        *w4 += (W)(float)(a.vzp1 * frz);
+        w4 += (W)(float)(a.vzp1 * frz);
         const float muss = rho * u * u;
-        *w3 = (W)((double)*w3 + (1.0 / (double)(muss * muss)) * (double)(fxz * a.sxz + fyz * a.syz));
+        const Recip rm(muss * muss);
+        w3 = (W)((double)w3 + rm.r * (double)(fxz * a.sxz + fyz * a.syz));
     }
 }
 
-// SEG: 0 fp32 snapshots, 1 fp16 segments, 2 int16 segments; ACC64: the sums
-// in double (gr.acc64)
-template <int PSV, int SH, int AC, int SEG, bool ACC64 = false>
-__global__ void k_correlate_pairs(KGrid g, KState<float> S, KModel<float> M, KSnap sn, KGrad gr, int snap) {
+// V consecutive floats or 16-bit values, one aligned access
+template <int V>
+struct Vec {
+    float v[V];
+    __device__ __forceinline__ static Vec load(const float *p) {
+        Vec r;
+        if constexpr (V == 4) {
+            const float4 a = *reinterpret_cast<const float4 *>(p);
+            r.v[0] = a.x, r.v[1] = a.y, r.v[2] = a.z, r.v[3] = a.w;
+        } else if constexpr (V == 2) {
+            const float2 a = *reinterpret_cast<const float2 *>(p);
+            r.v[0] = a.x, r.v[1] = a.y;
+        } else {
+            r.v[0] = *p;
+        }
+        return r;
+    }
+    __device__ __forceinline__ void store(float *p) const {
+        if constexpr (V == 4) *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+        else if constexpr (V == 2) *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+        else *p = v[0];
+    }
+    // 16-bit segment values times the segment's scale
+    __device__ __forceinline__ static Vec load16(const unsigned short *p, float sc, bool i16) {
+        unsigned short h[V];
+        if constexpr (V == 4) {
+            const uint2 a = *reinterpret_cast<const uint2 *>(p);
+            h[0] = (unsigned short)a.x, h[1] = (unsigned short)(a.x >> 16), h[2] = (unsigned short)a.y,
+            h[3] = (unsigned short)(a.y >> 16);
+        } else if constexpr (V == 2) {
+            const unsigned a = *reinterpret_cast<const unsigned *>(p);
+            h[0] = (unsigned short)a, h[1] = (unsigned short)(a >> 16);
+        } else {
+            h[0] = *p;
+        }
+        Vec r;
+#pragma unroll
+        for (int e = 0; e < V; e++) r.v[e] = seg_unpack(h[e], i16) * sc;
+        return r;
+    }
+};
+
+// Zero-lag correlation for fp32 state and fp32 or 16-bit-segment snapshots:
+// the arithmetic of k_correlate per cell, V adjacent cells of a row per thread
+// (V the largest of 4, 2, 1 that divides NX: rows of the snapshots and sums
+// then start V-aligned, and no group straddles a 64-cell segment).  Threads
+// walk the groups of a slot row by row without gaps; grid: x over groups, y =
+// slot.  SEG: 0 fp32 snapshots, 1 fp16 segments, 2 int16 segments; ACC64: the
+// sums in double (gr.acc64).
+template <int PSV, int SH, int AC, int SEG, int V, bool ACC64 = false>
+__global__ void __launch_bounds__(128) k_correlate_cells(KGrid g, KState<float> S, KModel<float> M, KSnap sn, KGrad gr,
+                                                         int snap) {
     pdl_wait();
     pdl_launch();
     constexpr int NC = (PSV ? (AC ? 3 : 5) : 0) + (SH ? 3 : 0);
     // accumulators in use: lambda', mu', rho' (P-SV; acoustic: lambda', rho'), mu_z', rho_z' (SH)
     constexpr bool use[5] = {PSV != 0, PSV && !AC, PSV != 0, SH != 0, SH != 0};
-    const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + 1;
-    const int j = blockIdx.y + 1;
-    const int slot = blockIdx.z;
-    if (i > g.nx) return;
+    const int per = g.nx / V;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = t / per + 1;
+    if (j > g.ny) return;
+    const int i = (t - (j - 1) * per) * V + 1;
+    const int slot = blockIdx.y;
     const long long c = pidx(g, j, i), q = (long long)(j - 1) * g.nx + (i - 1), n = gr.n;
     const float *st = S.base + slot * S.slot_stride + c;
     const char *sb = (const char *)sn.base + slot * sn.slot_bytes + snap * sn.snap_bytes;
-    float *acc = gr.acc + (long long)slot * 5 * n + q;
-    auto ld2 = [](const float *p) { return *reinterpret_cast<const float2 *>(p); };
-    CorrCell a0{}, a1{};
-    auto field = [&](int id, float &x0, float &x1) {
-        const float2 v = ld2(st + S.off[id]);
-        x0 = v.x;
-        x1 = v.y;
-    };
+    auto field = [&](int id) { return Vec<V>::load(st + S.off[id]); };
+    Vec<V> vx{}, vy{}, xx{}, yy{}, xy{}, sp{}, vz{}, xz{}, yz{}, f[8];
     if (PSV) {
-        field(P_VXP1, a0.vxp1, a1.vxp1);
-        field(P_VYP1, a0.vyp1, a1.vyp1);
+        vx = field(P_VXP1);
+        vy = field(P_VYP1);
         if (!AC) {
-            field(P_SXX, a0.sxx, a1.sxx);
-            field(P_SYY, a0.syy, a1.syy);
-            field(P_SXY, a0.sxy, a1.sxy);
+            xx = field(P_SXX);
+            yy = field(P_SYY);
+            xy = field(P_SXY);
         } else {
-            field(P_SP, a0.sp, a1.sp);
+            sp = field(P_SP);
         }
     }
     if (SH) {
-        field(P_VZP1, a0.vzp1, a1.vzp1);
-        field(P_SXZ, a0.sxz, a1.sxz);
-        field(P_SYZ, a0.syz, a1.syz);
+        vz = field(P_VZP1);
+        xz = field(P_SXZ);
+        yz = field(P_SYZ);
     }
     if constexpr (SEG != 0) {
-        // 16-bit segments: a pair never straddles a segment (both start at odd i)
         const unsigned short *hs = (const unsigned short *)sb + q;
-        const float *ex = (const float *)(sb + sn.ex_off) + (long long)(j - 1) * sn.segs + (i - 1) / kSegCells;
+        const float *ex = (const float *)(sb + sn.ex_off) + (j - 1) * sn.segs + (i - 1) / kSegCells;
+        const int es = g.ny * sn.segs;
 #pragma unroll
-        for (int k = 0; k < NC; k++) {
-            const unsigned u = *reinterpret_cast<const unsigned *>(hs + k * sn.n);
-            const float sc = ex[(long long)k * g.ny * sn.segs];
-            a0.f[k] = seg_unpack((unsigned short)(u & 0xffffu), SEG == 2) * sc;
-            a1.f[k] = seg_unpack((unsigned short)(u >> 16), SEG == 2) * sc;
-        }
+        for (int k = 0; k < NC; k++) f[k] = Vec<V>::load16(hs + k * sn.n, ex[(long long)k * es], SEG == 2);
     } else {
-        const float *fs = (const float *)sb + q;
 #pragma unroll
-        for (int k = 0; k < NC; k++) {
-            const float2 v = ld2(fs + k * sn.n);
-            a0.f[k] = v.x;
-            a1.f[k] = v.y;
-        }
+        for (int k = 0; k < NC; k++) f[k] = Vec<V>::load((const float *)sb + q + k * sn.n);
     }
     const long long mo = (long long)M.slot_model[slot] * M.model_stride + c;
-    float2 mm{0, 0}, ll{0, 0}, rho{0, 0}, u{0, 0};
+    Vec<V> mm{}, ll{}, rho{}, u{};
     if (PSV && !AC) {
-        mm = ld2(M.m[M_MM] + mo);
-        ll = ld2(M.m[M_LL] + mo);
+        mm = Vec<V>::load(M.m[M_MM] + mo);
+        ll = Vec<V>::load(M.m[M_LL] + mo);
     }
     if (SH) {
-        rho = ld2(M.m[M_RHO] + mo);
-        u = ld2(M.m[M_VS] + mo);
+        rho = Vec<V>::load(M.m[M_RHO] + mo);
+        u = Vec<V>::load(M.m[M_VS] + mo);
     }
-    const bool pair = i + 1 <= g.nx;
+    auto cell = [&](int e) {
+        CorrCell a{vx.v[e], vy.v[e], xx.v[e], yy.v[e], xy.v[e], sp.v[e], vz.v[e], xz.v[e], yz.v[e], {}};
+#pragma unroll
+        for (int k = 0; k < NC; k++) a.f[k] = f[k].v[e];
+        return a;
+    };
     if constexpr (ACC64) {
         double *acd = gr.acc64 + (long long)slot * 5 * n + q;
-        double2 w[5] = {};
+#pragma unroll
+        for (int e = 0; e < V; e++) {
+            double w[5] = {};
+#pragma unroll
+            for (int k = 0; k < 5; k++)
+                if (use[k]) w[k] = acd[k * n + e];
+            correlate_cell<PSV, SH, AC, double>(cell(e), mm.v[e], ll.v[e], rho.v[e], u.v[e], w[0], w[1], w[2], w[3],
+                                                w[4], g.mu_fix != 0);
+#pragma unroll
+            for (int k = 0; k < 5; k++)
+                if (use[k]) acd[k * n + e] = w[k];
+        }
+    } else {
+        float *acc = gr.acc + (long long)slot * 5 * n + q;
+        Vec<V> w[5] = {};
 #pragma unroll
         for (int k = 0; k < 5; k++)
-            if (use[k]) w[k] = *reinterpret_cast<const double2 *>(acd + k * n);
-        correlate_cell<PSV, SH, AC, double>(a0, mm.x, ll.x, rho.x, u.x, &w[0].x, &w[1].x, &w[2].x, &w[3].x, &w[4].x,
-                                            g.mu_fix != 0);
-        if (pair)
-            correlate_cell<PSV, SH, AC, double>(a1, mm.y, ll.y, rho.y, u.y, &w[0].y, &w[1].y, &w[2].y, &w[3].y,
-                                                &w[4].y, g.mu_fix != 0);
+            if (use[k]) w[k] = Vec<V>::load(acc + k * n);
 #pragma unroll
-        for (int k = 0; k < 5; k++) {
-            if (!use[k]) continue;
-            if (pair) *reinterpret_cast<double2 *>(acd + k * n) = w[k];
-            else acd[k * n] = w[k].x;
-        }
-        return;
-    }
-    float2 w[5] = {};
+        for (int e = 0; e < V; e++)
+            correlate_cell<PSV, SH, AC, float>(cell(e), mm.v[e], ll.v[e], rho.v[e], u.v[e], w[0].v[e], w[1].v[e],
+                                               w[2].v[e], w[3].v[e], w[4].v[e], g.mu_fix != 0);
 #pragma unroll
-    for (int k = 0; k < 5; k++)
-        if (use[k]) w[k] = ld2(acc + k * n);
-    correlate_cell<PSV, SH, AC>(a0, mm.x, ll.x, rho.x, u.x, &w[0].x, &w[1].x, &w[2].x, &w[3].x, &w[4].x, g.mu_fix != 0);
-    if (pair)
-        correlate_cell<PSV, SH, AC>(a1, mm.y, ll.y, rho.y, u.y, &w[0].y, &w[1].y, &w[2].y, &w[3].y, &w[4].y,
-                                    g.mu_fix != 0);
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-        if (!use[k]) continue;
-        if (pair) *reinterpret_cast<float2 *>(acc + k * n) = w[k];
-        else acc[k * n] = w[k].x;
+        for (int k = 0; k < 5; k++)
+            if (use[k]) w[k].store(acc + k * n);
     }
 }
-
-
 
 // The assembly of an fp64 context (the error oracle): the formulas of
 // src/IFOS2D.c:2477-2601 in double from the double sums, rounded once into

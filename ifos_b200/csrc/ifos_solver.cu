@@ -908,6 +908,44 @@ static int forward_t(ifos_ctx *c, int nshots, int store, int nsteps) {
     return IFOS_OK;
 }
 
+// The zero-lag correlation of fp32 contexts with fp32 or 16-bit-segment
+// snapshots; false for the formats it does not cover.
+template <int PSV, int SH, int AC, int SEG, int V, bool A64>
+static void correlate_launch(ifos_ctx *c, const Launcher<float> &L, const KSnap &sn, const KGrad &gr, int snap, int ns) {
+    const long long groups = (long long)(c->p.nx / V) * c->p.ny;
+    launch_dep(c->st, c->pdl, k_correlate_cells<PSV, SH, AC, SEG, V, A64>, dim3((unsigned)((groups + 127) / 128), ns),
+               dim3(128), 0, c->g, L.S, L.M, sn, gr, snap);
+}
+template <int SEG, int V, bool A64>
+static void correlate_physics(ifos_ctx *c, const Launcher<float> &L, const KSnap &sn, const KGrad &gr, int snap, int ns) {
+    if (c->ac) correlate_launch<1, 0, 1, SEG, V, A64>(c, L, sn, gr, snap, ns);
+    else if (c->psv && c->sh) correlate_launch<1, 1, 0, SEG, V, A64>(c, L, sn, gr, snap, ns);
+    else if (c->psv) correlate_launch<1, 0, 0, SEG, V, A64>(c, L, sn, gr, snap, ns);
+    else correlate_launch<0, 1, 0, SEG, V, A64>(c, L, sn, gr, snap, ns);
+}
+template <int SEG>
+static void correlate_width(ifos_ctx *c, const Launcher<float> &L, const KSnap &sn, const KGrad &gr, int snap, int ns) {
+    const int v = c->p.nx % 4 == 0 ? 4 : (c->p.nx % 2 == 0 ? 2 : 1);
+    if (gr.acc64) {  // even NX only
+        if (v == 4) correlate_physics<SEG, 4, true>(c, L, sn, gr, snap, ns);
+        else correlate_physics<SEG, 2, true>(c, L, sn, gr, snap, ns);
+    } else if (v == 4) {
+        correlate_physics<SEG, 4, false>(c, L, sn, gr, snap, ns);
+    } else if (v == 2) {
+        correlate_physics<SEG, 2, false>(c, L, sn, gr, snap, ns);
+    } else {
+        correlate_physics<SEG, 1, false>(c, L, sn, gr, snap, ns);
+    }
+}
+static bool correlate_cells(ifos_ctx *c, const Launcher<float> &L, const KSnap &sn, const KGrad &gr, int snap, int ns) {
+    switch (c->p.snap_format) {
+        case IFOS_SNAP_F32: correlate_width<0>(c, L, sn, gr, snap, ns); return true;
+        case IFOS_SNAP_F16S: correlate_width<1>(c, L, sn, gr, snap, ns); return true;
+        case IFOS_SNAP_I16S: correlate_width<2>(c, L, sn, gr, snap, ns); return true;
+        default: return false;
+    }
+}
+
 template <typename T>
 static int adjoint_t(ifos_ctx *c, int nshots) {
     const ifos_params &p = c->p;
@@ -955,52 +993,10 @@ static int adjoint_t(ifos_ctx *c, int nshots) {
         Lr.post_adj(nt, p.adjoint_type == 4);
         if (snap_step) {
             KTimer t(c, 3, sample);
-            bool pairs = false;
-            if constexpr (std::is_same<T, float>::value) {
-                const bool f16s = p.snap_format == IFOS_SNAP_F16S, i16s = p.snap_format == IFOS_SNAP_I16S;
-                if ((p.snap_format == IFOS_SNAP_F32 || f16s || i16s) && p.nx % 2 == 0) {
-                    const dim3 gc((unsigned)((p.nx / 2 + 127) / 128), (unsigned)p.ny, (unsigned)nshots);
-                    const int h = ntd - hin_a;
-                    auto corr = [&](auto kern) {
-                        launch_dep(c->st, c->pdl, kern, dim3(gc), dim3(128), 0, c->g, Lr.S, Lr.M, sn, gr, h);
-                    };
-                    if (gr.acc64) {  // the sums in double (grad_acc64)
-                        if (f16s) {
-                            if (c->ac) corr(k_correlate_pairs<1, 0, 1, 1, true>);
-                            else if (c->psv && c->sh) corr(k_correlate_pairs<1, 1, 0, 1, true>);
-                            else if (c->psv) corr(k_correlate_pairs<1, 0, 0, 1, true>);
-                            else corr(k_correlate_pairs<0, 1, 0, 1, true>);
-                        } else if (i16s) {
-                            if (c->ac) corr(k_correlate_pairs<1, 0, 1, 2, true>);
-                            else if (c->psv && c->sh) corr(k_correlate_pairs<1, 1, 0, 2, true>);
-                            else if (c->psv) corr(k_correlate_pairs<1, 0, 0, 2, true>);
-                            else corr(k_correlate_pairs<0, 1, 0, 2, true>);
-                        } else {
-                            if (c->ac) corr(k_correlate_pairs<1, 0, 1, 0, true>);
-                            else if (c->psv && c->sh) corr(k_correlate_pairs<1, 1, 0, 0, true>);
-                            else if (c->psv) corr(k_correlate_pairs<1, 0, 0, 0, true>);
-                            else corr(k_correlate_pairs<0, 1, 0, 0, true>);
-                        }
-                    } else if (f16s) {
-                        if (c->ac) corr(k_correlate_pairs<1, 0, 1, 1>);
-                        else if (c->psv && c->sh) corr(k_correlate_pairs<1, 1, 0, 1>);
-                        else if (c->psv) corr(k_correlate_pairs<1, 0, 0, 1>);
-                        else corr(k_correlate_pairs<0, 1, 0, 1>);
-                    } else if (i16s) {
-                        if (c->ac) corr(k_correlate_pairs<1, 0, 1, 2>);
-                        else if (c->psv && c->sh) corr(k_correlate_pairs<1, 1, 0, 2>);
-                        else if (c->psv) corr(k_correlate_pairs<1, 0, 0, 2>);
-                        else corr(k_correlate_pairs<0, 1, 0, 2>);
-                    } else {
-                        if (c->ac) corr(k_correlate_pairs<1, 0, 1, 0>);
-                        else if (c->psv && c->sh) corr(k_correlate_pairs<1, 1, 0, 0>);
-                        else if (c->psv) corr(k_correlate_pairs<1, 0, 0, 0>);
-                        else corr(k_correlate_pairs<0, 1, 0, 0>);
-                    }
-                    pairs = true;
-                }
-            }
-            if (!pairs)
+            bool cells = false;
+            if constexpr (std::is_same<T, float>::value)
+                cells = correlate_cells(c, Lr, sn, gr, ntd - hin_a, nshots);
+            if (!cells)
                 launch_dep(c->st, c->pdl, k_correlate<T>, dim3(Lr.grd), dim3(Lr.blk), 0, c->g, Lr.S, Lr.M, sn, gr, ntd - hin_a, c->psv, c->sh,
                                                             c->ac);
             c->launches++;
