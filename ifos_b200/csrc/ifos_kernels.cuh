@@ -51,19 +51,19 @@ struct KGrid {
     int adjoint_type;
     int k_one;       // every CPML K profile value is 1: d/K == d exactly
     int dh_pow2;     // DH is a power of two: x/DH == x*inv_dh exactly
-    float inv_dh;    // 1/DH (exact when dh_pow2)
+    float inv_dh;    // 1/DH, correctly rounded
     int tile_order;  // pipelined stencils: 0 slot-major tile sequence, 1 slot-minor
     int prod_polls;  // pipelined stencils: polls of the producer's stage-release wait (0: the default limit)
     int mu_fix;      // the mu correlation with the corrected grouping (ifos_params.mu_corrected)
+    // layout of the CPML strips: floats per row of an x strip and of a y strip,
+    // the column where the right x strip starts in a row (psx_lw), the grid
+    // column it starts at (psx_rs, 0-based, a multiple of 4) and the offset of
+    // a right-strip profile index (psx_roff).  Four cells of a group whose
+    // first column is a multiple of 4 are 16-byte aligned in every strip.
+    int psx, psy, psx_lw, psx_rs, psx_roff;
+    float div_lo, div_hi;  // |x| for which div_dh4 uses the reciprocal
     int lame;        // PARAMETERIZATION 3: the model planes hold lambda and mu, the assembly stops at the moduli
 };
-
-// x / DH, exact in both branches: multiplying by the reciprocal of a power of
-// two rounds exactly as the division does.
-template <typename T>
-__device__ __forceinline__ T div_dh(const KGrid &g, T x) {
-    return g.dh_pow2 ? x * (T)g.inv_dh : x / (T)g.dh;
-}
 
 template <typename T>
 struct KState {
@@ -71,17 +71,24 @@ struct KState {
     long long slot_stride;    // elements between slots
     long long off[NP_FIELD];  // plane offsets within a slot (-1 absent)
     long long mem_off[5];     // first plane of r,p,q,t,o (L planes each), -1 absent
-    T *psix[NX_STRIP];        // slot 0 strip, NY x 2FW each
-    T *psiy[NY_STRIP];        // slot 0 strip, 2FW x NX each
+    T *psix[NX_STRIP];        // slot 0 strip, NY rows of KGrid::psx
+    T *psiy[NY_STRIP];        // slot 0 strip, 2FW rows of KGrid::psy
     long long psix_slot, psiy_slot;  // elements between slots of one strip
 };
+
+// the CPML profiles as a stencil block stages them (KModel::proftab): the six x
+// profiles by column of a strip row, the six y profiles by profile index
+constexpr int kProfX = 72, kProfY = 64;
 
 template <typename T>
 struct KModel {
     const T *m[NM_PLANE];  // model 0 planes (NULL absent)
     long long model_stride;
     const int *slot_model;  // model index of every slot
+    int one_model;          // the context holds one model: every index is 0
     const T *prof;          // 12 x (2FW+1)
+    const T *proftab;       // 6 x kProfX, 6 x kProfY values (NULL: the strips are wider)
+    const T *profx;         // the six x profiles by grid column (6 x KGrid::psy; 1 and 0 outside the strips)
     const T *srf;           // 4 x NX per model: fjm, g, djm, e (row j=1)
     long long srf_stride;
 };
@@ -132,25 +139,16 @@ __device__ __forceinline__ double div_rn_pinned(double x, double y) {
     return q;
 }
 
-// CPML recursion of every kernel: psi = b*psi + a*d; d = d/K + psi.  With
-// every K equal to 1 (k_one) the quotient is d itself and no division runs.
+// CPML recursion of every kernel: psi = b*psi + a*d; d = d/K + psi
 template <typename T>
-__device__ inline T cpml(T *psi, T b, T a, T K, T d, int k_one = 0) {
+__device__ inline T cpml(T *psi, T b, T a, T K, T d) {
     const T ps = b * *psi + a * d;
     *psi = ps;
-    if (k_one) return d + ps;
     return div_rn_pinned(d, K) + ps;
 }
 
-// CPML on precomputed strip indices (0: not in the strip): hx is the 1-based
-// profile index of the x strip (left: i, right: i-NX+2FW), hy that of the y
-// strip (top without free surface: j, bottom: j-NY+2FW).
-__device__ __forceinline__ int strip_x(const KGrid &g, int i) {
-    if (g.boundary || g.fw == 0) return 0;
-    if (i <= g.fw) return i;
-    if (i >= g.nx - g.fw + 1) return i - g.nx + 2 * g.fw;
-    return 0;
-}
+// profile index of row j in a y strip (top without free surface: j, bottom:
+// j-NY+2FW; 0: not in a strip)
 __device__ __forceinline__ int strip_y(const KGrid &g, int j) {
     if (g.fw == 0) return 0;
     if (!g.free_surf && j <= g.fw) return j;
@@ -162,13 +160,12 @@ __device__ __forceinline__ int strip_y(const KGrid &g, int j) {
 template <typename T>
 __device__ inline T cpml_x(const KGrid &g, const KModel<T> &M, T *strip, int j, int i, int kk, int ka, int kb,
                            T d) {
-    const int n2 = 2 * g.fw;
     if (!g.boundary && i <= g.fw)
-        d = cpml(strip + (long long)(j - 1) * n2 + (i - 1), prof(M, g, kb, i), prof(M, g, ka, i), prof(M, g, kk, i),
+        d = cpml(strip + (long long)(j - 1) * g.psx + (i - 1), prof(M, g, kb, i), prof(M, g, ka, i), prof(M, g, kk, i),
                  d);
     if (!g.boundary && i >= g.nx - g.fw + 1) {
         int h = i - g.nx + 2 * g.fw;
-        d = cpml(strip + (long long)(j - 1) * n2 + (h - 1), prof(M, g, kb, h), prof(M, g, ka, h), prof(M, g, kk, h),
+        d = cpml(strip + (long long)(j - 1) * g.psx + (h - 1 + g.psx_roff), prof(M, g, kb, h), prof(M, g, ka, h), prof(M, g, kk, h),
                  d);
     }
     return d;
@@ -178,11 +175,11 @@ template <typename T>
 __device__ inline T cpml_y(const KGrid &g, const KModel<T> &M, T *strip, int j, int i, int kk, int ka, int kb,
                            T d) {
     if (!g.free_surf && j <= g.fw)
-        d = cpml(strip + (long long)(j - 1) * g.nx + (i - 1), prof(M, g, kb, j), prof(M, g, ka, j),
+        d = cpml(strip + (long long)(j - 1) * g.psy + (i - 1), prof(M, g, kb, j), prof(M, g, ka, j),
                  prof(M, g, kk, j), d);
     if (j >= g.ny - g.fw + 1) {
         int h = j - g.ny + 2 * g.fw;
-        d = cpml(strip + (long long)(h - 1) * g.nx + (i - 1), prof(M, g, kb, h), prof(M, g, ka, h),
+        d = cpml(strip + (long long)(h - 1) * g.psy + (i - 1), prof(M, g, kb, h), prof(M, g, ka, h),
                  prof(M, g, kk, h), d);
     }
     return d;
@@ -660,15 +657,6 @@ struct KRec {
     long long map_stride;
     int rmax;
 };
-
-// receiver indices of cells (j, i) and (j, i+1) of `slot` (-1: none)
-__device__ __forceinline__ int2 rec_pair(const KRec &r, int nx, int ny, int slot, int j, int i, bool v0, bool v1) {
-    const int *m = r.map + (long long)slot * r.map_stride;
-    const int rr = m[j - 1];
-    if (rr < 0) return make_int2(-1, -1);
-    const int *cells = m + ny + (long long)rr * nx + (i - 1);
-    return make_int2(v0 ? cells[0] : -1, v1 ? cells[1] : -1);
-}
 
 template <typename T>
 __global__ void k_inject_v_fwd(KGrid g, KState<T> S, KModel<T> M, KSrc src, int nt, int psv, int sh) {

@@ -28,29 +28,19 @@
 
 using namespace ifos;
 
-// rows of a pipelined tile (kTileX = 64 columns x kTileY rows)
-#ifndef IFOS_TILE_Y
-#define IFOS_TILE_Y 8
-#endif
-static constexpr int kTileY = IFOS_TILE_Y;
-// rows of the velocity ops' tiles (their own tensor maps when they differ)
-#ifndef IFOS_VTILE_Y
-#define IFOS_VTILE_Y 8
-#endif
-static constexpr int kTileYV = IFOS_VTILE_Y;
+static constexpr int kTileY = 8;  // rows of a pipelined tile (kTileX = 64 columns x kTileY rows)
 
-// Stages of an op's shared-memory ring: as many as fit when kRingBlocks
-// blocks share an SM's 227 KB (2..6).  Loads stay in flight in every stage
-// but the one being computed, so deeper rings keep more bytes in flight.
-#ifndef IFOS_RING_BLOCKS
-#define IFOS_RING_BLOCKS 3
-#endif
-constexpr int kRingBlocks = IFOS_RING_BLOCKS;
-template <int FD, int NH, int NP, int NO, int TY = kTileY, int RB = kRingBlocks>
+// shared memory of a block beside its ring: the tile queue, profiles and barriers, and
+// what the system reserves
+constexpr int kBlockSmem = 1024 + 2 * kTileBatch * (int)sizeof(TileInfo) + 6 * (kProfX + kProfY) * 4 + 128;
+
+// Stages of an op's shared-memory ring: as many as fit when `blocks` blocks
+// share an SM's 227 KB (1..6).
+template <int FD, int NH, int NP, int NO, int TY, int RB>
 constexpr int ring_stages() {
     constexpr size_t stage = Pipe<FD, TY, NH, NP, NO, 1>::bytes();
-    constexpr int n = (int)((232448 / RB - 1024) / stage);
-    return n < 2 ? 2 : (n > 6 ? 6 : n);
+    constexpr int n = (int)((232448 / RB - kBlockSmem) / stage);
+    return n < 1 ? 1 : (n > 6 ? 6 : n);
 }
 
 // Launch a kernel of the time loop as a programmatic dependent of the
@@ -98,6 +88,7 @@ struct LoopGraph {
     std::vector<TimedPair> pairs;
 };
 
+enum { MAP_HALO = 0, MAP_PLAIN, MAP_MODEL };
 struct ifos_ctx {
     ifos_params p{};
     int device = 0;
@@ -112,6 +103,8 @@ struct ifos_ctx {
     // state
     DevBuf state, psi, models, prof, srf, slot_model, src_pos, src_sig, src_n, rec_pos, rec_n, rec_map, adj, sec,
         snap, snap_scale, gacc, gacc64, gout, bad, dot_partial, dot_out, res_tr;
+    long long proftab_off = 0;  // elements from prof to the table the stencil blocks stage (0: none)
+    long long profx_off = 0;  // elements from prof to the x profiles by grid column
     long long slot_stride = 0, psix_len = 0, psiy_len = 0, psi_slot = 0, model_stride = 0;
     long long off[NP_FIELD];
     long long mem_off[5];
@@ -151,8 +144,9 @@ struct ifos_ctx {
     bool pipe = false;
     bool fused_snap = false;  // fp32 snapshots written by the stencil kernels
     bool pdl = true;          // time-loop kernels launched as programmatic dependents
-    KMaps maps{};
-    KMaps maps_v{};  // tensor maps of the velocity ops' tile height
+    // tensor maps by kind and planes per box, encoded by setup_pipeline for every depth an op loads
+    CUtensorMap tmaps[3][3 * kPipeMaxL + 1];
+    const CUtensorMap *tensor_map(int kind, int depth) const { return &tmaps[kind][depth]; }
     KTma ktma{};
     int num_sms = 148;
     // execution options (IFOS_OPT_*)
@@ -188,7 +182,10 @@ inline KModel<T> kmodel(const ifos_ctx *c) {
     }
     m.model_stride = c->model_stride;
     m.slot_model = (const int *)c->slot_model.p;
+    m.one_model = c->p.max_models == 1;
     m.prof = (const T *)c->prof.p;
+    m.profx = m.prof + c->profx_off;
+    m.proftab = c->proftab_off ? m.prof + c->proftab_off : nullptr;
     m.srf = (const T *)c->srf.p;
     m.srf_stride = 4LL * c->p.nx;
     return m;
@@ -280,6 +277,28 @@ struct Launcher {
         rec = krec(c);
         grd = dim3((c->p.nx + 31) / 32, (c->p.ny + 7) / 8, ns);
     }
+    // the snapshot a launch stores (hin < 0: none)
+    KSnapOut snap_out(int hin) const {
+        KSnapOut so{};
+        if (hin >= 0) {
+            so.base = (char *)c->snap.p + (size_t)hin * c->snap_bytes;
+            so.slot_bytes = c->snap_slot_bytes;
+            so.n = (long long)c->p.nx * c->p.ny;
+            so.align = c->p.nx % 4 == 0 ? 4 : (c->p.nx % 2 == 0 ? 2 : 1);
+            so.f16 = c->p.snap_format == IFOS_SNAP_F16S;
+            so.ex_off = c->snap_ex_off;
+            so.segs = (c->p.nx + 63) / 64;
+        }
+        return so;
+    }
+    // the pipelined launches of half width FD: defined where ifos_pipe.cu is
+    // compiled for that width, so that their kernels are compiled once
+    // hin: snapshot index stored by this step's kernels (-1 none)
+    template <int FD>
+    void v_pipe(int sw, int want_p1, int hin);
+    template <int FD>
+    void s_pipe(int hin);
+#ifdef IFOS_PIPE_FD
     // one persistent launch of a pipelined stencil op over all tiles of all slots
     template <typename Op>
     void pipelined(const Op &op0) {
@@ -291,7 +310,7 @@ struct Launcher {
         op.rec_j0 = rec_j0;
         op.rec_j1 = rec_j1;
         op.bad = (int *)c->bad.p;
-        static_assert(P::bytes() + 1024 <= 232448, "shared-memory ring exceeds 227 KB");
+        static_assert(P::bytes() + kBlockSmem <= 232448, "shared-memory ring exceeds 227 KB");
         auto kern = kp_stencil<Op>;
         constexpr int kMaxDev = 64;
         static int occ[kMaxDev] = {0};  // resident blocks per SM, per device (0: not queried)
@@ -299,30 +318,23 @@ struct Launcher {
         if (!occ[d]) {
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::bytes());
             int o = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, kBlockThreads, P::bytes());
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, P::THREADS, P::bytes());
             occ[d] = o > 0 ? o : 1;
         }
         const long long ntiles =
             (long long)((c->p.nx + kTileX - 1) / kTileX) * ((c->p.ny + P::TILE_Y - 1) / P::TILE_Y) * nshots;
         const int bps = c->blocks_per_sm > 0 ? std::min(c->blocks_per_sm, occ[d]) : occ[d];
         const int grid = (int)std::min<long long>(ntiles, (long long)bps * c->num_sms);
-        const KMaps &mp = P::TILE_Y == kTileY ? c->maps : c->maps_v;
-        launch_dep(c->st, c->pdl, kern, dim3(grid), dim3(32, kComputeWarps + 1), P::bytes(), mp, op, nshots,
+        KMaps mp;
+        mp.halo = *c->tensor_map(MAP_HALO, Op::NH_);
+        for (int k = 0; k < Op::NG; k++) mp.grp[k] = *c->tensor_map(Op::gm(k) ? MAP_MODEL : MAP_PLAIN, Op::gd(k));
+        // A dependent launch pays while the grid leaves slots free: its start is
+        // then hidden.  A launch that fills the GPU can only take the slots that come free first and end unevenly spread
+        // over the SMs (4000 x 1200: 110 against 100 us a step; 300 x 100:
+        // 10 against 12 us).
+        const bool dep = c->pdl && grid < occ[d] * c->num_sms;
+        launch_dep(c->st, dep, kern, dim3(grid), dim3(32, P::NCW + 1), P::bytes(), mp, op, nshots,
                    (int *)c->bad.p);
-    }
-    // the snapshot a launch stores (hin < 0: none)
-    KSnapOut snap_out(int hin) const {
-        KSnapOut so{};
-        if (hin >= 0) {
-            so.base = (char *)c->snap.p + (size_t)hin * c->snap_bytes;
-            so.slot_bytes = c->snap_slot_bytes;
-            so.n = (long long)c->p.nx * c->p.ny;
-            so.pairs = (c->p.nx % 2) == 0;
-            so.f16 = c->p.snap_format == IFOS_SNAP_F16S;
-            so.ex_off = c->snap_ex_off;
-            so.segs = (c->p.nx + 63) / 64;
-        }
-        return so;
     }
     template <int FD, bool Q, int SW, bool P1>
     void v_one(int hin) {
@@ -330,17 +342,16 @@ struct Launcher {
         const KTma &t = c->ktma;
         if (c->ac) {
             constexpr int NP = (SW == 1 && !Q) ? 6 : 4;
-            pipelined(OpVPsv<FD, kTileYV, ring_stages<FD, 1, NP, 0, kTileYV, vblocks(FD)>(), Q, SW, P1, true>{g, S, M, t, snap_out(hin)});
+            pipelined(OpVPsv<FD, kTileY, ring_stages<FD, 1, NP, 0, kTileY, vblocks(FD)>(), Q, SW, P1, true>{g, S, M, t, snap_out(hin)});
             return;
         }
         if (c->psv) {
             constexpr int NP = (SW == 1 && !Q) ? 6 : 4;
-            pipelined(OpVPsv<FD, kTileYV, ring_stages<FD, 3, NP, 0, kTileYV, vblocks(FD)>(), Q, SW, P1, false>{g, S, M, t, snap_out(hin)});
+            pipelined(OpVPsv<FD, kTileY, ring_stages<FD, 3, NP, 0, kTileY, vblocks(FD)>(), Q, SW, P1, false>{g, S, M, t, snap_out(hin)});
         }
     }
-    // hin: snapshot index stored by this step's kernels (-1 none)
     template <int FD>
-    void v_pipe(int sw, int want_p1, int hin) {
+    void v_pipe_(int sw, int want_p1, int hin) {
         bool done = false;
         if constexpr (FD >= 5) {
             if (c->g.quirk_hi) {
@@ -353,12 +364,12 @@ struct Launcher {
             else if (want_p1) v_one<FD, false, 0, true>(hin);
             else v_one<FD, false, 0, false>(-1);
         }
-        if (c->sh) pipelined(OpVSh<FD, kTileYV, ring_stages<FD, 2, 2, 0, kTileYV, vblocks(FD)>()>{c->g, S, M, c->ktma, snap_out(hin)});
+        if (c->sh) pipelined(OpVSh<FD, kTileY, ring_stages<FD, 2, 2, 0, kTileY, vblocks(FD)>()>{c->g, S, M, c->ktma, snap_out(hin)});
     }
     template <int FD, int LL>
     void s_visc_pipe(int hin) {
         const KGrid &g = c->g;
-        constexpr int NST = ring_stages<FD, 2, 3 + 3 * LL + 6, 0>();
+        constexpr int NST = ring_stages<FD, 2, 3 + 3 * LL + 6, 0, kTileY, visc_blocks(LL)>();
         if (c->psv) {
             bool done = false;
             if constexpr (FD >= 5) {
@@ -372,14 +383,14 @@ struct Launcher {
                 pipelined(OpSVisc<FD, kTileY, LL, NST, false>{g, S, M, c->ktma, snap_out(hin), src, nt_cur, fsurf, fps, src_j0,
                                                               src_j1});
         }
-        if (c->sh) pipelined(OpSSh<FD, kTileY, LL, ring_stages<FD, 1, 2 + 2 * LL + 4, 0>()>{g, S, M, c->ktma, snap_out(hin)});
+        if (c->sh) pipelined(OpSSh<FD, kTileY, LL, ring_stages<FD, 1, 2 + 2 * LL + 4, 0, kTileY, 3>()>{g, S, M, c->ktma, snap_out(hin)});
     }
     template <int FD, int LL>
     void p_visc_pipe(int hin) {
-        pipelined(OpPVisc<FD, kTileY, LL, ring_stages<FD, 2, 3 + LL, 0>()>{c->g, S, M, c->ktma, snap_out(hin)});
+        pipelined(OpPVisc<FD, kTileY, LL, ring_stages<FD, 2, 3 + LL, 0, kTileY, 3>()>{c->g, S, M, c->ktma, snap_out(hin)});
     }
     template <int FD>
-    void s_pipe(int hin) {
+    void s_pipe_(int hin) {
         const KGrid &g = c->g;
         const KTma &t = c->ktma;
         bool quirk = false;
@@ -395,7 +406,7 @@ struct Launcher {
             return;
         }
         if (c->ac) {
-            constexpr int NST = ring_stages<FD, 2, 2, 0>();
+            constexpr int NST = ring_stages<FD, 2, 2, 0, kTileY, sblocks(FD)>();
             if constexpr (FD >= 5) {
                 if (quirk) {
                     pipelined(OpPAc<FD, kTileY, NST, true>{g, S, M, t, snap_out(hin)});
@@ -418,7 +429,7 @@ struct Launcher {
                     }
                     if (!done) pipelined(OpSEl<FD, kTileY, NST, false>{g, S, M, t, snap_out(hin), src, nt_cur, fsurf, fps, src_j0, src_j1});
                 }
-                if (c->sh) pipelined(OpSSh<FD, kTileY, 0, ring_stages<FD, 1, 4, 0>()>{g, S, M, t, snap_out(hin)});
+                if (c->sh) pipelined(OpSSh<FD, kTileY, 0, ring_stages<FD, 1, 4, 0, kTileY, sblocks(FD)>()>{g, S, M, t, snap_out(hin)});
                 break;
             case 1: s_visc_pipe<FD, 1>(hin); break;
             case 2: s_visc_pipe<FD, 2>(hin); break;
@@ -427,6 +438,7 @@ struct Launcher {
             default: s_visc_pipe<FD, 5>(hin); break;
         }
     }
+#endif
     void v_step(int sw, int want_p1, int hin = -1) {
         const KGrid &g = c->g;
         if constexpr (std::is_same<T, float>::value) {
@@ -502,7 +514,18 @@ struct Launcher {
 // The pipelined stencil launches of each width are instantiated in their own
 // translation unit (ifos_pipe.cu with IFOS_PIPE_FD set); everywhere else they
 // are only declared.
-#ifndef IFOS_PIPE_FD
+#ifdef IFOS_PIPE_FD
+template <typename T>
+template <int FD>
+void Launcher<T>::v_pipe(int sw, int want_p1, int hin) {
+    v_pipe_<FD>(sw, want_p1, hin);
+}
+template <typename T>
+template <int FD>
+void Launcher<T>::s_pipe(int hin) {
+    s_pipe_<FD>(hin);
+}
+#else
 #define IFOS_EXTERN_PIPE(FD)                                      \
     extern template void Launcher<float>::v_pipe<FD>(int, int, int); \
     extern template void Launcher<float>::s_pipe<FD>(int);

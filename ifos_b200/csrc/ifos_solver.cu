@@ -144,6 +144,7 @@ struct Layout {
     long long snap_bytes_per, snap_slot_bytes;
     long long snap_ex_off;  // fp16 segments: bytes from a snapshot to its exponents
     int ncomp, segs;
+    int psx, psy, psx_lw, psx_rs;
 };
 
 static Layout layout_of(const ifos_params &p) {
@@ -157,8 +158,16 @@ static Layout layout_of(const ifos_params &p) {
     if (sh) L.nfield += 4;
     L.nmem = p.L ? (psv ? (p.acoustic ? 1 : 3) * p.L : 0) + (sh ? 2 * p.L : 0) : 0;
     L.slot_elems = (long long)(L.nfield + L.nmem) * L.plane;
-    L.psix = (long long)p.ny * 2 * p.fw;
-    L.psiy = (long long)2 * p.fw * p.nx;
+    // CPML strips in aligned groups of four columns: an x-strip row holds the
+    // left strip's groups, then the right strip's
+    if (p.fw > 0) {
+        L.psy = (p.nx + 3) / 4 * 4;
+        L.psx_lw = (p.fw + 3) / 4 * 4;
+        L.psx_rs = (p.nx - p.fw) / 4 * 4;
+        L.psx = L.psx_lw + L.psy - L.psx_rs;
+    }
+    L.psix = (long long)p.ny * L.psx;
+    L.psiy = (long long)2 * p.fw * L.psy;
     L.psi_slot = NX_STRIP * L.psix + NY_STRIP * L.psiy;
     // model planes: rho vp vs rip rjp always; + elastic (uipjp f g mm ll) or acoustic g;
     // + visco (fipjp f g mu pi muipjp [taus taup tausipjp]) or viscoacoustic (g pi [taup])
@@ -262,14 +271,14 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 // fp32 planes of `pitch` x `rows` elements, `planes` of them back to back;
-// boxes of box_w x box_h x 1, zero fill outside
+// boxes of box_w x box_h x box_d, zero fill outside
 static bool encode_planes(CUtensorMap *m, void *base, long long pitch, long long rows, long long planes, int box_w,
-                          int box_h) {
+                          int box_h, int box_d) {
     PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
     if (!enc) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)pitch, (cuuint64_t)rows, (cuuint64_t)planes};
     const cuuint64_t strides[2] = {(cuuint64_t)pitch * 4, (cuuint64_t)(pitch * rows) * 4};
-    const cuuint32_t box[3] = {(cuuint32_t)box_w, (cuuint32_t)box_h, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)box_w, (cuuint32_t)box_h, (cuuint32_t)box_d};
     const cuuint32_t estr[3] = {1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -290,16 +299,12 @@ static void setup_pipeline(ifos_ctx *c, const Layout &L) {
     const int fdoh = c->g.fdoh, xh = ((fdoh + 3) / 4) * 4;
     const long long st_planes = (long long)t.planes_per_slot * c->p.max_shots;
     const long long md_planes = (long long)t.model_planes * c->p.max_models;
-    if (!encode_planes(&c->maps.halo, c->state.p, L.pitch, L.rows, st_planes, kTileX + 2 * xh, kTileY + 2 * fdoh) ||
-        !encode_planes(&c->maps.plain, c->state.p, L.pitch, L.rows, st_planes, kTileX, kTileY) ||
-        !encode_planes(&c->maps.model, c->models.p, L.pitch, L.rows, md_planes, kTileX, kTileY))
-        return;
-    c->maps_v = c->maps;
-    if (kTileYV != kTileY &&
-        (!encode_planes(&c->maps_v.halo, c->state.p, L.pitch, L.rows, st_planes, kTileX + 2 * xh, kTileYV + 2 * fdoh) ||
-         !encode_planes(&c->maps_v.plain, c->state.p, L.pitch, L.rows, st_planes, kTileX, kTileYV) ||
-         !encode_planes(&c->maps_v.model, c->models.p, L.pitch, L.rows, md_planes, kTileX, kTileYV)))
-        return;
+    for (int d = 1; d <= 3 * kPipeMaxL; d++)
+        if ((d <= 3 && !encode_planes(&c->tmaps[MAP_HALO][d], c->state.p, L.pitch, L.rows, st_planes, kTileX + 2 * xh,
+                                      kTileY + 2 * fdoh, d)) ||
+            !encode_planes(&c->tmaps[MAP_PLAIN][d], c->state.p, L.pitch, L.rows, st_planes, kTileX, kTileY, d) ||
+            (d <= 6 && !encode_planes(&c->tmaps[MAP_MODEL][d], c->models.p, L.pitch, L.rows, md_planes, kTileX, kTileY, d)))
+            return;
     // fp32 snapshots are written by the stencil kernels themselves
     t.snap_ntd = c->p.nt / c->p.dtinv;
     t.snap_ncomp = c->ncomp;
@@ -356,6 +361,11 @@ extern "C" int ifos_ctx_create(const ifos_params *pp, int device, int with_snaps
     g.pitch = (int)L.pitch;
     g.plane = L.plane;
     g.fw = p.fw;
+    g.psx = L.psx;
+    g.psy = L.psy;
+    g.psx_lw = L.psx_lw;
+    g.psx_rs = L.psx_rs;
+    g.psx_roff = L.psx_lw + p.nx - 2 * p.fw - L.psx_rs;
     g.free_surf = p.free_surf;
     g.boundary = p.boundary;
     g.fdoh = p.fdorder / 2;
@@ -448,7 +458,13 @@ extern "C" int ifos_ctx_create(const ifos_params *pp, int device, int with_snaps
     if ((rc = dev_alloc(c, c->psi, (size_t)S * L.psi_slot * e + e))) return bail(rc);
     c->model_stride = L.model_elems;
     if ((rc = dev_alloc(c, c->models, (size_t)p.max_models * L.model_elems * e))) return bail(rc);
-    if ((rc = dev_alloc(c, c->prof, (size_t)12 * (2 * p.fw + 1) * e))) return bail(rc);
+    c->profx_off = (12LL * (2 * p.fw + 1) + 3) / 4 * 4;
+    long long prof_len = c->profx_off + 6LL * L.psy;
+    if (p.fw > 0 && L.psx <= kProfX && 2 * p.fw + 1 <= kProfY) {
+        c->proftab_off = prof_len;
+        prof_len += 6 * (kProfX + kProfY);
+    }
+    if ((rc = dev_alloc(c, c->prof, (size_t)prof_len * e))) return bail(rc);
     if ((rc = dev_alloc(c, c->srf, (size_t)p.max_models * 4 * p.nx * e))) return bail(rc);
     if ((rc = dev_alloc(c, c->slot_model, (size_t)S * sizeof(int)))) return bail(rc);
     const int ms = std::max(1, p.max_src), mr = std::max(1, p.max_rec);
@@ -488,13 +504,38 @@ extern "C" int ifos_ctx_create(const ifos_params *pp, int device, int with_snaps
     // CPML profiles
     CpmlProfiles pr = cpml_profiles(p);
     {
-        std::vector<char> hb((size_t)12 * (2 * p.fw + 1) * e);
+        std::vector<char> hb((size_t)prof_len * e, 0);
         for (int a = 0; a < 12; a++)
             for (int h = 0; h <= 2 * p.fw; h++) {
                 size_t idx = (size_t)a * (2 * p.fw + 1) + h;
                 if (c->dbl) ((double *)hb.data())[idx] = pr.arr[a][h];
                 else ((float *)hb.data())[idx] = pr.arr[a][h];
             }
+        // the x profiles by grid column: K a b at the full points, then at the half points
+        for (int a = 0; a < 6; a++)
+            for (int i = 1; i <= L.psy; i++) {
+                const int h = i <= p.fw ? i : (i >= p.nx - p.fw + 1 && i <= p.nx ? i - p.nx + 2 * p.fw : 0);
+                const float v = h ? pr.arr[a][h] : (a % 3 == 0 ? 1.0f : 0.0f);
+                const size_t idx = (size_t)(c->profx_off + (long long)a * L.psy + i - 1);
+                if (c->dbl) ((double *)hb.data())[idx] = v;
+                else ((float *)hb.data())[idx] = v;
+            }
+        if (c->proftab_off) {
+            auto at = [&](long long idx) -> float {
+                return c->dbl ? (float)((double *)hb.data())[idx] : ((float *)hb.data())[idx];
+            };
+            auto set = [&](long long idx, float v) {
+                if (c->dbl) ((double *)hb.data())[idx] = v;
+                else ((float *)hb.data())[idx] = v;
+            };
+            for (int a = 0; a < 6; a++) {
+                for (int k = 0; k < L.psx; k++)
+                    set(c->proftab_off + a * kProfX + k,
+                        at(c->profx_off + (long long)a * L.psy + (k < L.psx_lw ? k : L.psx_rs + k - L.psx_lw)));
+                for (int h = 0; h <= 2 * p.fw; h++)
+                    set(c->proftab_off + 6 * kProfX + a * kProfY + h, pr.arr[6 + a][h]);
+            }
+        }
         CK(cudaMemcpyAsync(c->prof.p, hb.data(), hb.size(), cudaMemcpyHostToDevice, c->st));
         // exact shortcuts of the kernels: d/K with K == 1 everywhere, x/DH with DH a power of two
         g.k_one = 1;
@@ -503,7 +544,11 @@ extern "C" int ifos_ctx_create(const ifos_params *pp, int device, int with_snaps
                 if (pr.arr[a][h] != 1.0) g.k_one = 0;
         int ex = 0;
         g.dh_pow2 = std::frexp(p.dh, &ex) == 0.5f ? 1 : 0;
-        g.inv_dh = g.dh_pow2 ? 1.0f / p.dh : 0.0f;
+        g.inv_dh = 1.0f / p.dh;
+        // the reciprocal form of x/DH needs exact remainders: far from underflow and overflow
+        const bool ok = p.dh > 0x1p-20f && p.dh < 0x1p20f;
+        g.div_lo = ok ? 0x1p-100f : INFINITY;
+        g.div_hi = 0x1p100f;
     }
     // model plane table
     for (int m = 0; m < NM_PLANE; m++) {
@@ -709,7 +754,7 @@ static bool any_force_source(const ifos_ctx *c, int nshots) {
 
 // error codes >= 16 in the status word come from a bounded barrier wait of a
 // pipelined kernel that gave up (16/17: a consumer on a stage's loads, 18: the
-// producer on a stage's release)
+// producer on a stage's release; 19: a consumer on a batch of tile indices)
 static int pipeline_timeout(ifos_ctx *c, int code) {
     return fail(c, IFOS_ERR_CUDA, "pipelined stencil kernel: barrier wait timed out (code " + std::to_string(code) + ")");
 }

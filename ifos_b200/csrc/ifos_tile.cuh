@@ -7,18 +7,16 @@
 // the velocity update, the velocities in the stress update) as tile + halo
 // boxes, the per-cell planes (fields, memory variables, coefficients) as
 // plain tile boxes.  The compute warps release a stage as soon as they have
-// read it and write their results straight to HBM with 8-byte stores (on
+// read it and write their results straight to HBM with vector stores (on
 // snapshot steps also the stored wavefield components, into the snapshot
 // buffer), so the ring only ever waits on loads.
 //
-// A thread owns two adjacent columns (float2 shared-memory accesses) of the
-// RT = TY / (compute warps) consecutive rows of its warp: the x-taps of both
-// columns come from one aligned window, the y-taps of neighbouring rows from
-// the same words, and the cells of a thread are independent work.  Interior
-// tiles (no CPML strip cell) take a path without strip code.  The per-cell
-// arithmetic is the reference's, in the same order and with the same
-// float/double promotions as the one-thread-per-cell kernels of
-// ifos_kernels.cuh.
+// A thread owns four adjacent cells of one row and a warp two rows of the
+// tile, or two cells and one row (Pipe's V).  Warps whose rows need nothing but the plain update (no CPML strip cell, no
+// free surface, receiver, source or ragged edge) take a path without any of
+// that code.  The per-cell arithmetic is the reference's, in the same order
+// and with the same float/double promotions as the one-thread-per-cell
+// kernels of ifos_kernels.cuh.
 #pragma once
 #include <type_traits>
 
@@ -32,37 +30,29 @@
 #define IFOS_EXACT 1
 #endif
 
-// compute warps per block (the block adds one producer warp)
-#ifndef IFOS_NCW
-#define IFOS_NCW 8
-#endif
-
 namespace ifos {
 
-constexpr int kComputeWarps = IFOS_NCW;
-// Resident blocks per SM the elastic stress op's launch bounds aim for: four
-// for FDORDER <= 4 (400 x 160 batch of 128: 100-105 vs 109 us per launch),
-// three otherwise.
-constexpr int sblocks(int fdoh) {
-#ifdef IFOS_SBLOCKS
-    return IFOS_SBLOCKS + 0 * fdoh;
-#else
-    return fdoh <= 2 ? 4 : 3;
-#endif
-}
-// Resident blocks per SM the velocity ops' launch bounds aim for.  Four
-// (registers capped at 56, two ring stages) were faster for FDORDER <= 4
-// (400 x 160 batch of 128: 94 vs 103 us per launch), three for the wider
-// stencils (2000 x 600, FDORDER 8, one shot: 22.3 vs 24.6 us).
-constexpr int vblocks(int fdoh) {
-#ifdef IFOS_VBLOCKS
-    return IFOS_VBLOCKS + 0 * fdoh;
-#else
-    return fdoh <= 2 ? 4 : 3;
-#endif
-}
-constexpr int kBlockThreads = 32 * kComputeWarps + 32;
+// Resident blocks per SM that the launch bounds and the ring are sized for.
+// More blocks cap the registers and spill: 64 shots of 400 x 160 at FDORDER 4
+// with 4, 5 and 6 blocks: velocity 47, 51 and 54 us, stress 46, 52 and 51;
+// 4000 x 1200 at FDORDER 8 with 3, 5 and 6: velocity 53, 56 and 57, stress 46,
+// 49 and 53.  The viscoelastic stress fills the shared memory with two blocks
+// of two 46 KB stages; three or four blocks of one stage were slower (2000 x
+// 600: 42 us against 46 and 52).
+constexpr int sblocks(int fdoh) { return fdoh <= 2 ? 4 : 3; }
+constexpr int vblocks(int fdoh) { return fdoh <= 2 ? 4 : 3; }
+constexpr int visc_blocks(int LL) { return LL <= 1 ? 3 : 2; }
 constexpr int kTileX = 64;
+// Cells per thread.  Four halve the loads, addresses and bookkeeping per cell;
+// two leave room for twice the warps.  Four win where instructions bound the
+// op (64 shots of 400 x 160, FDORDER 4: velocity 48 against 54 us, stress 48
+// against 60; 4000 x 1200, FDORDER 8: elastic stress 47.2 against 48.7, SH
+// 28.7 against 30.8), two in the viscoelastic stress, whose four cells need
+// 168 registers (6 shots of 2000 x 600: 177 against 185 us; 3000 x 1000: 76
+// against 82), and in the P-SV velocity of the wide stencils (4000 x 1200,
+// FDORDER 8: 47.1 against 49.8).
+constexpr int kCells = 4, kCellsVisc = 2;
+constexpr int cells_v(int fdoh) { return fdoh <= 2 ? 4 : 2; }
 
 using D = std::conditional<IFOS_EXACT != 0, double, float>::type;
 
@@ -79,10 +69,13 @@ struct KTma {
     int snap_comp[NP_FIELD];  // component index of a state plane (-1: not stored)
 };
 
+// The tensor maps of a launch: the halo planes of a tile are one box of NH_
+// consecutive state planes, the per-cell planes up to five boxes of
+// consecutive state or model planes each (Op::GD, Op::GM).
+constexpr int kMaxGroups = 5;
 struct KMaps {
-    CUtensorMap halo;   // state planes, box (64+2XH) x (TY+2H)
-    CUtensorMap plain;  // state planes, box 64 x TY (loads and stores)
-    CUtensorMap model;  // model planes, box 64 x TY
+    CUtensorMap halo;             // state planes, box (64+2XH) x (TY+2H) x NH_
+    CUtensorMap grp[kMaxGroups];  // state or model planes, box 64 x TY x GD[k]
 };
 
 // fp32 snapshot written by a launch: snapshot of slot 0 being stored (NULL:
@@ -93,39 +86,51 @@ struct KSnapOut {
     char *base;            // this snapshot of slot 0
     long long slot_bytes;  // bytes between slots
     long long n;           // NX*NY
-    int pairs;             // NX even: column pairs are aligned for vector stores
+    int align;             // 4, 2 or 1: cells of a row that are aligned for vector stores (by NX)
     int f16;               // fp16 segments (IFOS_SNAP_F16S); else fp32
     long long ex_off;      // fp16: bytes from a snapshot to its segment scales [comp][NY][segs]
     int segs;              // fp16: segments per row
 };
 
 // NH halo boxes, NP loaded plain boxes, NO output-only plain boxes, NST stages
-template <int FDOH, int TY, int NH, int NP, int NO, int NST, int BCAP = 3>
+// V cells per thread: 4 (a compute warp takes two tile rows) or 2 (one row)
+template <int FDOH, int TY, int NH, int NP, int NO, int NST, int BCAP = 3, int V = 4>
 struct Pipe {
+    static constexpr int ROWS = V / 2;                // tile rows of a compute warp
+    static constexpr int NCW = TY / ROWS;             // compute warps; the block adds one producer warp
+    static constexpr int THREADS = 32 * NCW + 32;
     static constexpr int TX = kTileX, H = FDOH;
-    static constexpr int HE = (FDOH + 1) & ~1;       // x window half width (even)
     static constexpr int XH = ((FDOH + 3) / 4) * 4;  // staged x halo (16-byte TMA alignment)
     static constexpr int BW = TX + 2 * XH, BH = TY + 2 * H;
-    static constexpr int BOXS = ((BW * BH * 4 + 127) / 128) * 32;  // 128-byte aligned box stride
+    static constexpr int BOXS = BW * BH;                        // a plane of the halo box
+    static constexpr int HALO = (NH * BOXS + 31) / 32 * 32;     // the halo box, 128-byte aligned
     static constexpr int PLS = TX * TY;
     static constexpr int NHALO = NH, NLOAD = NP, NPL = NP + NO, STAGES = NST;
-    static constexpr int STAGE = NH * BOXS + NPL * PLS;
-    static constexpr int RT = TY / kComputeWarps;  // rows per thread
+    static constexpr int STAGE = HALO + NPL * PLS;
     static constexpr int TILE_Y = TY;
     static constexpr uint32_t TXB = (uint32_t)((NH * BW * BH + NP * PLS) * 4);
     static constexpr size_t bytes() { return (size_t)NST * STAGE * 4; }
     static constexpr int BLOCK_CAP = BCAP;  // resident blocks per SM the launch bounds aim for
-    static_assert(TY % kComputeWarps == 0, "tile height must be a multiple of the compute warps");
-    static_assert(HE <= XH, "x window exceeds the staged halo");
+    static_assert((V == 4 || V == 2) && TY % ROWS == 0 && NCW <= 8, "tile rows and compute warps");
 };
 
 // One tile as the producer hands it to the compute warps.
 struct __align__(16) TileInfo {
     int slot, i0, j0;
-    int model;   // model index of the slot
-    int ystrip;  // some row of the tile lies in a CPML y strip
-    int pad[3];
+    int bits;  // model index of the slot * 256, + bit w: the rows of compute warp w need more than the plain update
+    __device__ __forceinline__ int model() const { return bits >> 8; }
+    __device__ __forceinline__ bool edge(int w) const { return (bits >> w) & 1; }
 };
+
+// a / b and the remainder for 0 <= a < 2^24, rb = 1/b: the float quotient is
+// off by at most one
+__device__ __forceinline__ int div_small(int a, int b, float rb, int &rem) {
+    int q = (int)((float)a * rb);
+    rem = a - q * b;
+    if (rem < 0) q--, rem += b;
+    if (rem >= b) q++, rem -= b;
+    return q;
+}
 
 // Tile t of a launch.  Slot-major order walks all tiles of slot 0, then of
 // slot 1, ...; slot-minor order gives consecutive t the same tile of
@@ -140,153 +145,235 @@ struct __align__(16) TileInfo {
 // over the persistent CTAs hands each CTA the same number of them (within
 // one), so the CTAs finish together instead of the ones that drew the strip
 // columns finishing last.  A bijection on [0, ntx*nty).
-__device__ __forceinline__ int cpml_first(int rank, int ntx, int nty, int TY, const KGrid &g) {
-    if (g.fw <= 0) return rank;
-    const int cl = min(ntx, (g.fw - 1) / kTileX + 1);  // tile columns with i0 <= FW
-    const int vx = g.nx - g.fw + 1 - kTileX;            // right strip: min(i0+63, NX) >= NX-FW+1
-    const int xr0 = max(cl, vx <= 0 ? 0 : (vx + kTileX - 1) / kTileX);
-    const int rt = g.free_surf ? 0 : min(nty, (g.fw - 1) / TY + 1);  // tile rows with j0 <= FW
-    const int vy = g.ny - g.fw + 1 - TY;                              // bottom strip: j0+TY-1 >= NY-FW+1
-    const int yb0 = min(nty, max(rt, vy <= 0 ? 0 : (vy + TY - 1) / TY));
-    const int nys = rt + (nty - yb0);  // rows in a y strip
-    if (rank < nys * ntx) {
-        const int r = rank / ntx;
-        return (r < rt ? r : yb0 + (r - rt)) * ntx + (rank - r * ntx);
+struct TileWalk {
+    int ntx, nty, nshots, ntiles;
+    float r_ntx, r_shots, r_per;
+    // CPML-first regions: rows in a top y strip, first row of the bottom one,
+    // rows in y strips; left x-strip columns, first right one, x-strip columns
+    int rt, yb0, nys, cl, xr0, ce;
+    float r_ce, r_w;
+    __device__ __forceinline__ TileWalk(const KGrid &g, int TY, int shots) {
+        ntx = (g.nx + kTileX - 1) / kTileX, nty = (g.ny + TY - 1) / TY;
+        nshots = shots, ntiles = ntx * nty * shots;
+        r_ntx = 1.0f / ntx, r_shots = 1.0f / shots, r_per = 1.0f / (ntx * nty);
+        cl = min(ntx, (g.fw - 1) / kTileX + 1);  // tile columns with i0 <= FW
+        const int vx = g.nx - g.fw + 1 - kTileX;  // right strip: min(i0+63, NX) >= NX-FW+1
+        xr0 = max(cl, vx <= 0 ? 0 : (vx + kTileX - 1) / kTileX);
+        rt = g.free_surf ? 0 : min(nty, (g.fw - 1) / TY + 1);  // tile rows with j0 <= FW
+        const int vy = g.ny - g.fw + 1 - TY;                   // bottom strip: j0+TY-1 >= NY-FW+1
+        yb0 = min(nty, max(rt, vy <= 0 ? 0 : (vy + TY - 1) / TY));
+        nys = rt + (nty - yb0);
+        ce = cl + (ntx - xr0);
+        r_ce = 1.0f / ce, r_w = 1.0f / (ntx - ce);
     }
-    rank -= nys * ntx;
-    const int ce = cl + (ntx - xr0);  // x-strip columns
-    const int mid = nty - nys;        // rows between the y strips: rt .. yb0-1
-    if (rank < mid * ce) {
-        const int r = rank / ce, c = rank - r * ce;
-        return (rt + r) * ntx + (c < cl ? c : xr0 + (c - cl));
+    // tile row and column of a spatial rank in CPML-first order
+    __device__ __forceinline__ int first(int rank, int &tx) const {
+        if (rank < nys * ntx) {
+            const int r = div_small(rank, ntx, r_ntx, tx);
+            return r < rt ? r : yb0 + (r - rt);
+        }
+        rank -= nys * ntx;
+        const int mid = nty - nys;  // rows between the y strips: rt .. yb0-1
+        int c;
+        if (rank < mid * ce) {
+            const int r = div_small(rank, ce, r_ce, c);
+            tx = c < cl ? c : xr0 + (c - cl);
+            return rt + r;
+        }
+        rank -= mid * ce;
+        const int r = div_small(rank, ntx - ce, r_w, c);  // ce < ntx here: the regions above hold every tile when it is not
+        tx = cl + c;
+        return rt + r;
     }
-    rank -= mid * ce;
-    const int w = ntx - ce;  // > 0 here: the regions above hold every tile when it is 0
-    const int r = rank / w;
-    return (rt + r) * ntx + cl + (rank - r * w);
-}
-
-__device__ __forceinline__ void tile_of(int t, int ntx, int nty, int TY, int nshots, int order, const KGrid &g,
-                                        TileInfo &r) {
-    int rem;
-    if (order & 1) {
-        rem = t / nshots;
-        r.slot = t - rem * nshots;
-    } else {
-        const int per = ntx * nty;
-        r.slot = t / per;
-        rem = t - r.slot * per;
+    __device__ __forceinline__ void tile(int t, int TY, int order, int fw, TileInfo &r) const {
+        int rem, tx;
+        if (nshots == 1) r.slot = 0, rem = t;
+        else if (order & 1) rem = div_small(t, nshots, r_shots, r.slot);
+        else r.slot = div_small(t, ntx * nty, r_per, rem);
+        const int ty = (order & 2) && fw > 0 ? first(rem, tx) : div_small(rem, ntx, r_ntx, tx);
+        r.i0 = tx * kTileX + 1;
+        r.j0 = ty * TY + 1;
     }
-    if (order & 2) rem = cpml_first(rem, ntx, nty, TY, g);
-    const int tyi = rem / ntx;
-    r.i0 = (rem - tyi * ntx) * kTileX + 1;
-    r.j0 = tyi * TY + 1;
-}
-
-// rows j0 .. j0+TY-1 meet a y strip (top: j <= FW without free surface,
-// bottom: j >= NY-FW+1)
-__device__ __forceinline__ int tile_in_ystrip(const KGrid &g, int j0, int TY) {
-    if (g.fw == 0) return 0;
-    if (!g.free_surf && j0 <= g.fw) return 1;
-    return j0 + TY - 1 >= g.ny - g.fw + 1 ? 1 : 0;
-}
-
-// source of a plain-box load: a state plane or a model plane
-struct PlainSrc {
-    int z;
-    bool model;
 };
 
-// Warp-specialised persistent driver.  Warps 0..kComputeWarps-1 compute; lane
-// 0 of the last warp produces: it walks the same tile sequence, waits until a
-// stage has been released by all compute warps ("empty" barrier, one arrival
-// per warp), and issues the bulk tensor loads of the next tile into it
-// ("full" barrier, completed by the transaction bytes).  The tile's indices
-// travel through shared memory with the stage.  Every wait is bounded: a
-// wait that gives up records its code in *err (16/17: a compute warp on a
-// stage's loads, 18: the producer on a stage's release) and the block winds
-// down after its copies in flight: when the producer gives up before tile
-// k_stop it records k_stop (stop_at) and issues nothing more; the compute
-// warps still wait for every tile it issued (so that no copy into the ring is
-// in flight when the block exits), compute none of them, and leave at k_stop.
+// Compute warps of a tile whose rows need more than the plain update of whole
+// rows: a CPML strip, the imaged rows of the free surface (velocity), the
+// surface itself, a source, receiver or probe row, or cells outside the grid.
+template <typename Op>
+__device__ __forceinline__ int edge_warps(const Op &op, const TileInfo &ti) {
+    const KGrid &g = op.g;
+    using P = typename Op::P;
+    constexpr int all = (1 << P::NCW) - 1;
+    const bool strips = Op::CPML && g.fw > 0;
+    if (ti.i0 + kTileX - 1 > g.nx || (Op::MIRROR && g.free_surf && ti.j0 == 1)) return all;
+    if (strips && !g.boundary && (ti.i0 <= g.fw || ti.i0 + kTileX - 1 >= g.nx - g.fw + 1)) return all;
+    int m = 0;
+#pragma unroll
+    for (int w = 0; w < P::NCW; w++) {
+        const int a = ti.j0 + P::ROWS * w, b = a + P::ROWS - 1;
+        bool e = b > g.ny || (strips && ((!g.free_surf && a <= g.fw) || b >= g.ny - g.fw + 1));
+        e = e || (op.rec_mode && a <= op.rec_j1 && b >= op.rec_j0);
+        e = e || (op.rec_mode == 1 && (a == g.ny / 2 || b == g.ny / 2));
+        e = e || (op.fps && a <= op.src_j1 && b >= op.src_j0) || (op.fsurf && a == 1);
+        m |= e ? 1 << w : 0;
+    }
+    return m;
+}
+
+// The profiles a block reads: in shared memory (staged once per block) when
+// the strips are no wider than kProfX columns and kProfY rows, else the global
+// tables.  Read from global memory the four profiles of a strip cell were four
+// L2 round trips one after another, 2000 of the 3000 cycles of a strip tile.
+struct ProfTab {
+    const float *x, *y;  // K a b at the full points, K a b at the half points
+    int xs, ys;          // values between two of them
+    bool local;          // x is indexed by the column of a strip row, else by the grid column
+};
+// Tiles whose indices the producer warp works out at a time, one per lane.
+constexpr int kTileBatch = 32;
+
+// Warp-specialised persistent driver.  Warps 0..NCW-1 compute; the
+// last warp produces: it walks the same tile sequence, waits until a stage
+// has been released by all compute warps ("empty" barrier, one arrival per
+// warp), and issues the bulk tensor loads of the next tile into it ("full"
+// barrier, completed by the transaction bytes).  The indices of 32 tiles at a
+// time are worked out by the 32 lanes into shared memory (tq), ahead of their
+// loads; a compute warp may read those of its next tile as soon as the
+// batch's barrier has completed, and starts the loads that its CPML needs
+// (Op::prefetch) before it waits for the stage.  One lane working out one tile
+// after another took 1700-2300 cycles a tile, more than the update itself
+// (4000 x 1200, FDORDER 8: 900-1900), and held back the first loads of every
+// launch by 2 us.  The planes of a tile arrive as a few boxes of consecutive
+// planes (about 100 cycles of issue per box).
+//
+// Every wait is bounded: a wait that gives up records its code in *err (16/17:
+// a compute warp on a stage's loads, 18: the producer on a stage's release,
+// 19: a compute warp on a batch of tile indices) and the block winds down
+// after its copies in flight: when the producer gives up before tile k_stop it
+// records k_stop (stop_at) and issues nothing more; the compute warps still
+// wait for every tile it issued (so that no copy into the ring is in flight
+// when the block exits), compute none of them, and leave at k_stop.
 template <typename P, typename Op>
 __device__ __forceinline__ void run_pipeline(const KGrid &g, const KMaps &mp, int nshots, const Op &op, int *err) {
-    constexpr int NST = P::STAGES, NH = P::NHALO, NP = P::NLOAD, TY = P::TILE_Y;
+    constexpr int NST = P::STAGES, TY = P::TILE_Y;
     extern __shared__ __align__(1024) unsigned char sm_raw[];
-    __shared__ __align__(8) uint64_t full[NST], empty[NST];
-    __shared__ TileInfo tinfo[NST];
+    __shared__ __align__(8) uint64_t full[NST], empty[NST], filled;
+    __shared__ TileInfo tq[2 * kTileBatch];
+    __shared__ __align__(16) float sprof[Op::CPML ? 6 * (kProfX + kProfY) : 4];
     __shared__ int stop_at;  // -1 while the producer runs, else the first tile it did not issue
     float *smem = reinterpret_cast<float *>(sm_raw);
-    const int ntx = (g.nx + kTileX - 1) / kTileX, nty = (g.ny + TY - 1) / TY;
-    const int ntiles = ntx * nty * nshots;
-    const int warp = threadIdx.y;
-    if (warp == kComputeWarps && threadIdx.x == 0) {
+    const int ntiles = ((g.nx + kTileX - 1) / kTileX) * ((g.ny + TY - 1) / TY) * nshots;
+    const int warp = threadIdx.y, lane = threadIdx.x;
+    if (warp == P::NCW && lane == 0) {
         for (int s = 0; s < NST; s++) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], kComputeWarps);
+            mbar_init(&empty[s], P::NCW);
         }
+        mbar_init(&filled, 1);
         stop_at = -1;
         fence_mbar_init();
     }
     __syncthreads();
-    if (warp == kComputeWarps) {
-        if (threadIdx.x != 0) return;
-        // Tile k in stage k % NST.  The per-cell planes of the first NST tiles
-        // are not written by the preceding kernel of the stream, so they are
-        // requested before waiting for it; everything else after.
-        auto issue = [&](int k, bool halo, bool plain) {
-            const int st = k % NST;
-            TileInfo ti;
-            tile_of(blockIdx.x + k * gridDim.x, ntx, nty, TY, nshots, g.tile_order, g, ti);
+    volatile int *stop = &stop_at;
+    if (warp == P::NCW) {
+        // tiles k0 .. k0+31 of this block; the entries they replace belong to
+        // tiles the compute warps have left (they are at most NST behind)
+        const TileWalk walk(g, TY, nshots);
+        auto fill = [&](int k0) {
+            const int k = k0 + lane, t = blockIdx.x + k * gridDim.x;
+            if (t < ntiles) {
+                TileInfo ti;
+                walk.tile(t, TY, g.tile_order, g.fw, ti);
+                ti.bits = (op.M.one_model ? 0 : op.M.slot_model[ti.slot] * 256) + edge_warps(op, ti);
+                tq[k % (2 * kTileBatch)] = ti;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&filled);
+        };
+        auto issue = [&](int k, int st, bool halo, bool plain) {
+            const TileInfo ti = tq[k % (2 * kTileBatch)];
             float *stage = smem + st * P::STAGE;
             uint64_t *bar = &full[st];
-            if (plain) {
-                ti.model = op.M.slot_model[ti.slot];
-                ti.ystrip = tile_in_ystrip(g, ti.j0, TY);
-                tinfo[st] = ti;
-                mbar_expect_tx(bar, P::TXB);
-            } else {
-                ti.model = tinfo[st].model;
-            }
-            int hz[NH > 0 ? NH : 1];
-            PlainSrc pz[NP > 0 ? NP : 1];
-            op.planes(ti, hz, pz);
-            if (halo) {
-                const int bx = HX + ti.i0 - 1 - P::XH, by = HY + ti.j0 - 1 - P::H;
-#pragma unroll
-                for (int h = 0; h < NH; h++) tma_load_3d(stage + h * P::BOXS, &mp.halo, bx, by, hz[h], bar);
-            }
+            int hz, gz[Op::NG];
+            op.planes(ti, hz, gz);
+            if (plain) mbar_expect_tx(bar, P::TXB);
+            if (halo)
+                tma_load_3d(stage, &mp.halo, HX + ti.i0 - 1 - P::XH, HY + ti.j0 - 1 - P::H, hz, bar);
             if (plain) {
                 const int px = HX + ti.i0 - 1, py = HY + ti.j0 - 1;
+                int q = 0;
 #pragma unroll
-                for (int q = 0; q < NP; q++)
-                    tma_load_3d(stage + NH * P::BOXS + q * P::PLS, pz[q].model ? &mp.model : &mp.plain, px, py,
-                                pz[q].z, bar);
+                for (int k = 0; k < Op::NG; k++) {
+                    tma_load_3d(stage + P::HALO + q * P::PLS, &mp.grp[k], px, py, gz[k], bar);
+                    q += Op::gd(k);
+                }
             }
         };
+        fill(0);
+        // The per-cell planes of the first NST tiles are not written by the
+        // preceding kernel of the stream, so they are requested before
+        // waiting for it; everything else after.
         int npre = 0;
-        while (npre < NST && blockIdx.x + npre * gridDim.x < ntiles) issue(npre++, false, true);
-        pdl_wait();
-        for (int k = 0; k < npre; k++) issue(k, true, false);
-        pdl_launch();
-        for (int k = npre;; k++) {
-            const int t = blockIdx.x + k * gridDim.x;
-            if (t >= ntiles) break;
-            const int st = k % NST;
-            if (!mbar_wait_bounded(&empty[st], (uint32_t)(((k / NST) - 1) & 1), err, 18, (long)g.prod_polls)) {
-                *(volatile int *)&stop_at = k;
-                break;
-            }
-            issue(k, true, true);
+        if (lane == 0) {
+            for (; npre < NST && blockIdx.x + npre * gridDim.x < ntiles; npre++) issue(npre, npre, false, true);
+            pdl_wait();
+            for (int k = 0; k < npre; k++) issue(k, k, true, false);
         }
+        npre = __shfl_sync(0xffffffffu, npre, 0);
+        int st = 0;
+        uint32_t parity = 0;
+        for (int k = npre, t = blockIdx.x + k * gridDim.x; t < ntiles; k++, t += gridDim.x) {
+            if (k % kTileBatch == 0) {
+                __syncwarp();
+                if (*stop >= 0) break;
+                fill(k);
+            }
+            if (lane == 0 && *stop < 0) {
+                if (mbar_wait_bounded(&empty[st], parity, err, 18, (long)g.prod_polls)) issue(k, st, true, true);
+                else *stop = k;
+            }
+            if (++st == NST) {
+                st = 0;
+                parity ^= 1;
+            }
+        }
+        // Only now may the next kernel's blocks start: they then find this
+        // launch's blocks leaving and spread evenly over the SMs.  Released
+        // after the first tiles they took the slots of the blocks that left
+        // first and the SMs ended with two to four of them (4000 x 1200: 54
+        // instead of 36 us a block).
+        pdl_launch();
         return;
     }
-    volatile int *stop = &stop_at;
-    for (int k = 0;; k++) {
-        const int t = blockIdx.x + k * gridDim.x;
-        if (t >= ntiles) break;
-        const int st = k % NST;
-        const uint32_t parity = (uint32_t)((k / NST) & 1);
+    ProfTab pt{op.M.profx, op.M.prof + 6 * (2 * g.fw + 1), g.psy, 2 * g.fw + 1, false};
+    if (Op::CPML && op.M.proftab) {
+        constexpr int n = 6 * (kProfX + kProfY) / 4;
+        for (int k = warp * 32 + lane; k < n; k += 32 * P::NCW)
+            reinterpret_cast<float4 *>(sprof)[k] = reinterpret_cast<const float4 *>(op.M.proftab)[k];
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * P::NCW) : "memory");
+        pt = ProfTab{sprof, sprof + 6 * kProfX, kProfX, kProfY, true};
+    }
+    int st = -1;
+    uint32_t parity = 1;
+    for (int k = 0, t = blockIdx.x; t < ntiles; k++, t += gridDim.x) {
+        st = st + 1 == NST ? 0 : st + 1;
+        if (st == 0) parity ^= 1;
+        if (k % kTileBatch == 0) {
+            bool ready = false;
+            for (long it = 0; it < (1L << 16) && !ready; it++) {
+                ready = mbar_try_wait(&filled, (uint32_t)(k / kTileBatch) & 1);
+                if (!ready && *stop >= 0 && k >= *stop) return;  // never filled
+            }
+            if (!ready) {
+                if (err) atomicExch(err, 19);
+                mbar_wait_bounded(&full[st], parity, err, 17);
+                return;
+            }
+        }
+        const TileInfo ti = tq[k % (2 * kTileBatch)];
+        const bool edge = ti.edge(warp);
+        typename Op::Pre pre;
+        if (edge) op.prefetch(ti, pre);
         bool landed = false;
         for (long it = 0; it < (1L << 16) && !landed; it++) {
             landed = mbar_try_wait(&full[st], parity);
@@ -298,22 +385,21 @@ __device__ __forceinline__ void run_pipeline(const KGrid &g, const KMaps &mp, in
             return;
         }
         if (*stop >= 0) continue;  // the producer stopped: drain the tiles it issued, compute none
-        const TileInfo ti = tinfo[st];
         const float *stage = smem + st * P::STAGE;
-        op.compute(ti, stage, stage + NH * P::BOXS, &empty[st]);
+        if (edge) op.template rows<true>(ti, pre, pt, stage, stage + P::HALO, &empty[st]);
+        else op.template rows<false>(ti, pre, pt, stage, stage + P::HALO, &empty[st]);
     }
 }
 
 // ---------------------------------------------------------------------------
-// Difference stencils of a thread's column pair (cells e = 0, 1 at staged
-// columns c0 + e).  The m=1 term starts each sum and the others are added in
-// order, as in the reference's written-out expressions
-// (src/update_v_PML.c:164-175); Z0: the sum is accumulated from zero, as in
-// its generic loops (the FDORDER 10/12 default branches, e.g.
-// src/update_p_PML.c:275-287).  fwd: sum_m w_m (f[+m] - f[-m+1]);
-// bwd: sum_m w_m (f[+m-1] - f[-m]).
+// A thread owns four adjacent cells of one row (16-byte shared-memory reads
+// and global stores): 16 lanes cover a tile row, a warp two rows.  Against a
+// column pair per thread this halves the loads, the address arithmetic and
+// the per-row bookkeeping of a cell; the stencils were bound by instruction
+// issue, not by HBM (400 x 160, 64 shots, FDORDER 4: 263 instructions a cell
+// in the velocity update with DRAM at 25 % of its peak).
 
-// FD weights of one launch, in registers
+// FD weights of one launch
 template <int FDOH>
 struct Hc {
     float w[FDOH + 1];
@@ -323,176 +409,324 @@ struct Hc {
     }
 };
 
-// staged values of one row at columns c0-HE .. c0+HE+1 (c0 - HE even)
-template <int HE>
+// V adjacent cells
+template <int V>
+struct FV {
+    float v[V];
+    __device__ __forceinline__ static FV of(float x) {
+        FV r;
+#pragma unroll
+        for (int e = 0; e < V; e++) r.v[e] = x;
+        return r;
+    }
+};
+template <int V>
+__device__ __forceinline__ FV<V> ldv(const float *p) {
+    if constexpr (V == 4) {
+        const float4 a = *reinterpret_cast<const float4 *>(p);
+        return {{a.x, a.y, a.z, a.w}};
+    } else {
+        const float2 a = *reinterpret_cast<const float2 *>(p);
+        return {{a.x, a.y}};
+    }
+}
+template <int V>
+__device__ __forceinline__ void stv(float *p, const float (&v)[V]) {
+    if constexpr (V == 4) *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+}
+
+// Difference stencils of a thread's four cells.  The m=1 term starts each sum
+// and the others are added in order, as in the reference's written-out
+// expressions (src/update_v_PML.c:164-175); Z0: the sum is accumulated from
+// zero, as in its generic loops (the FDORDER 10/12 default branches, e.g.
+// src/update_p_PML.c:275-287).  fwd: sum_m w_m (f[+m] - f[-m+1]);
+// bwd: sum_m w_m (f[+m-1] - f[-m]).
+
+// staged values of one row at columns c0-XB .. c0+V-1+XB (c0 a multiple of V)
+template <int FDOH, int V>
 struct XWin {
-    float v[2 * HE + 2];
+    static constexpr int XB = (FDOH + V - 1) / V * V, N = V + 2 * XB;
+    float v[N];
     __device__ __forceinline__ void load(const float *row, int c0) {
 #pragma unroll
-        for (int q = 0; q <= HE; q++) {
-            const float2 a = *reinterpret_cast<const float2 *>(row + c0 - HE + 2 * q);
-            v[2 * q] = a.x;
-            v[2 * q + 1] = a.y;
+        for (int q = 0; q < N / V; q++) {
+            const FV<V> a = ldv<V>(row + c0 - XB + V * q);
+#pragma unroll
+            for (int e = 0; e < V; e++) v[V * q + e] = a.v[e];
         }
     }
 };
-template <int FDOH, int HE, bool Z0 = false>
-__device__ __forceinline__ float xfwd(const Hc<FDOH> &hc, const XWin<HE> &W, int e) {
-    float s = hc.w[1] * (W.v[HE + e + 1] - W.v[HE + e]);
+template <bool Z0 = false, int FDOH, int V>
+__device__ __forceinline__ float xfwd(const Hc<FDOH> &hc, const XWin<FDOH, V> &W, int e) {
+    constexpr int XB = XWin<FDOH, V>::XB;
+    float s = hc.w[1] * (W.v[XB + e + 1] - W.v[XB + e]);
     if (Z0) s = 0.0f + s;
 #pragma unroll
-    for (int m = 2; m <= FDOH; m++) s += hc.w[m] * (W.v[HE + e + m] - W.v[HE + e - m + 1]);
+    for (int m = 2; m <= FDOH; m++) s += hc.w[m] * (W.v[XB + e + m] - W.v[XB + e - m + 1]);
     return s;
 }
-template <int FDOH, int HE, bool Z0 = false>
-__device__ __forceinline__ float xbwd(const Hc<FDOH> &hc, const XWin<HE> &W, int e) {
-    float s = hc.w[1] * (W.v[HE + e] - W.v[HE + e - 1]);
+template <bool Z0 = false, int FDOH, int V>
+__device__ __forceinline__ float xbwd(const Hc<FDOH> &hc, const XWin<FDOH, V> &W, int e) {
+    constexpr int XB = XWin<FDOH, V>::XB;
+    float s = hc.w[1] * (W.v[XB + e] - W.v[XB + e - 1]);
     if (Z0) s = 0.0f + s;
 #pragma unroll
-    for (int m = 2; m <= FDOH; m++) s += hc.w[m] * (W.v[HE + e + m - 1] - W.v[HE + e - m]);
+    for (int m = 2; m <= FDOH; m++) s += hc.w[m] * (W.v[XB + e + m - 1] - W.v[XB + e - m]);
     return s;
 }
 
-// Column pair of a staged halo box at row offset dy from tile row jj.  In the
-// top row of tiles with a free surface (MIR) rows j<=0 read the imaged value
-// the reference's ghost rows hold when the velocity is updated: -f(2-j) for
-// syy, syz, sp (src/surface_elastic_PML.c:59) and -f(1-j) for sxy (:60).
-template <bool MIR, bool ODD, typename P>
-__device__ __forceinline__ float2 ldy2(const float *t, int jj, int c0, int dy) {
+// A thread's cells of a staged halo box at row offset dy from tile row jj.  MIR: the
+// tile is the top one under a free surface, whose rows j<=0 read the imaged
+// value the reference's ghost rows hold when the velocity is updated:
+// -f(2-j) for syy, syz, sp (src/surface_elastic_PML.c:59) and -f(1-j) for sxy
+// (:60).
+template <bool MIR, bool ODD, typename P, int V>
+__device__ __forceinline__ FV<V> ldy(const float *t, int jj, int c0, int dy) {
     const int rr = jj + P::H + dy;
     if (MIR && rr < P::H) {
-        const int src = ODD ? 2 * P::H - rr - 1 : 2 * P::H - rr;
-        const float2 a = *reinterpret_cast<const float2 *>(t + src * P::BW + c0);
-        return make_float2(-a.x, -a.y);
-    }
-    return *reinterpret_cast<const float2 *>(t + rr * P::BW + c0);
-}
-template <bool MIR, bool ODD, typename P, int FDOH, bool Z0 = false>
-__device__ __forceinline__ float2 yfwd2(const Hc<FDOH> &hc, const float *t, int jj, int c0) {
-    float2 a = ldy2<MIR, ODD, P>(t, jj, c0, 1), b = ldy2<MIR, ODD, P>(t, jj, c0, 0);
-    float2 s = make_float2(hc.w[1] * (a.x - b.x), hc.w[1] * (a.y - b.y));
-    if (Z0) s = make_float2(0.0f + s.x, 0.0f + s.y);
+        FV<V> a = ldv<V>(t + (ODD ? 2 * P::H - rr - 1 : 2 * P::H - rr) * P::BW + c0);
 #pragma unroll
-    for (int m = 2; m <= FDOH; m++) {
-        a = ldy2<MIR, ODD, P>(t, jj, c0, m);
-        b = ldy2<MIR, ODD, P>(t, jj, c0, 1 - m);
-        s.x += hc.w[m] * (a.x - b.x);
-        s.y += hc.w[m] * (a.y - b.y);
+        for (int e = 0; e < V; e++) a.v[e] = -a.v[e];
+        return a;
     }
-    return s;
+    return ldv<V>(t + rr * P::BW + c0);
 }
-template <bool MIR, bool ODD, typename P, int FDOH, bool Z0 = false>
-__device__ __forceinline__ float2 ybwd2(const Hc<FDOH> &hc, const float *t, int jj, int c0) {
-    float2 a = ldy2<MIR, ODD, P>(t, jj, c0, 0), b = ldy2<MIR, ODD, P>(t, jj, c0, -1);
-    float2 s = make_float2(hc.w[1] * (a.x - b.x), hc.w[1] * (a.y - b.y));
-    if (Z0) s = make_float2(0.0f + s.x, 0.0f + s.y);
+// FWD: rows +m and 1-m, else m-1 and -m
+template <bool FWD, bool MIR, bool ODD, typename P, bool Z0 = false, int FDOH, int V>
+__device__ __forceinline__ void ydiff(const Hc<FDOH> &hc, const float *t, int jj, int c0, float (&s)[V]) {
 #pragma unroll
-    for (int m = 2; m <= FDOH; m++) {
-        a = ldy2<MIR, ODD, P>(t, jj, c0, m - 1);
-        b = ldy2<MIR, ODD, P>(t, jj, c0, -m);
-        s.x += hc.w[m] * (a.x - b.x);
-        s.y += hc.w[m] * (a.y - b.y);
+    for (int m = 1; m <= FDOH; m++) {
+        const FV<V> a = ldy<MIR, ODD, P, V>(t, jj, c0, FWD ? m : m - 1);
+        const FV<V> b = ldy<MIR, ODD, P, V>(t, jj, c0, FWD ? 1 - m : -m);
+#pragma unroll
+        for (int e = 0; e < V; e++) {
+            const float d = hc.w[m] * (a.v[e] - b.v[e]);
+            if (m == 1) s[e] = Z0 ? 0.0f + d : d;
+            else s[e] += d;
+        }
     }
-    return s;
+}
+// the same with the imaged rows where mir is set (the velocity ops)
+template <bool FWD, bool EDGE, bool ODD, typename P, bool Z0 = false, int FDOH, int V>
+__device__ __forceinline__ void ydiff_fs(const Hc<FDOH> &hc, const float *t, int jj, int c0, bool mir, float (&s)[V]) {
+    if (EDGE && mir) ydiff<FWD, true, ODD, P, Z0>(hc, t, jj, c0, s);
+    else ydiff<FWD, false, ODD, P, Z0>(hc, t, jj, c0, s);
 }
 
-__device__ __forceinline__ float2 lds2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
-__device__ __forceinline__ void sts2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
-__device__ __forceinline__ float pick(const float2 &v, int e) { return e ? v.y : v.x; }
-
-// CPML on a cell known to lie in the strip (hx / hy > 0), src/update_v_PML.c:177-226
-__device__ __forceinline__ float pml_x(const KGrid &g, const KModel<float> &M, float *strip, int j, int hx, int kk,
-                                       int ka, int kb, float d) {
-    return cpml(strip + (j - 1) * (2 * g.fw) + (hx - 1), prof(M, g, kb, hx), prof(M, g, ka, hx), prof(M, g, kk, hx),
-                d, g.k_one);
-}
-__device__ __forceinline__ float pml_y(const KGrid &g, const KModel<float> &M, float *strip, int i, int hy, int kk,
-                                       int ka, int kb, float d) {
-    return cpml(strip + (hy - 1) * g.nx + (i - 1), prof(M, g, kb, hy), prof(M, g, ka, hy), prof(M, g, kk, hy), d,
-                g.k_one);
-}
-
-// Per-thread geometry of a tile: the column pair, its validity and strip
-// indices, and whether the tile needs the CPML path at all.
-struct Cols {
-    int lane, c0, i;
-    bool v0, v1;
-    int hx0, hx1;
-    __device__ __forceinline__ Cols(const KGrid &g, const TileInfo &ti, int XH, bool strips) {
-        lane = threadIdx.x;
-        c0 = XH + 2 * lane;
-        i = ti.i0 + 2 * lane;
-        v0 = i <= g.nx;
-        v1 = i + 1 <= g.nx;
-        hx0 = (strips && v0) ? strip_x(g, i) : 0;
-        hx1 = (strips && v1) ? strip_x(g, i + 1) : 0;
+// A thread's place in its tile: row jj, staged column c0, cell (j, i) of its
+// first column, and the number of its cells inside the grid (nv; 4 on tiles
+// that are not EDGE).
+struct Lane {
+    int jj, c, i, j, nv;
+    template <bool EDGE, int V>
+    static __device__ __forceinline__ Lane of(const KGrid &g, const TileInfo &ti) {
+        Lane q;
+        q.jj = V == 4 ? 2 * threadIdx.y + (threadIdx.x >> 4) : threadIdx.y;
+        q.c = V == 4 ? 4 * (threadIdx.x & 15) : 2 * threadIdx.x;
+        q.i = ti.i0 + q.c;
+        q.j = ti.j0 + q.jj;
+        q.nv = !EDGE ? V : (q.j > g.ny ? 0 : max(0, min(V, g.nx - q.i + 1)));
+        return q;
     }
-    __device__ __forceinline__ int hx(int e) const { return e ? hx1 : hx0; }
-    __device__ __forceinline__ bool valid(int e) const { return e ? v1 : v0; }
 };
 
-// Store a column pair: both cells (8-byte store) or only the first one
-// (the last column of an odd NX).
-__device__ __forceinline__ void gput2(float *p, float n0, float n1, bool pair, bool v0) {
-    if (pair) *reinterpret_cast<float2 *>(p) = make_float2(n0, n1);
-    else if (v0) *p = n0;
+// CPML of the thread's cells (src/update_v_PML.c:177-226).  The strip rows are
+// laid out so that a group of four cells is one aligned 16-byte access
+// (KGrid::psx, psy); cells of the group outside the strip have zero factors
+// and keep their difference.  The memory values are loaded before the wait
+// for the stage (Op::prefetch) and used after the differences.
+template <int V>
+struct Psi {
+    int at;  // index of the group in its strip (-1: in no strip)
+    FV<V> v;
+};
+template <int V>
+__device__ __forceinline__ void psi_x(const KGrid &g, const float *strip, const Lane &q, Psi<V> &s) {
+    s.at = -1;
+    if (g.boundary || g.fw == 0 || q.nv == 0) return;
+    const bool right = q.i + V - 1 >= g.nx - g.fw + 1;
+    if (q.i > g.fw && !right) return;
+    s.at = (q.j - 1) * g.psx + (right ? q.i - 1 - g.psx_rs + g.psx_lw : q.i - 1);
+    s.v = ldv<V>(strip + s.at);
+}
+template <int V>
+__device__ __forceinline__ void psi_y(const KGrid &g, const float *strip, const Lane &q, Psi<V> &s) {
+    s.at = -1;
+    const int hy = q.nv == 0 ? 0 : strip_y(g, q.j);
+    if (!hy) return;
+    s.at = (hy - 1) * g.psy + (q.i - 1);
+    s.v = ldv<V>(strip + s.at);
+}
+// cells lo..hi of the group lie in the strip
+template <int V>
+__device__ __forceinline__ void cpml_group(const KGrid &g, float *strip, Psi<V> &s, const FV<V> &b, const FV<V> &a,
+                                           const FV<V> &K, int lo, int hi, float (&d)[V]) {
+#pragma unroll
+    for (int e = 0; e < V; e++) s.v.v[e] = b.v[e] * s.v.v[e] + a.v[e] * d[e];
+    stv<V>(strip + s.at, s.v.v);
+    if (g.k_one) {  // every K is 1: d/K is d
+#pragma unroll
+        for (int e = 0; e < V; e++) {
+            const float t = d[e] + s.v.v[e];
+            d[e] = e >= lo && e <= hi ? t : d[e];
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < V; e++)
+            if (e >= lo && e <= hi) d[e] = div_rn_pinned(d[e], K.v[e]) + s.v.v[e];
+    }
+}
+// A group that meets both x strips (2 FW close to NX): its left cells one by
+// one; its right cells are the group's own.
+template <int V>
+__device__ __noinline__ FV<V> cpml_left_cells(const KGrid &g, const KModel<float> &M, float *strip, Lane q, bool half,
+                                              FV<V> d) {
+#pragma unroll
+    for (int e = 0; e < V; e++) {
+        const int h = q.i + e;
+        if (h <= g.fw && e < q.nv)
+            d.v[e] = cpml(strip + (q.j - 1) * g.psx + (h - 1), prof(M, g, half ? B_XH : B_X, h),
+                          prof(M, g, half ? A_XH : A_X, h), prof(M, g, half ? K_XH : K_X, h), d.v[e]);
+    }
+    return d;
+}
+// x strips; half: the profiles at half points
+template <int V>
+__device__ __forceinline__ void cpml_x(const KGrid &g, const KModel<float> &M, const ProfTab &pt, float *strip,
+                                       Psi<V> &s, const Lane &q, bool half, float (&d)[V]) {
+    if (s.at < 0) return;
+    const bool left = q.i <= g.fw, right = q.i + V - 1 >= g.nx - g.fw + 1;
+    const float *pr = pt.x + (half ? 3 * pt.xs : 0) + (pt.local ? s.at - (q.j - 1) * g.psx : q.i - 1);
+    if (left && right) {
+        FV<V> t;
+#pragma unroll
+        for (int e = 0; e < V; e++) t.v[e] = d[e];
+        t = cpml_left_cells<V>(g, M, strip, q, half, t);
+#pragma unroll
+        for (int e = 0; e < V; e++) d[e] = t.v[e];
+    }
+    FV<V> K{};
+    if (!g.k_one) K = ldv<V>(pr);
+    cpml_group(g, strip, s, ldv<V>(pr + 2 * pt.xs), ldv<V>(pr + pt.xs), K, right ? g.nx - g.fw + 1 - q.i : 0,
+               right ? q.nv - 1 : g.fw - q.i, d);
+}
+template <int V>
+__device__ __forceinline__ void cpml_y(const KGrid &g, const ProfTab &pt, float *strip, Psi<V> &s, const Lane &q,
+                                       bool half, float (&d)[V]) {
+    if (s.at < 0) return;
+    const int hy = strip_y(g, q.j);
+    const float *pr = pt.y + (half ? 3 * pt.ys : 0) + hy;
+    const float k = g.k_one ? 1.0f : pr[0], a = pr[pt.ys], b = pr[2 * pt.ys];
+    cpml_group(g, strip, s, FV<V>::of(b), FV<V>::of(a), FV<V>::of(k), 0, V - 1, d);
 }
 
-// Row addresses of a thread's column pair: the cell (j, i) in the state of a
-// slot and, on snapshot steps, in the snapshot being stored.
+// x / DH of a thread's values, rounded as the division: by the reciprocal when DH
+// is a power of two, else by the reciprocal and two exact-remainder
+// corrections (Markstein, IBM J. Res. Dev. 34, 1990: with the correctly
+// rounded reciprocal, one correction of a quotient that is off by less than
+// one ulp rounds correctly; the first correction makes it so).  Outside the
+// range where the remainders are exact the division itself runs; a zero is
+// its own quotient.
+template <int V>
+__device__ __forceinline__ void div_dh(const KGrid &g, float (&x)[V]) {
+    if (g.dh_pow2) {
+#pragma unroll
+        for (int e = 0; e < V; e++) x[e] = x[e] * g.inv_dh;
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < V; e++) {
+        const float a = x[e], m = fabsf(a);
+        float q = a * g.inv_dh;
+        q = __fmaf_rn(__fmaf_rn(-q, g.dh, a), g.inv_dh, q);
+        q = __fmaf_rn(__fmaf_rn(-q, g.dh, a), g.inv_dh, q);
+        if (!(m >= g.div_lo && m <= g.div_hi)) q = a == 0.0f ? a : div_rn_pinned(a, g.dh);
+        x[e] = q;
+    }
+}
+
+// Where a thread's cells go: the state of a slot and, on snapshot steps, the
+// snapshot being stored.
+template <bool EDGE, int V>
 struct RowOut {
-    float *st;          // state plane 0 at (j, i)
-    float *sn;          // fp32 snapshot component 0 at (j, i), NULL when not storing fp32
-    __half *sh;         // fp16 snapshot component 0 at (j, i), NULL when not storing fp16
-    float *se;          // fp16: scale of component 0 for this row segment
-    long long se_comp;  // fp16: scales between components
-    bool pair, v0, spair;
-    __device__ __forceinline__ RowOut(const KGrid &g, const KState<float> &S, const KSnapOut &so, int slot, int j,
-                                      const Cols &cl) {
-        st = S.base + (long long)slot * S.slot_stride + ((j - 1 + HY) * g.pitch + (cl.i - 1 + HX));
-        sn = nullptr;
-        sh = nullptr;
-        se = nullptr;
-        se_comp = 0;
-        if (so.base) {
-            char *b = so.base + slot * so.slot_bytes;
-            const long long q = (long long)(j - 1) * g.nx + (cl.i - 1);
-            if (so.f16) {
-                sh = reinterpret_cast<__half *>(b) + q;
-                se = reinterpret_cast<float *>(b + so.ex_off) + (long long)(j - 1) * so.segs + (cl.i - 1) / kSegCells;
-                se_comp = (long long)g.ny * so.segs;
-            } else {
-                sn = reinterpret_cast<float *>(b) + q;
-            }
-        }
-        pair = cl.v1;
-        v0 = cl.v0;
-        spair = cl.v1 && so.pairs;
+    float *st;  // state plane 0 at (j, i)
+    int nv;
+    __device__ __forceinline__ RowOut(const KGrid &g, const KState<float> &S, int slot, const Lane &q) {
+        st = S.base + (long long)slot * S.slot_stride + ((q.j - 1 + HY) * g.pitch + (q.i - 1 + HX));
+        nv = q.nv;
     }
-    __device__ __forceinline__ void put(long long off, float n0, float n1) const { gput2(st + off, n0, n1, pair, v0); }
-    // every lane of the warp calls this for its column pair of the row
-    __device__ __forceinline__ void snap(long long n, int comp, float n0, float n1) const {
-        if (comp < 0) return;
-        if (sn) {
-            float *p = sn + comp * n;
-            if (spair) *reinterpret_cast<float2 *>(p) = make_float2(n0, n1);
-            else {
-                if (v0) p[0] = n0;
-                if (pair) p[1] = n1;
-            }
-        } else if (sh) {
-            float q, inv;
-            seg_scales(seg_absmax_warp(n0, n1, v0, pair), q, inv);
-            __half *p = sh + comp * n;
-            if (spair) *reinterpret_cast<__half2 *>(p) = __floats2half2_rn(n0 * q, n1 * q);
-            else {
-                if (v0) p[0] = __float2half_rn(n0 * q);
-                if (pair) p[1] = __float2half_rn(n1 * q);
-            }
-            if (threadIdx.x == 0) se[comp * se_comp] = inv;
+    __device__ __forceinline__ void put(long long off, const float (&v)[V]) const {
+        float *p = st + off;
+        if (!EDGE || nv == V) {
+            stv<V>(p, v);
+        } else {
+#pragma unroll
+            for (int e = 0; e < V - 1; e++)
+                if (e < nv) p[e] = v[e];
         }
     }
 };
+
+// Component comp of the snapshot being stored, at the thread's cells.  Every
+// lane of the warp calls it: an fp16 segment is one tile row.
+template <bool EDGE, int V>
+__device__ __forceinline__ void snap(const KGrid &g, const KSnapOut &so, int slot, const Lane &q, int comp,
+                                      const float (&v)[V]) {
+    if (comp < 0) return;
+    char *b = so.base + slot * so.slot_bytes;
+    const long long at = comp * so.n + ((long long)(q.j - 1) * g.nx + (q.i - 1));
+    if (!so.f16) {
+        float *p = reinterpret_cast<float *>(b) + at;
+        if (so.align >= V && q.nv == V) {
+            stv<V>(p, v);
+        } else if (V == 4 && so.align == 2 && q.nv == V) {
+#pragma unroll
+            for (int e = 0; e < V; e += 2) *reinterpret_cast<float2 *>(p + e) = make_float2(v[e], v[e + 1]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < V; e++)
+                if (e < q.nv) p[e] = v[e];
+        }
+        return;
+    }
+    unsigned m = 0;
+#pragma unroll
+    for (int e = 0; e < V; e++)
+        if (!EDGE || e < q.nv) m = max(m, __float_as_uint(v[e]) & 0x7fffffffu);
+    if constexpr (V == 4) {
+        const bool low = threadIdx.x < 16;
+        const unsigned m0 = __reduce_max_sync(0xffffffffu, low ? m : 0u);
+        const unsigned m1 = __reduce_max_sync(0xffffffffu, low ? 0u : m);
+        m = low ? m0 : m1;
+    } else {
+        m = __reduce_max_sync(0xffffffffu, m);
+    }
+    float f, inv;
+    seg_scales(__uint_as_float(m), f, inv);
+    if (EDGE && q.nv == 0) return;
+    __half *p = reinterpret_cast<__half *>(b) + at;
+    if (so.align >= 2 && q.nv == V) {
+        unsigned w[V / 2];
+#pragma unroll
+        for (int e = 0; e < V; e += 2) {
+            const __half2 h2 = __floats2half2_rn(v[e] * f, v[e + 1] * f);
+            w[e / 2] = *reinterpret_cast<const unsigned *>(&h2);
+        }
+        if (V == 4 && so.align == 4) {
+            *reinterpret_cast<uint2 *>(p) = make_uint2(w[0], w[V / 2 - 1]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < V / 2; e++) reinterpret_cast<unsigned *>(p)[e] = w[e];
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < V; e++)
+            if (e < q.nv) p[e] = __float2half_rn(v[e] * f);
+    }
+    if (q.c == 0)
+        reinterpret_cast<float *>(b + so.ex_off)[((long long)comp * g.ny + (q.j - 1)) * so.segs + (q.i - 1) / kSegCells] = inv;
+}
 
 // release a stage once every lane of the warp has read its part of it
 __device__ __forceinline__ void release_stage(uint64_t *empty) {
@@ -500,150 +734,141 @@ __device__ __forceinline__ void release_stage(uint64_t *empty) {
     if (threadIdx.x == 0) mbar_arrive(empty);
 }
 
+// The rarely taken rows (sources, free surface, receivers) are out of line
+// and by value, so that they add nothing to the register budget of the main
+// path.
+
 // Explosive sources of step nt on row j, as src/psource.c:47-55 applies
 // them after the stress update and before the free surface
 // (src/IFOS2D.c:1758-1764): the lane holding a source cell adds half the
 // source term to its sxx and syy, sources in list order (psource_apply).
-__device__ __forceinline__ void psource_row(const KGrid &g, const KSrc &src, int slot, int nt, int j, const Cols &cl,
-                                            float (&sxx)[2], float (&syy)[2]) {
-    if (!psource_fires(src, slot)) return;
-    const int n = src.nsrc[slot];
+struct SxxSyy {
+    float xx[4], yy[4];
+};
+static __device__ __noinline__ SxxSyy psource_row(const KGrid &g, const KSrc &src, int slot, int nt, Lane q, SxxSyy v) {
     const float *pos = src.pos + (long long)slot * 8 * src.max_src;
+    const int n = src.nsrc[slot];
+    // the first source's place, type and term are requested with the count: one round trip for the usual single source
+    const float x0 = pos[0], y0 = pos[src.max_src], type0 = pos[7 * src.max_src];
+    const float amp0 = psource_amp(src, slot, 0, nt, g.dh);
+    if (n <= 0 || (int)(n == 1 ? type0 : pos[7 * src.max_src + n - 1]) != 1) return v;  // psource_fires
     for (int l = 0; l < n; l++) {
-        if ((int)pos[src.max_src + l] != j) continue;
-        const int e = (int)pos[l] - cl.i;
-        if ((e != 0 && e != 1) || !cl.valid(e)) continue;
-        const float amp = psource_amp(src, slot, l, nt, g.dh);
-        if (e == 0) {
-            sxx[0] = (float)((double)sxx[0] + 0.5 * (double)amp);
-            syy[0] = (float)((double)syy[0] + 0.5 * (double)amp);
-        } else {
-            sxx[1] = (float)((double)sxx[1] + 0.5 * (double)amp);
-            syy[1] = (float)((double)syy[1] + 0.5 * (double)amp);
-        }
+        if ((int)(l ? pos[src.max_src + l] : y0) != q.j) continue;
+        const int e = (int)(l ? pos[l] : x0) - q.i;
+        if (e < 0 || e >= q.nv) continue;
+        const float amp = l ? psource_amp(src, slot, l, nt, g.dh) : amp0;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (e == k) {
+                v.xx[k] = (float)((double)v.xx[k] + 0.5 * (double)amp);
+                v.yy[k] = (float)((double)v.yy[k] + 0.5 * (double)amp);
+            }
     }
+    return v;
 }
 
 // The free surface of row 1 on a stress op's results (surface_cell: the
 // elastic src/surface_elastic_PML.c:53-104 and, with L memory variables, the
-// viscoelastic src/surface_PML.c:60-157), from the staged velocities (wx:
-// the vx window of row 1; vy2: the zero-started y difference of vy, formed
-// before the stage was released): the derivatives are zero-started sums
-// scaled by 1/DH, vxx carries its own x CPML (psi_vxxs).  p and q are the
-// p and q memory variables (LL each).
-template <int FDOH, int HE, int LL>
-__device__ __forceinline__ void surface_row(const KGrid &g, const KState<float> &S, const KModel<float> &M,
-                                            const Hc<FDOH> &hc, const XWin<HE> &wx, float2 vy2, const Cols &cl,
-                                            int slot, int model, float (&sxx)[2], float (&syy)[2], float (*p)[2],
-                                            float (*q)[2]) {
+// viscoelastic src/surface_PML.c:60-157), from the zero-started differences
+// of the staged velocities (vxx, vyy, formed before the stage was released):
+// scaled by 1/DH, vxx with its own x CPML (psi_vxxs).  p and q are the p and q
+// memory variables (LL each).
+template <int LL, int V>
+struct SurfVals {
+    float xx[V], yy[V], vxx[V], vyy[V], p[LL > 0 ? LL : 1][V], q[LL > 0 ? LL : 1][V];
+};
+template <int LL, int V>
+__device__ __noinline__ SurfVals<LL, V> surface_row(const KGrid &g, const KState<float> &S, const KModel<float> &M,
+                                                 ProfTab pt, Lane c, int slot, int model, SurfVals<LL, V> r) {
     const float DT = g.dt, DH = g.dh;
     const float dh24 = (float)(1.0 / (double)DH), dthalbe = (float)((double)DT / 2.0);
     const float *srf = M.srf + (long long)model * M.srf_stride;
+    float vx4[V];
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-        if (!cl.valid(e)) continue;
-        const int i = cl.i + e;
-        syy[e] = 0.0f;
+    for (int e = 0; e < V; e++) vx4[e] = r.vxx[e] * dh24;
+    // the surface has its x CPML also where the stress update has none (10/12)
+    float *strip = S.psix[X_VXXS] + slot * S.psix_slot;
+    Psi<V> ps;
+    psi_x(g, strip, c, ps);
+    cpml_x<V>(g, M, pt, strip, ps, c, false, vx4);
 #pragma unroll
-        for (int l = 0; l < LL; l++) q[l][e] = 0.0f;
-        float vxx = xbwd<FDOH, HE, true>(hc, wx, e) * dh24;
-        const float vyy = pick(vy2, e) * dh24;
-        const int hx = strip_x(g, i);  // the surface has its x CPML also where the stress update has none (10/12)
-        if (hx) vxx = pml_x(g, M, S.psix[X_VXXS] + slot * S.psix_slot, 1, hx, K_X, A_X, B_X, vxx);
+    for (int e = 0; e < V; e++) {
+        if (e >= c.nv) continue;
+        const int i = c.i + e;
+        r.yy[e] = 0.0f;
+#pragma unroll
+        for (int l = 0; l < LL; l++) r.q[l][e] = 0.0f;
+        const float vxx = vx4[e], vyy = r.vyy[e] * dh24;
         const float fjm = srf[i - 1], gg = srf[g.nx + i - 1];
         if (LL == 0) {
-            sxx[e] += -DT * ((gg * gg) / (gg + fjm) * vxx + gg * vyy);
+            r.xx[e] += -DT * ((gg * gg) / (gg + fjm) * vxx + gg * vyy);
             continue;
         }
         const float djm = srf[2 * g.nx + i - 1], ee = srf[3 * g.nx + i - 1];
         float sump = 0;
 #pragma unroll
-        for (int l = 0; l < LL; l++) sump += p[l][e];
-        sxx[e] += -(DT * (gg - fjm) * (gg - fjm) * vxx / gg) - (DT * (gg - fjm) * vyy) - (dthalbe * sump);
+        for (int l = 0; l < LL; l++) sump += r.p[l][e];
+        r.xx[e] += -(DT * (gg - fjm) * (gg - fjm) * vxx / gg) - (DT * (gg - fjm) * vyy) - (dthalbe * sump);
         sump = 0;
 #pragma unroll
         for (int l = 0; l < LL; l++) {
             const float bjm = g.bjm_srf[l + 1];
-            p[l][e] = (float)((double)p[l][e] + (double)bjm * (((double)(djm - ee) * ((double)(fjm / gg) - 1.0) *
-                                                                 (double)vxx) - (double)((djm - ee) * vyy)));
-            sump += p[l][e];
+            r.p[l][e] = (float)((double)r.p[l][e] + (double)bjm * (((double)(djm - ee) * ((double)(fjm / gg) - 1.0) *
+                                                                    (double)vxx) - (double)((djm - ee) * vyy)));
+            sump += r.p[l][e];
         }
-        sxx[e] += (dthalbe * sump);
+        r.xx[e] += (dthalbe * sump);
     }
+    return r;
 }
 
-// By-value forms of the two for out-of-line calls from the viscoelastic
-// stress op: its rarely taken source and surface rows then do not add to the
-// register budget of its main path (the elastic op has room and inlines them).
-template <int LL>
-struct RowVals {
-    float sxx[2], syy[2], p[LL > 0 ? LL : 1][2], q[LL > 0 ? LL : 1][2];
+// The receivers of the thread's cells in row j on the new vx, vy before they
+// are stored: mode 1 copies them into the seismograms of step nt, as
+// src/seismo_ssg.c:26-140 samples vx, vy after the step (SEISMO 1); mode 2
+// adds the adjoint sources of step nt, as src/update_v_PML.c:567-578 does
+// after the velocity update (ADJOINT_TYPE 1: both components, 2: vy, 3: vx).
+// The slot's cell map gives each cell its receiver (-1: none).
+struct RecIdx {
+    int l[4];
 };
-static __device__ __noinline__ float4 psource_row_v(const KGrid &g, const KSrc &src, int slot, int nt, int j, Cols cl,
-                                             float4 v) {
-    float sxx[2] = {v.x, v.y}, syy[2] = {v.z, v.w};
-    psource_row(g, src, slot, nt, j, cl, sxx, syy);
-    return make_float4(sxx[0], sxx[1], syy[0], syy[1]);
+__device__ __forceinline__ RecIdx rec_lookup(const KGrid &g, const KRec &rec, int slot, const Lane &q) {
+    RecIdx r{{-1, -1, -1, -1}};
+    const int *m = rec.map + (long long)slot * rec.map_stride;
+    const int rr = q.nv > 0 ? m[q.j - 1] : -1;
+    if (rr < 0) return r;
+    const int *cells = m + g.ny + (long long)rr * g.nx + (q.i - 1);
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+        if (e < q.nv) r.l[e] = cells[e];
+    return r;
 }
-// Receiver indices of the thread's column pair in row j (-1: none) when
-// the velocity op samples or injects the receivers in place (rec_mode), read
-// from the slot's cell map at the start of the row so that the two loads are
-// in flight while the row is computed.
-__device__ __forceinline__ int2 rec_lookup(const KGrid &g, const KRec &rec, int mode, int rec_j0, int rec_j1,
-                                           int slot, int j, const Cols &cl) {
-    if (!mode || j < rec_j0 || j > rec_j1 || j > g.ny) return make_int2(-1, -1);
-    return rec_pair(rec, g.nx, g.ny, slot, j, cl.i, cl.v0, cl.v1);
-}
-
-// The receivers of the thread's cells in row j (rl: their indices) on the
-// new vx, vy before they are stored: mode 1 copies them into the seismograms
-// of step nt, as src/seismo_ssg.c:26-140 samples vx, vy after the step
-// (SEISMO 1); mode 2 adds the adjoint sources of step nt, as
-// src/update_v_PML.c:567-578 does after the velocity update (ADJOINT_TYPE 1:
-// both components, 2: vy, 3: vx).
-__device__ __forceinline__ void rec_apply(const KGrid &g, const KRec &rec, int mode, int slot, int nt, int2 rl,
-                                          float (&vx)[2], float (&vy)[2]) {
+static __device__ __noinline__ SxxSyy rec_row(const KGrid &g, const KRec &rec, int mode, int slot, int nt, RecIdx r,
+                                              SxxSyy v) {
     const long long cs = (long long)rec.max_rec * g.nt_total;
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-        const int l = e ? rl.y : rl.x;
+    for (int e = 0; e < 4; e++) {
+        const int l = r.l[e];
         if (l < 0) continue;
         const long long o = (long long)l * g.nt_total + nt - 1;
         if (mode == 2) {
             const float *adj = rec.adj + (long long)slot * 3 * cs + o;
             const int at = g.adjoint_type;
-            if (at == 1 || at == 3) vx[e] += adj[0];
-            if (at == 1 || at == 2) vy[e] += adj[cs];
+            if (at == 1 || at == 3) v.xx[e] += adj[0];
+            if (at == 1 || at == 2) v.yy[e] += adj[cs];
         } else {
             float *sec = rec.sec + (long long)slot * 6 * cs + o;
-            sec[0] = vx[e];
-            sec[cs] = vy[e];
+            sec[0] = v.xx[e];
+            sec[cs] = v.yy[e];
         }
     }
-}
-
-template <int FDOH, int HE, int LL>
-__device__ __noinline__ RowVals<LL> surface_row_v(const KGrid &g, const KState<float> &S, const KModel<float> &M,
-                                                  Hc<FDOH> hc, XWin<HE> wx, float2 vy2, Cols cl, int slot, int model,
-                                                  RowVals<LL> v) {
-    surface_row<FDOH, HE, LL>(g, S, M, hc, wx, vy2, cl, slot, model, v.sxx, v.syy, v.p, v.q);
     return v;
 }
 
-// Interior tiles take rows<false>; tiles with a strip cell rows<true>.
-// The path is chosen per warp (all lanes take the same one, so that the
-// warp-wide operations of the snapshot store and the stage release meet):
-// lanes outside the strips of a strip tile see hx = 0 and no y strip.
-#define IFOS_TILE_COMPUTE(NOPML_)                                                                     \
-    __device__ __forceinline__ void compute(const TileInfo &ti, const float *h, const float *pl,      \
-                                            uint64_t *empty) const {                                  \
-        const Cols cl(g, ti, P::XH, !(NOPML_));                                                       \
-        if ((NOPML_) || (!__any_sync(0xffffffffu, cl.hx0 != 0 || cl.hx1 != 0) && !ti.ystrip))         \
-            rows<false>(ti, cl, h, pl, empty);                                                        \
-        else                                                                                          \
-            rows<true>(ti, cl, h, pl, empty);                                                         \
-    }
-
+// rows<true> runs on warps whose rows of the tile need anything beyond the
+// plain update (TileInfo::edge), rows<false> on the others.  prefetch starts
+// the loads of the CPML memories that rows<true> uses (Pre); they are written
+// by the op's own previous launch only, which has completed before this one
+// starts.
 // the common members of an op
 // src, nt, fsurf, fps: the stress ops apply the explosive sources of step nt
 // (fps; rows src_j0..src_j1 hold every slot's sources) and the free surface
@@ -675,171 +900,166 @@ __device__ __noinline__ RowVals<LL> surface_row_v(const KGrid &g, const KState<f
 // writes sxx syy sxy r p q.  Non-uniform tau planes are read from HBM.
 template <int FDOH, int TY, int LL, int NST, bool QUIRK>
 struct OpSVisc {
-    static constexpr int NH_ = 2, NP_ = 3 + 3 * LL + 6, NOUT = 3 + 3 * LL;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST>;
+    static constexpr int V = kCellsVisc;
+    static constexpr int NH_ = 2, NP_ = 3 + 3 * LL + 6;
+    static constexpr bool CPML = !QUIRK, MIRROR = false;
+    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, visc_blocks(LL), V>;
     IFOS_OP_MEMBERS
-    __device__ void planes(const TileInfo &ti, int *hz, PlainSrc *pz) const {
-        const int zb = ti.slot * tm.planes_per_slot;
-        const int mb = ti.model * tm.model_planes;
-        hz[0] = zb + tm.pid[P_VX];
-        hz[1] = zb + tm.pid[P_VY];
-        pz[0] = {zb + tm.pid[P_SXX], false};
-        pz[1] = {zb + tm.pid[P_SYY], false};
-        pz[2] = {zb + tm.pid[P_SXY], false};
-#pragma unroll
-        for (int l = 0; l < LL; l++) {
-            pz[3 + l] = {zb + tm.mem_pid[0] + l, false};
-            pz[3 + LL + l] = {zb + tm.mem_pid[1] + l, false};
-            pz[3 + 2 * LL + l] = {zb + tm.mem_pid[2] + l, false};
-        }
-        pz[3 + 3 * LL + 0] = {mb + tm.mid[M_FIPJPV], true};
-        pz[3 + 3 * LL + 1] = {mb + tm.mid[M_FV], true};
-        pz[3 + 3 * LL + 2] = {mb + tm.mid[M_GV], true};
-        pz[3 + 3 * LL + 3] = {mb + tm.mid[M_MUR], true};
-        pz[3 + 3 * LL + 4] = {mb + tm.mid[M_PIR], true};
-        pz[3 + 3 * LL + 5] = {mb + tm.mid[M_MUIPJPR], true};
+    // boxes of consecutive planes: their number, planes of box k, whether they are model planes
+    static constexpr int NG = 3;
+    __host__ __device__ static constexpr int gd(int k) { return k == 0 ? 3 : (k == 1 ? 3 * LL : 6); }
+    __host__ __device__ static constexpr bool gm(int k) { return k == 2; }
+    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
+        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
+        hz = zb + tm.pid[P_VX];
+        gz[0] = zb + tm.pid[P_SXX];
+        gz[1] = zb + tm.mem_pid[0];
+        gz[2] = mb + tm.mid[M_FIPJPV];
     }
-    IFOS_TILE_COMPUTE(QUIRK)
-    template <bool PML>
-    __device__ __forceinline__ void rows(const TileInfo &ti, const Cols &cl, const float *h, const float *pl,
-                                         uint64_t *empty) const {
-        constexpr int RT = P::RT;
+    struct Pre {
+        Psi<V> x0, x1, y0, y1;
+    };
+    __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
+        if (!CPML) return;
+        const Lane q = Lane::of<true, V>(g, ti);
+        psi_x<V>(g, S.psix[X_VXX] + ti.slot * S.psix_slot, q, pre.x0);
+        psi_x<V>(g, S.psix[X_VYX] + ti.slot * S.psix_slot, q, pre.x1);
+        psi_y<V>(g, S.psiy[Y_VYY] + ti.slot * S.psiy_slot, q, pre.y0);
+        psi_y<V>(g, S.psiy[Y_VXY] + ti.slot * S.psiy_slot, q, pre.y1);
+    }
+    template <bool EDGE>
+    __device__ __forceinline__ void rows(const TileInfo &ti, Pre &pre, const ProfTab &pt, const float *h,
+                                         const float *pl, uint64_t *empty) const {
+        const Lane q = Lane::of<EDGE, V>(g, ti);
         const float *t_vx = h, *t_vy = h + P::BOXS;
-        float2 vys = make_float2(0.0f, 0.0f);  // the free surface's vy difference (row 1)
+        const int c0 = P::XH + q.c;
         const Hc<FDOH> hc(g);
-        // everything this warp needs from the stage, then release it
-        XWin<P::HE> wx[RT], wy[RT];
-        float2 dxy[RT], dyy[RT], in[RT][NP_];
-#pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int jj = threadIdx.y * RT + r;
-            wx[r].load(t_vx + (jj + P::H) * P::BW, cl.c0);
-            wy[r].load(t_vy + (jj + P::H) * P::BW, cl.c0);
-            dxy[r] = yfwd2<false, false, P, FDOH, QUIRK>(hc, t_vx, jj, cl.c0);
-            dyy[r] = ybwd2<false, false, P, FDOH, QUIRK>(hc, t_vy, jj, cl.c0);
-            if (fsurf && ti.j0 + jj == 1) vys = ybwd2<false, false, P, FDOH, true>(hc, t_vy, jj, cl.c0);
-#pragma unroll
-            for (int q = 0; q < NP_; q++) in[r][q] = lds2(pl + q * P::PLS + jj * kTileX + 2 * cl.lane);
-        }
-        release_stage(empty);
-        const int slot = ti.slot;
-        const long long mo = (long long)ti.model * M.model_stride;
-        const float *ts_p = M.m[M_TAUS] ? M.m[M_TAUS] + mo : nullptr;
-        const float *tp_p = M.m[M_TAUP] ? M.m[M_TAUP] + mo : nullptr;
-        const float *tsij_p = M.m[M_TAUSIPJP] ? M.m[M_TAUSIPJP] + mo : nullptr;
         const float DT = g.dt, DH = g.dh;
         const float dhi = (float)(1.0 / (double)DH), dthalbe = (float)((double)DT / 2.0);
+        const int slot = ti.slot;
+        const bool surf = EDGE && fsurf && q.j == 1;
+        float vxx[V], vyx[V], vxy[V], vyy[V], sx[V], sy[V];  // sx, sy: the surface's zero-started differences
+        {
+            XWin<FDOH, V> w;
+            w.load(t_vx + (q.jj + P::H) * P::BW, c0);
+#pragma unroll
+            for (int e = 0; e < V; e++) vxx[e] = xbwd<QUIRK>(hc, w, e) * dhi;
+            if (surf) {
+#pragma unroll
+                for (int e = 0; e < V; e++) sx[e] = xbwd<true>(hc, w, e);
+            }
+            w.load(t_vy + (q.jj + P::H) * P::BW, c0);
+#pragma unroll
+            for (int e = 0; e < V; e++) vyx[e] = xfwd<QUIRK>(hc, w, e) * dhi;
+        }
+        ydiff<true, false, false, P, QUIRK>(hc, t_vx, q.jj, c0, vxy);
+        ydiff<false, false, false, P, QUIRK>(hc, t_vy, q.jj, c0, vyy);
+        if (surf) ydiff<false, false, false, P, true>(hc, t_vy, q.jj, c0, sy);
+#pragma unroll
+        for (int e = 0; e < V; e++) vxy[e] *= dhi, vyy[e] *= dhi;
+        if (EDGE && CPML) {
+            cpml_x<V>(g, M, pt, S.psix[X_VXX] + slot * S.psix_slot, pre.x0, q, false, vxx);
+            cpml_x<V>(g, M, pt, S.psix[X_VYX] + slot * S.psix_slot, pre.x1, q, true, vyx);
+            cpml_y<V>(g, pt, S.psiy[Y_VYY] + slot * S.psiy_slot, pre.y0, q, false, vyy);
+            cpml_y<V>(g, pt, S.psiy[Y_VXY] + slot * S.psiy_slot, pre.y1, q, true, vxy);
+        }
+        const float *in = pl + q.jj * kTileX + q.c;
+        auto ld = [&](int k) { return ldv<V>(in + k * P::PLS); };
         constexpr int CO = 3 + 3 * LL;  // first coefficient plane
+        const FV<V> s0 = ld(0), s1 = ld(1), s2 = ld(2), fipjp = ld(CO), f = ld(CO + 1), gg = ld(CO + 2);
+        const FV<V> mu = ld(CO + 3), pi = ld(CO + 4), muij = ld(CO + 5);
+        FV<V> mr[LL], mp[LL], mq[LL];
 #pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int j = ti.j0 + threadIdx.y * RT + r;
-            if (j > g.ny) break;
-            float o[NOUT][2];
+        for (int l = 0; l < LL; l++) mr[l] = ld(3 + l), mp[l] = ld(3 + LL + l), mq[l] = ld(3 + 2 * LL + l);
+        release_stage(empty);
+        const RowOut<EDGE, V> out(g, S, slot, q);
+        float div[V], shear[V], o[3][V], sumr[V], sump[V], sumq[V];
 #pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const float2 *v = in[r];
-                float vxx = xbwd<FDOH, P::HE, QUIRK>(hc, wx[r], e) * dhi;
-                float vyx = xfwd<FDOH, P::HE, QUIRK>(hc, wy[r], e) * dhi;
-                float vxy = pick(dxy[r], e) * dhi, vyy = pick(dyy[r], e) * dhi;
-                const bool ok = cl.valid(e);
-                if (PML && ok) {
-                    const int hx = cl.hx(e), ii = cl.i + e;
-                    if (hx) {
-                        vxx = pml_x(g, M, S.psix[X_VXX] + slot * S.psix_slot, j, hx, K_X, A_X, B_X, vxx);
-                        vyx = pml_x(g, M, S.psix[X_VYX] + slot * S.psix_slot, j, hx, K_XH, A_XH, B_XH, vyx);
-                    }
-                    const int hy = strip_y(g, j);
-                    if (hy) {
-                        vyy = pml_y(g, M, S.psiy[Y_VYY] + slot * S.psiy_slot, ii, hy, K_Y, A_Y, B_Y, vyy);
-                        vxy = pml_y(g, M, S.psiy[Y_VXY] + slot * S.psiy_slot, ii, hy, K_YH, A_YH, B_YH, vxy);
-                    }
-                }
-                float sumr = 0, sump = 0, sumq = 0;
-#pragma unroll
-                for (int l = 0; l < LL; l++) {
-                    sumr += pick(v[3 + l], e);
-                    sump += pick(v[3 + LL + l], e);
-                    sumq += pick(v[3 + 2 * LL + l], e);
-                }
-                const float fipjp = pick(v[CO], e), f = pick(v[CO + 1], e), gg = pick(v[CO + 2], e);
-                const float mu = pick(v[CO + 3], e), pi = pick(v[CO + 4], e), muij = pick(v[CO + 5], e);
-                float ts = g.taus0, tp = g.taup0, tsij = g.tausipjp0;
-                if (ok && (ts_p || tp_p || tsij_p)) {
-                    const int c = (j - 1 + HY) * g.pitch + (cl.i + e - 1 + HX);
-                    if (ts_p) ts = ts_p[c];
-                    if (tp_p) tp = tp_p[c];
-                    if (tsij_p) tsij = tsij_p[c];
-                }
-                const float s_xy = pick(v[2], e) + ((fipjp * (vxy + vyx)) + (dthalbe * sumr));
-                const float s_xx = (float)((D)pick(v[0], e) + ((D)(gg * (vxx + vyy)) - ((D)2 * (D)f * (D)vyy) +
-                                                              (D)(dthalbe * sump)));
-                const float s_yy = (float)((D)pick(v[1], e) + ((D)(gg * (vxx + vyy)) - ((D)2 * (D)f * (D)vxx) +
-                                                              (D)(dthalbe * sumq)));
-                sumr = sump = sumq = 0;
-#pragma unroll
-                for (int l = 0; l < LL; l++) {
-                    const float eta = g.eta[l + 1];
-                    // dip, d, e of src/prepare_update_s.c:57-59, formed in the same order
-                    const float dip = muij * eta * tsij, dd = mu * eta * ts, ee = pi * eta * tp;
-                    const float rr = g.bip[l + 1] * (pick(v[3 + l], e) * g.cip[l + 1] - (dip * (vxy + vyx)));
-                    const float pp = (float)((D)g.bjm[l + 1] *
-                                             ((D)(pick(v[3 + LL + l], e) * g.cjm[l + 1] - (ee * (vxx + vyy))) +
-                                              ((D)2 * (D)dd * (D)vyy)));
-                    const float qq = (float)((D)g.bjm[l + 1] *
-                                             ((D)(pick(v[3 + 2 * LL + l], e) * g.cjm[l + 1] - (ee * (vxx + vyy))) +
-                                              ((D)2 * (D)dd * (D)vxx)));
-                    o[3 + l][e] = rr;
-                    o[3 + LL + l][e] = pp;
-                    o[3 + 2 * LL + l][e] = qq;
-                    sumr += rr;
-                    sump += pp;
-                    sumq += qq;
-                }
-                o[0][e] = s_xx + (dthalbe * sump);
-                o[1][e] = s_yy + (dthalbe * sumq);
-                o[2][e] = s_xy + (dthalbe * sumr);
-            }
-            if (fps && j >= src_j0 && j <= src_j1) {
-                const float4 r4 = psource_row_v(g, src, slot, nt, j, cl, make_float4(o[0][0], o[0][1], o[1][0], o[1][1]));
-                o[0][0] = r4.x, o[0][1] = r4.y, o[1][0] = r4.z, o[1][1] = r4.w;
-            }
-            if (fsurf && j == 1) {
-                RowVals<LL> rv;
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    rv.sxx[e] = o[0][e];
-                    rv.syy[e] = o[1][e];
-#pragma unroll
-                    for (int l = 0; l < LL; l++) {
-                        rv.p[l][e] = o[3 + LL + l][e];
-                        rv.q[l][e] = o[3 + 2 * LL + l][e];
-                    }
-                }
-                rv = surface_row_v<FDOH, P::HE, LL>(g, S, M, hc, wx[r], vys, cl, slot, ti.model, rv);
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    o[0][e] = rv.sxx[e];
-                    o[1][e] = rv.syy[e];
-#pragma unroll
-                    for (int l = 0; l < LL; l++) {
-                        o[3 + LL + l][e] = rv.p[l][e];
-                        o[3 + 2 * LL + l][e] = rv.q[l][e];
-                    }
-                }
-            }
-            const RowOut out(g, S, so, slot, j, cl);
-            out.put(S.off[P_SXX], o[0][0], o[0][1]);
-            out.put(S.off[P_SYY], o[1][0], o[1][1]);
-            out.put(S.off[P_SXY], o[2][0], o[2][1]);
+        for (int e = 0; e < V; e++) {
+            div[e] = vxx[e] + vyy[e], shear[e] = vxy[e] + vyx[e];
+            sumr[e] = sump[e] = sumq[e] = 0;
 #pragma unroll
             for (int l = 0; l < LL; l++) {
-                out.put(S.mem_off[0] + l * g.plane, o[3 + l][0], o[3 + l][1]);
-                out.put(S.mem_off[1] + l * g.plane, o[3 + LL + l][0], o[3 + LL + l][1]);
-                out.put(S.mem_off[2] + l * g.plane, o[3 + 2 * LL + l][0], o[3 + 2 * LL + l][1]);
+                sumr[e] += mr[l].v[e];
+                sump[e] += mp[l].v[e];
+                sumq[e] += mq[l].v[e];
             }
-            out.snap(so.n, tm.snap_comp[P_SXX], o[0][0], o[0][1]);
-            out.snap(so.n, tm.snap_comp[P_SYY], o[1][0], o[1][1]);
-            out.snap(so.n, tm.snap_comp[P_SXY], o[2][0], o[2][1]);
+            const D gd = (D)(gg.v[e] * div[e]), f2 = (D)2 * (D)f.v[e];
+            o[2][e] = s2.v[e] + ((fipjp.v[e] * shear[e]) + (dthalbe * sumr[e]));
+            o[0][e] = (float)((D)s0.v[e] + (gd - f2 * (D)vyy[e] + (D)(dthalbe * sump[e])));
+            o[1][e] = (float)((D)s1.v[e] + (gd - f2 * (D)vxx[e] + (D)(dthalbe * sumq[e])));
+            sumr[e] = sump[e] = sumq[e] = 0;
+        }
+        FV<V> ts = FV<V>::of(g.taus0), tp = FV<V>::of(g.taup0), tsij = FV<V>::of(g.tausipjp0);
+        if (M.m[M_TAUS]) {  // the three tau planes are present together; pad cells read what is there
+            const long long at = (long long)ti.model() * M.model_stride + (min(q.j, g.ny) - 1 + HY) * g.pitch +
+                                 (q.nv ? q.i - 1 + HX : 0);
+            ts = ldv<V>(M.m[M_TAUS] + at);
+            tp = ldv<V>(M.m[M_TAUP] + at);
+            tsij = ldv<V>(M.m[M_TAUSIPJP] + at);
+        }
+#pragma unroll
+        for (int l = 0; l < LL; l++) {
+            const float eta = g.eta[l + 1];
+#pragma unroll
+            for (int e = 0; e < V; e++) {
+                // dip, d, e of src/prepare_update_s.c:57-59, formed in the same order
+                const float dip = muij.v[e] * eta * tsij.v[e], dd = mu.v[e] * eta * ts.v[e], ee = pi.v[e] * eta * tp.v[e];
+                const D d2 = (D)2 * (D)dd;
+                mr[l].v[e] = g.bip[l + 1] * (mr[l].v[e] * g.cip[l + 1] - (dip * shear[e]));
+                mp[l].v[e] = (float)((D)g.bjm[l + 1] * ((D)(mp[l].v[e] * g.cjm[l + 1] - (ee * div[e])) + (d2 * (D)vyy[e])));
+                mq[l].v[e] = (float)((D)g.bjm[l + 1] * ((D)(mq[l].v[e] * g.cjm[l + 1] - (ee * div[e])) + (d2 * (D)vxx[e])));
+                sumr[e] += mr[l].v[e];
+                sump[e] += mp[l].v[e];
+                sumq[e] += mq[l].v[e];
+            }
+            out.put(S.mem_off[0] + l * g.plane, mr[l].v);
+            out.put(S.mem_off[1] + l * g.plane, mp[l].v);
+            out.put(S.mem_off[2] + l * g.plane, mq[l].v);
+        }
+#pragma unroll
+        for (int e = 0; e < V; e++) {
+            o[0][e] = o[0][e] + (dthalbe * sump[e]);
+            o[1][e] = o[1][e] + (dthalbe * sumq[e]);
+            o[2][e] = o[2][e] + (dthalbe * sumr[e]);
+        }
+        if (EDGE) {
+            if (fps && q.j >= src_j0 && q.j <= src_j1) {
+                SxxSyy v{};
+#pragma unroll
+                for (int e = 0; e < V; e++) v.xx[e] = o[0][e], v.yy[e] = o[1][e];
+                v = psource_row(g, src, slot, nt, q, v);
+#pragma unroll
+                for (int e = 0; e < V; e++) o[0][e] = v.xx[e], o[1][e] = v.yy[e];
+            }
+            if (surf) {  // changes the thread's own p and q of row 1, stored above
+                SurfVals<LL, V> r;
+#pragma unroll
+                for (int e = 0; e < V; e++) r.xx[e] = o[0][e], r.yy[e] = o[1][e], r.vxx[e] = sx[e], r.vyy[e] = sy[e];
+#pragma unroll
+                for (int l = 0; l < LL; l++)
+#pragma unroll
+                    for (int e = 0; e < V; e++) {
+                        r.p[l][e] = e < q.nv ? out.st[S.mem_off[1] + l * g.plane + e] : 0.0f;
+                        r.q[l][e] = 0.0f;
+                    }
+                r = surface_row<LL, V>(g, S, M, pt, q, slot, ti.model(), r);
+#pragma unroll
+                for (int e = 0; e < V; e++) o[0][e] = r.xx[e], o[1][e] = r.yy[e];
+#pragma unroll
+                for (int l = 0; l < LL; l++) {
+                    out.put(S.mem_off[1] + l * g.plane, r.p[l]);
+                    out.put(S.mem_off[2] + l * g.plane, r.q[l]);
+                }
+            }
+        }
+        out.put(S.off[P_SXX], o[0]);
+        out.put(S.off[P_SYY], o[1]);
+        out.put(S.off[P_SXY], o[2]);
+        if (so.base) {
+            snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SXX], o[0]);
+            snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SYY], o[1]);
+            snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SXY], o[2]);
         }
     }
 };
@@ -849,92 +1069,117 @@ struct OpSVisc {
 // writes sxx syy sxy
 template <int FDOH, int TY, int NST, bool QUIRK>
 struct OpSEl {
+    static constexpr int V = kCells;
     static constexpr int NH_ = 2, NP_ = 6;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, sblocks(FDOH)>;
+    static constexpr bool CPML = !QUIRK, MIRROR = false;
+    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, sblocks(FDOH), V>;
     IFOS_OP_MEMBERS
-    __device__ void planes(const TileInfo &ti, int *hz, PlainSrc *pz) const {
-        const int zb = ti.slot * tm.planes_per_slot;
-        const int mb = ti.model * tm.model_planes;
-        hz[0] = zb + tm.pid[P_VX];
-        hz[1] = zb + tm.pid[P_VY];
-        pz[0] = {zb + tm.pid[P_SXX], false};
-        pz[1] = {zb + tm.pid[P_SYY], false};
-        pz[2] = {zb + tm.pid[P_SXY], false};
-        pz[3] = {mb + tm.mid[M_UIPJP], true};
-        pz[4] = {mb + tm.mid[QUIRK ? M_VS : M_F], true};
-        pz[5] = {mb + tm.mid[QUIRK ? M_VP : M_G], true};
+    // boxes of consecutive planes: their number, planes of box k, whether they are model planes
+    static constexpr int NG = QUIRK ? 4 : 2;
+    __host__ __device__ static constexpr int gd(int k) { return k == 0 || !QUIRK ? 3 : 1; }
+    __host__ __device__ static constexpr bool gm(int k) { return k > 0; }
+    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
+        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
+        hz = zb + tm.pid[P_VX];
+        gz[0] = zb + tm.pid[P_SXX];
+        gz[1] = mb + tm.mid[M_UIPJP];
+        if (QUIRK) gz[2 % NG] = mb + tm.mid[M_VS], gz[3 % NG] = mb + tm.mid[M_VP];
     }
-    IFOS_TILE_COMPUTE(QUIRK)
-    template <bool PML>
-    __device__ __forceinline__ void rows(const TileInfo &ti, const Cols &cl, const float *h, const float *pl,
-                                         uint64_t *empty) const {
-        constexpr int RT = P::RT;
+    struct Pre {
+        Psi<V> x0, x1, y0, y1;
+    };
+    __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
+        if (!CPML) return;
+        const Lane q = Lane::of<true, V>(g, ti);
+        psi_x<V>(g, S.psix[X_VXX] + ti.slot * S.psix_slot, q, pre.x0);
+        psi_x<V>(g, S.psix[X_VYX] + ti.slot * S.psix_slot, q, pre.x1);
+        psi_y<V>(g, S.psiy[Y_VYY] + ti.slot * S.psiy_slot, q, pre.y0);
+        psi_y<V>(g, S.psiy[Y_VXY] + ti.slot * S.psiy_slot, q, pre.y1);
+    }
+    template <bool EDGE>
+    __device__ __forceinline__ void rows(const TileInfo &ti, Pre &pre, const ProfTab &pt, const float *h,
+                                         const float *pl, uint64_t *empty) const {
+        const Lane q = Lane::of<EDGE, V>(g, ti);
         const float *t_vx = h, *t_vy = h + P::BOXS;
-        float2 vys = make_float2(0.0f, 0.0f);  // the free surface's vy difference (row 1)
+        const int c0 = P::XH + q.c;
         const Hc<FDOH> hc(g);
-        XWin<P::HE> wx[RT], wy[RT];
-        float2 dxy[RT], dyy[RT], in[RT][NP_];
-#pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int jj = threadIdx.y * RT + r;
-            wx[r].load(t_vx + (jj + P::H) * P::BW, cl.c0);
-            wy[r].load(t_vy + (jj + P::H) * P::BW, cl.c0);
-            dxy[r] = yfwd2<false, false, P, FDOH>(hc, t_vx, jj, cl.c0);
-            dyy[r] = ybwd2<false, false, P, FDOH>(hc, t_vy, jj, cl.c0);
-            if (fsurf && ti.j0 + jj == 1) vys = ybwd2<false, false, P, FDOH, true>(hc, t_vy, jj, cl.c0);
-#pragma unroll
-            for (int q = 0; q < NP_; q++) in[r][q] = lds2(pl + q * P::PLS + jj * kTileX + 2 * cl.lane);
-        }
-        release_stage(empty);
-        const int slot = ti.slot;
         const float DT = g.dt, DH = g.dh;
         const float dhi = DT / DH;
+        const int slot = ti.slot;
+        const bool surf = EDGE && fsurf && q.j == 1;
+        float vxx[V], vyx[V], vxy[V], vyy[V], sx[V], sy[V];  // sx, sy: the surface's zero-started differences
+        {
+            XWin<FDOH, V> w;
+            w.load(t_vx + (q.jj + P::H) * P::BW, c0);
 #pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int j = ti.j0 + threadIdx.y * RT + r;
-            if (j > g.ny) break;
-            float o[3][2];
+            for (int e = 0; e < V; e++) vxx[e] = xbwd(hc, w, e) * dhi;
+            if (surf) {
 #pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const float2 *v = in[r];
-                float vxx = xbwd<FDOH, P::HE>(hc, wx[r], e) * dhi;
-                float vyx = xfwd<FDOH, P::HE>(hc, wy[r], e) * dhi;
-                float vxy = pick(dxy[r], e) * dhi, vyy = pick(dyy[r], e) * dhi;
-                const float sxx0 = pick(v[0], e), syy0 = pick(v[1], e), sxy0 = pick(v[2], e);
-                if (QUIRK) {
-                    const float fipjp = pick(v[3], e) * DT, f = pick(v[4], e) * DT, gg = pick(v[5], e) * DT;
-                    o[2][e] = sxy0 + (fipjp * (vxy + vyx));
-                    o[0][e] = (float)((D)sxx0 + ((D)(gg * (vxx + vyy)) - ((D)2 * (D)f * (D)vyy)));
-                    o[1][e] = (float)((D)syy0 + ((D)(gg * (vxx + vyy)) - ((D)2 * (D)f * (D)vxx)));
-                    continue;
-                }
-                if (PML && cl.valid(e)) {
-                    const int hx = cl.hx(e), ii = cl.i + e;
-                    if (hx) {
-                        vxx = pml_x(g, M, S.psix[X_VXX] + slot * S.psix_slot, j, hx, K_X, A_X, B_X, vxx);
-                        vyx = pml_x(g, M, S.psix[X_VYX] + slot * S.psix_slot, j, hx, K_XH, A_XH, B_XH, vyx);
-                    }
-                    const int hy = strip_y(g, j);
-                    if (hy) {
-                        vyy = pml_y(g, M, S.psiy[Y_VYY] + slot * S.psiy_slot, ii, hy, K_Y, A_Y, B_Y, vyy);
-                        vxy = pml_y(g, M, S.psiy[Y_VXY] + slot * S.psiy_slot, ii, hy, K_YH, A_YH, B_YH, vxy);
-                    }
-                }
-                const float fipjp = pick(v[3], e), f = pick(v[4], e), gg = pick(v[5], e);
-                o[2][e] = sxy0 + fipjp * (vyx + vxy);
-                o[0][e] = (float)((D)sxx0 + ((D)(gg * (vxx + vyy)) + ((D)2 * (D)f * (D)vxx)));
-                o[1][e] = (float)((D)syy0 + ((D)(gg * (vxx + vyy)) + ((D)2 * (D)f * (D)vyy)));
+                for (int e = 0; e < V; e++) sx[e] = xbwd<true>(hc, w, e);
             }
-            if (fps && j >= src_j0 && j <= src_j1) psource_row(g, src, slot, nt, j, cl, o[0], o[1]);
-            if (fsurf && j == 1)
-                surface_row<FDOH, P::HE, 0>(g, S, M, hc, wx[r], vys, cl, slot, ti.model, o[0], o[1], nullptr, nullptr);
-            const RowOut out(g, S, so, slot, j, cl);
-            out.put(S.off[P_SXX], o[0][0], o[0][1]);
-            out.put(S.off[P_SYY], o[1][0], o[1][1]);
-            out.put(S.off[P_SXY], o[2][0], o[2][1]);
-            out.snap(so.n, tm.snap_comp[P_SXX], o[0][0], o[0][1]);
-            out.snap(so.n, tm.snap_comp[P_SYY], o[1][0], o[1][1]);
-            out.snap(so.n, tm.snap_comp[P_SXY], o[2][0], o[2][1]);
+            w.load(t_vy + (q.jj + P::H) * P::BW, c0);
+#pragma unroll
+            for (int e = 0; e < V; e++) vyx[e] = xfwd(hc, w, e) * dhi;
+        }
+        ydiff<true, false, false, P>(hc, t_vx, q.jj, c0, vxy);
+        ydiff<false, false, false, P>(hc, t_vy, q.jj, c0, vyy);
+        if (surf) ydiff<false, false, false, P, true>(hc, t_vy, q.jj, c0, sy);
+        const float *in = pl + q.jj * kTileX + q.c;
+        auto ld = [&](int k) { return ldv<V>(in + k * P::PLS); };
+        const FV<V> sxx0 = ld(0), syy0 = ld(1), sxy0 = ld(2), fipjp = ld(3), f = ld(4), gg = ld(5);
+        release_stage(empty);
+#pragma unroll
+        for (int e = 0; e < V; e++) vxy[e] *= dhi, vyy[e] *= dhi;
+        float o[3][V];
+        if (QUIRK) {
+#pragma unroll
+            for (int e = 0; e < V; e++) {
+                const float fi = fipjp.v[e] * DT, ff = f.v[e] * DT, gd = gg.v[e] * DT;
+                o[2][e] = sxy0.v[e] + (fi * (vxy[e] + vyx[e]));
+                o[0][e] = (float)((D)sxx0.v[e] + ((D)(gd * (vxx[e] + vyy[e])) - ((D)2 * (D)ff * (D)vyy[e])));
+                o[1][e] = (float)((D)syy0.v[e] + ((D)(gd * (vxx[e] + vyy[e])) - ((D)2 * (D)ff * (D)vxx[e])));
+            }
+        } else {
+            if (EDGE) {
+                cpml_x<V>(g, M, pt, S.psix[X_VXX] + slot * S.psix_slot, pre.x0, q, false, vxx);
+                cpml_x<V>(g, M, pt, S.psix[X_VYX] + slot * S.psix_slot, pre.x1, q, true, vyx);
+                cpml_y<V>(g, pt, S.psiy[Y_VYY] + slot * S.psiy_slot, pre.y0, q, false, vyy);
+                cpml_y<V>(g, pt, S.psiy[Y_VXY] + slot * S.psiy_slot, pre.y1, q, true, vxy);
+            }
+#pragma unroll
+            for (int e = 0; e < V; e++) {
+                o[2][e] = sxy0.v[e] + fipjp.v[e] * (vyx[e] + vxy[e]);
+                o[0][e] = (float)((D)sxx0.v[e] + ((D)(gg.v[e] * (vxx[e] + vyy[e])) + ((D)2 * (D)f.v[e] * (D)vxx[e])));
+                o[1][e] = (float)((D)syy0.v[e] + ((D)(gg.v[e] * (vxx[e] + vyy[e])) + ((D)2 * (D)f.v[e] * (D)vyy[e])));
+            }
+        }
+        if (EDGE) {
+            if (fps && q.j >= src_j0 && q.j <= src_j1) {
+                SxxSyy v{};
+#pragma unroll
+                for (int e = 0; e < V; e++) v.xx[e] = o[0][e], v.yy[e] = o[1][e];
+                v = psource_row(g, src, slot, nt, q, v);
+#pragma unroll
+                for (int e = 0; e < V; e++) o[0][e] = v.xx[e], o[1][e] = v.yy[e];
+            }
+            if (surf) {
+                SurfVals<0, V> r;
+#pragma unroll
+                for (int e = 0; e < V; e++)
+                    r.xx[e] = o[0][e], r.yy[e] = o[1][e], r.vxx[e] = sx[e], r.vyy[e] = sy[e], r.p[0][e] = r.q[0][e] = 0.0f;
+                r = surface_row<0, V>(g, S, M, pt, q, slot, ti.model(), r);
+#pragma unroll
+                for (int e = 0; e < V; e++) o[0][e] = r.xx[e], o[1][e] = r.yy[e];
+            }
+        }
+        const RowOut<EDGE, V> out(g, S, slot, q);
+        out.put(S.off[P_SXX], o[0]);
+        out.put(S.off[P_SYY], o[1]);
+        out.put(S.off[P_SXY], o[2]);
+        if (so.base) {
+            snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SXX], o[0]);
+            snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SYY], o[1]);
+            snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SXY], o[2]);
         }
     }
 };
@@ -948,153 +1193,157 @@ struct OpSEl {
 // the snapshot when the launch stores one, else to the state).
 template <int FDOH, int TY, int NST, bool QUIRK, int SW, bool P1, bool AC>
 struct OpVPsv {
+    static constexpr int V = cells_v(FDOH);
     static constexpr int NH_ = AC ? 1 : 3;
     static constexpr int NP_ = (SW == 1 && !QUIRK) ? 6 : 4;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, vblocks(FDOH)>;
+    static constexpr bool CPML = !QUIRK, MIRROR = true;
+    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, vblocks(FDOH), V>;
     IFOS_OP_MEMBERS
-    __device__ void planes(const TileInfo &ti, int *hz, PlainSrc *pz) const {
-        const int zb = ti.slot * tm.planes_per_slot;
-        const int mb = ti.model * tm.model_planes;
-        if (AC) {
-            hz[0] = zb + tm.pid[P_SP];
-        } else {
-            hz[0] = zb + tm.pid[P_SXX];
-            hz[(1 < NH_) ? 1 : 0] = zb + tm.pid[P_SYY];
-            hz[(2 < NH_) ? 2 : 0] = zb + tm.pid[P_SXY];
-        }
-        pz[0] = {zb + tm.pid[P_VX], false};
-        pz[1] = {zb + tm.pid[P_VY], false};
-        pz[2] = {mb + tm.mid[M_RIP], true};
-        pz[3] = {mb + tm.mid[M_RJP], true};
-        if (NP_ > 4) {
-            pz[4 % NP_] = {zb + tm.pid[P_VXP1], false};
-            pz[5 % NP_] = {zb + tm.pid[P_VYP1], false};
-        }
+    // boxes of consecutive planes: their number, planes of box k, whether they are model planes
+    static constexpr int NG = NP_ / 2;
+    __host__ __device__ static constexpr int gd(int k) { return 2 + 0 * k; }
+    __host__ __device__ static constexpr bool gm(int k) { return k == 1; }
+    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
+        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
+        hz = zb + tm.pid[AC ? P_SP : P_SXX];
+        gz[0] = zb + tm.pid[P_VX];
+        gz[1] = mb + tm.mid[M_RIP];
+        if (NG > 2) gz[2 % NG] = zb + tm.pid[P_VXP1];
     }
-    __device__ __forceinline__ void compute(const TileInfo &ti, const float *h, const float *pl,
-                                            uint64_t *empty) const {
-        const Cols cl(g, ti, P::XH, !QUIRK);
-        const bool mir = g.free_surf && ti.j0 == 1;
-        if (QUIRK || (cl.hx0 == 0 && cl.hx1 == 0 && !ti.ystrip)) {
-            if (mir) rows<true, false>(ti, cl, h, pl, empty);
-            else rows<false, false>(ti, cl, h, pl, empty);
-        } else {
-            if (mir) rows<true, true>(ti, cl, h, pl, empty);
-            else rows<false, true>(ti, cl, h, pl, empty);
-        }
+    struct Pre {
+        Psi<V> x0, x1, y0, y1;
+        RecIdx rec;
+    };
+    __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
+        const Lane q = Lane::of<true, V>(g, ti);
+        if (rec_mode && q.j >= rec_j0 && q.j <= rec_j1) pre.rec = rec_lookup(g, rec, ti.slot, q);
+        else pre.rec = RecIdx{{-1, -1, -1, -1}};
+        if (!CPML) return;
+        psi_x<V>(g, S.psix[X_SXX] + ti.slot * S.psix_slot, q, pre.x0);
+        if (!AC) psi_x<V>(g, S.psix[X_SXY] + ti.slot * S.psix_slot, q, pre.x1);
+        psi_y<V>(g, S.psiy[Y_SYY] + ti.slot * S.psiy_slot, q, pre.y0);
+        if (!AC) psi_y<V>(g, S.psiy[Y_SXY] + ti.slot * S.psiy_slot, q, pre.y1);
     }
-    template <bool MIR, bool PML>
-    __device__ __forceinline__ void rows(const TileInfo &ti, const Cols &cl, const float *h, const float *pl,
-                                         uint64_t *empty) const {
-        constexpr int RT = P::RT;
+    template <bool EDGE>
+    __device__ __forceinline__ void rows(const TileInfo &ti, Pre &pre, const ProfTab &pt, const float *h,
+                                         const float *pl, uint64_t *empty) const {
+        const Lane q = Lane::of<EDGE, V>(g, ti);
         // P-SV: sxx, syy, sxy boxes; acoustic: the sp box serves as all three
         const float *t_sxx = h, *t_syy = AC ? h : h + P::BOXS, *t_sxy = AC ? h : h + 2 * P::BOXS;
+        const int c0 = P::XH + q.c, slot = ti.slot;
         const Hc<FDOH> hc(g);
-        int2 rl[RT];  // receivers of the thread's cells (rec_mode)
+        const bool mir = EDGE && g.free_surf && ti.j0 == 1;
+        // P-SV: sxx_x, syy_y, sxy_x, sxy_y; acoustic: sp_x, sp_y
+        float a_x[V], a_y[V], b_x[V], b_y[V];
+        {
+            XWin<FDOH, V> w;
+            w.load(t_sxx + (q.jj + P::H) * P::BW, c0);
 #pragma unroll
-        for (int r = 0; r < RT; r++)
-            rl[r] = rec_lookup(g, rec, rec_mode, rec_j0, rec_j1, ti.slot, ti.j0 + threadIdx.y * RT + r, cl);
-        XWin<P::HE> wxx[RT], wxy[RT];
-        float2 dyy[RT], dxy[RT], in[RT][NP_];
-        float2 qa[RT][QUIRK && !AC ? FDOH : 1];  // reference 10/12 P-SV form: the sxy y-taps one by one
+            for (int e = 0; e < V; e++) a_x[e] = xfwd<QUIRK && AC>(hc, w, e);
+        }
+        ydiff_fs<true, EDGE, false, P, QUIRK && AC>(hc, t_syy, q.jj, c0, mir, a_y);
+        if (!AC) {
+            XWin<FDOH, V> w;
+            w.load(t_sxy + (q.jj + P::H) * P::BW, c0);
+            if (!QUIRK) {
 #pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int jj = threadIdx.y * RT + r;
-            wxx[r].load(t_sxx + (jj + P::H) * P::BW, cl.c0);
-            if (!AC) wxy[r].load(t_sxy + (jj + P::H) * P::BW, cl.c0);
-            dyy[r] = yfwd2<MIR, false, P, FDOH, QUIRK && AC>(hc, t_syy, jj, cl.c0);
-            if (!AC && !QUIRK) dxy[r] = ybwd2<MIR, true, P, FDOH>(hc, t_sxy, jj, cl.c0);
-            if (!AC && QUIRK) {
+                for (int e = 0; e < V; e++) b_x[e] = xbwd(hc, w, e);
+                ydiff_fs<false, EDGE, true, P>(hc, t_sxy, q.jj, c0, mir, b_y);
+            } else {
+                // one written-out sum per component (src/update_v_PML.c:469-490)
 #pragma unroll
-                for (int m = 1; m <= (QUIRK && !AC ? FDOH : 1); m++) {
-                    const float2 a = ldy2<MIR, true, P>(t_sxy, jj, cl.c0, m - 1);
-                    const float2 b = ldy2<MIR, true, P>(t_sxy, jj, cl.c0, -m);
-                    qa[r][m - 1] = make_float2(a.x - b.x, a.y - b.y);
+                for (int m = 1; m <= FDOH; m++) {
+                    const FV<V> a = EDGE && mir ? ldy<true, true, P, V>(t_sxy, q.jj, c0, m - 1)
+                                             : ldy<false, true, P, V>(t_sxy, q.jj, c0, m - 1);
+                    const FV<V> b = EDGE && mir ? ldy<true, true, P, V>(t_sxy, q.jj, c0, -m)
+                                             : ldy<false, true, P, V>(t_sxy, q.jj, c0, -m);
+#pragma unroll
+                    for (int e = 0; e < V; e++) {
+                        a_x[e] += hc.w[m] * (a.v[e] - b.v[e]);
+                        a_y[e] += hc.w[m] * (w.v[XWin<FDOH, V>::XB + e + m - 1] - w.v[XWin<FDOH, V>::XB + e - m]);
+                    }
                 }
             }
-#pragma unroll
-            for (int q = 0; q < NP_; q++) in[r][q] = lds2(pl + q * P::PLS + jj * kTileX + 2 * cl.lane);
         }
+        const float *in = pl + q.jj * kTileX + q.c;
+        auto ld = [&](int k) { return ldv<V>(in + k * P::PLS); };
+        const FV<V> vxo = ld(0), vyo = ld(1), rip = ld(2), rjp = ld(3);
+        FV<V> px{}, py{};
+        if (NP_ > 4) px = ld(4 % NP_), py = ld(5 % NP_);
         release_stage(empty);
-        const int slot = ti.slot;
         const float DT = g.dt, DH = g.dh;
+        float o[4][V];
+        if (QUIRK) {
+            const float dtdh = DT * DT / DH;
 #pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int j = ti.j0 + threadIdx.y * RT + r;
-            if (j > g.ny) break;
-            float o[4][2];
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const float2 *v = in[r];
-                const float vxo = pick(v[0], e), vyo = pick(v[1], e), rip = pick(v[2], e), rjp = pick(v[3], e);
-                float a_x, a_y, b_x = 0.0f, b_y = 0.0f;  // P-SV: sxx_x, syy_y, sxy_x, sxy_y; acoustic: sp_x, sp_y
-                if (QUIRK) {
-                    const float dtdh = DT * DT / DH;
-                    if (AC) {
-                        a_x = xfwd<FDOH, P::HE, true>(hc, wxx[r], e);
-                        a_y = pick(dyy[r], e);
-                    } else {
-                        // one written-out sum per component (src/update_v_PML.c:469-490)
-                        a_x = xfwd<FDOH, P::HE>(hc, wxx[r], e);
-#pragma unroll
-                        for (int m = 1; m <= (QUIRK && !AC ? FDOH : 1); m++) a_x += hc.w[m] * pick(qa[r][m - 1], e);
-                        a_y = pick(dyy[r], e);
-#pragma unroll
-                        for (int m = 1; m <= FDOH; m++)
-                            a_y += hc.w[m] * (wxy[r].v[P::HE + e + m - 1] - wxy[r].v[P::HE + e - m]);
-                    }
-                    o[0][e] = vxo + a_x * dtdh * rip;
-                    o[1][e] = vyo + a_y * dtdh * rjp;
-                    continue;
-                }
-                a_x = xfwd<FDOH, P::HE>(hc, wxx[r], e);
-                a_y = pick(dyy[r], e);
+            for (int e = 0; e < V; e++) {
+                o[0][e] = vxo.v[e] + a_x[e] * dtdh * rip.v[e];
+                o[1][e] = vyo.v[e] + a_y[e] * dtdh * rjp.v[e];
+            }
+        } else {
+            if (EDGE) {
+                cpml_x<V>(g, M, pt, S.psix[X_SXX] + slot * S.psix_slot, pre.x0, q, true, a_x);
+                cpml_y<V>(g, pt, S.psiy[Y_SYY] + slot * S.psiy_slot, pre.y0, q, true, a_y);
                 if (!AC) {
-                    b_x = xbwd<FDOH, P::HE>(hc, wxy[r], e);
-                    b_y = pick(dxy[r], e);
+                    cpml_x<V>(g, M, pt, S.psix[X_SXY] + slot * S.psix_slot, pre.x1, q, false, b_x);
+                    cpml_y<V>(g, pt, S.psiy[Y_SXY] + slot * S.psiy_slot, pre.y1, q, false, b_y);
                 }
-                if (PML && cl.valid(e)) {
-                    const int hx = cl.hx(e), ii = cl.i + e;
-                    if (hx) {
-                        a_x = pml_x(g, M, S.psix[X_SXX] + slot * S.psix_slot, j, hx, K_XH, A_XH, B_XH, a_x);
-                        if (!AC) b_x = pml_x(g, M, S.psix[X_SXY] + slot * S.psix_slot, j, hx, K_X, A_X, B_X, b_x);
-                    }
-                    const int hy = strip_y(g, j);
-                    if (hy) {
-                        a_y = pml_y(g, M, S.psiy[Y_SYY] + slot * S.psiy_slot, ii, hy, K_YH, A_YH, B_YH, a_y);
-                        if (!AC) b_y = pml_y(g, M, S.psiy[Y_SXY] + slot * S.psiy_slot, ii, hy, K_Y, A_Y, B_Y, b_y);
-                    }
-                }
+            }
+            float fx[V], fy[V];
+#pragma unroll
+            for (int e = 0; e < V; e++) {
                 // P-SV: x force sxx_x + sxy_y, y force sxy_x + syy_y; acoustic: sp_x, sp_y
-                const float fx = AC ? (a_x) : (a_x + b_y), fy = AC ? (a_y) : (b_x + a_y);
+                const float x = AC ? (a_x[e]) : (a_x[e] + b_y[e]), y = AC ? (a_y[e]) : (b_x[e] + a_y[e]);
                 if (SW == 0) {
                     if (P1) {
-                        o[2][e] = div_dh(g, rip * fx);
-                        o[3][e] = div_dh(g, rjp * fy);
+                        o[2][e] = rip.v[e] * x;
+                        o[3][e] = rjp.v[e] * y;
                     }
                 } else {
-                    o[2][e] = pick(v[4 % NP_], e) + vxo * DT;
-                    o[3][e] = pick(v[5 % NP_], e) + vyo * DT;
+                    o[2][e] = px.v[e] + vxo.v[e] * DT;
+                    o[3][e] = py.v[e] + vyo.v[e] * DT;
                 }
-                o[0][e] = vxo + div_dh(g, DT * rip * fx);
-                o[1][e] = vyo + div_dh(g, DT * rjp * fy);
+                fx[e] = DT * rip.v[e] * x;
+                fy[e] = DT * rjp.v[e] * y;
             }
-            if (rl[r].x >= 0 || rl[r].y >= 0) rec_apply(g, rec, rec_mode, slot, nt, rl[r], o[0], o[1]);
-            if (rec_mode == 1 && j == g.ny / 2) {  // the instability probe of the driver (src/IFOS2D.c:1660-1672)
-                const int e = g.nx / 2 - cl.i;
-                if ((e == 0 || e == 1) && cl.valid(e) && isnan(e ? o[1][1] : o[1][0])) atomicExch(bad, 1);
+            if (SW == 0 && P1) {
+                div_dh(g, o[2]);
+                div_dh(g, o[3]);
             }
-            const RowOut out(g, S, so, slot, j, cl);
-            out.put(S.off[P_VX], o[0][0], o[0][1]);
-            out.put(S.off[P_VY], o[1][0], o[1][1]);
-            if (!QUIRK && (SW == 1 || (P1 && !out.sn && !out.sh))) {
-                out.put(S.off[P_VXP1], o[2][0], o[2][1]);
-                out.put(S.off[P_VYP1], o[3][0], o[3][1]);
+            div_dh(g, fx);
+            div_dh(g, fy);
+#pragma unroll
+            for (int e = 0; e < V; e++) {
+                o[0][e] = vxo.v[e] + fx[e];
+                o[1][e] = vyo.v[e] + fy[e];
             }
-            if (!QUIRK && SW == 0 && P1) {
-                out.snap(so.n, tm.snap_comp[P_VXP1], o[2][0], o[2][1]);
-                out.snap(so.n, tm.snap_comp[P_VYP1], o[3][0], o[3][1]);
+        }
+        if (EDGE && rec_mode && q.nv > 0) {
+            if (max(max(pre.rec.l[0], pre.rec.l[1]), max(pre.rec.l[2], pre.rec.l[3])) >= 0) {
+                SxxSyy v{};
+#pragma unroll
+                for (int e = 0; e < V; e++) v.xx[e] = o[0][e], v.yy[e] = o[1][e];
+                v = rec_row(g, rec, rec_mode, slot, nt, pre.rec, v);
+#pragma unroll
+                for (int e = 0; e < V; e++) o[0][e] = v.xx[e], o[1][e] = v.yy[e];
             }
+            if (rec_mode == 1 && q.j == g.ny / 2) {  // the instability probe of the driver (src/IFOS2D.c:1660-1672)
+                const int at = g.nx / 2 - q.i;
+#pragma unroll
+                for (int e = 0; e < V; e++)
+                    if (e == at && e < q.nv && isnan(o[1][e])) atomicExch(bad, 1);
+            }
+        }
+        const RowOut<EDGE, V> out(g, S, slot, q);
+        out.put(S.off[P_VX], o[0]);
+        out.put(S.off[P_VY], o[1]);
+        if (!QUIRK && (SW == 1 || (P1 && !so.base))) {
+            out.put(S.off[P_VXP1], o[2]);
+            out.put(S.off[P_VYP1], o[3]);
+        }
+        if (!QUIRK && SW == 0 && P1 && so.base) {
+            snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_VXP1], o[2]);
+            snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_VYP1], o[3]);
         }
     }
 };
@@ -1103,69 +1352,61 @@ struct OpVPsv {
 // halo: sxz syz; plain: vz rjp; writes vz and vzp1 = previous vz
 template <int FDOH, int TY, int NST>
 struct OpVSh {
+    static constexpr int V = kCells;
     static constexpr int NH_ = 2, NP_ = 2;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, vblocks(FDOH)>;
+    static constexpr bool CPML = true, MIRROR = true;
+    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, vblocks(FDOH), V>;
     IFOS_OP_MEMBERS
-    __device__ void planes(const TileInfo &ti, int *hz, PlainSrc *pz) const {
-        const int zb = ti.slot * tm.planes_per_slot;
-        const int mb = ti.model * tm.model_planes;
-        hz[0] = zb + tm.pid[P_SXZ];
-        hz[1] = zb + tm.pid[P_SYZ];
-        pz[0] = {zb + tm.pid[P_VZ], false};
-        pz[1] = {mb + tm.mid[M_RJP], true};
+    // boxes of consecutive planes: their number, planes of box k, whether they are model planes
+    static constexpr int NG = 2;
+    __host__ __device__ static constexpr int gd(int k) { return 1 + 0 * k; }
+    __host__ __device__ static constexpr bool gm(int k) { return k == 1; }
+    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
+        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
+        hz = zb + tm.pid[P_SXZ];
+        gz[0] = zb + tm.pid[P_VZ];
+        gz[1] = mb + tm.mid[M_RJP];
     }
-    __device__ __forceinline__ void compute(const TileInfo &ti, const float *h, const float *pl,
-                                            uint64_t *empty) const {
-        const Cols cl(g, ti, P::XH, true);
-        const bool mir = g.free_surf && ti.j0 == 1;
-        if (cl.hx0 == 0 && cl.hx1 == 0 && !ti.ystrip) {
-            if (mir) rows<true, false>(ti, cl, h, pl, empty);
-            else rows<false, false>(ti, cl, h, pl, empty);
-        } else {
-            if (mir) rows<true, true>(ti, cl, h, pl, empty);
-            else rows<false, true>(ti, cl, h, pl, empty);
-        }
+    struct Pre {
+        Psi<V> x0, y0;
+    };
+    __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
+        if (!CPML) return;
+        const Lane q = Lane::of<true, V>(g, ti);
+        psi_x<V>(g, S.psix[X_SXZ] + ti.slot * S.psix_slot, q, pre.x0);
+        psi_y<V>(g, S.psiy[Y_SYZ] + ti.slot * S.psiy_slot, q, pre.y0);
     }
-    template <bool MIR, bool PML>
-    __device__ __forceinline__ void rows(const TileInfo &ti, const Cols &cl, const float *h, const float *pl,
-                                         uint64_t *empty) const {
-        constexpr int RT = P::RT;
-        const float *t_sxz = h, *t_syz = h + P::BOXS;
+    template <bool EDGE>
+    __device__ __forceinline__ void rows(const TileInfo &ti, Pre &pre, const ProfTab &pt, const float *h,
+                                         const float *pl, uint64_t *empty) const {
+        const Lane q = Lane::of<EDGE, V>(g, ti);
+        const int c0 = P::XH + q.c, slot = ti.slot;
         const Hc<FDOH> hc(g);
-        XWin<P::HE> wxz[RT];
-        float2 dyz[RT], vz2[RT], rjp2[RT];
+        float sxz_x[V], syz_y[V];
+        {
+            XWin<FDOH, V> w;
+            w.load(h + (q.jj + P::H) * P::BW, c0);
 #pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int jj = threadIdx.y * RT + r;
-            wxz[r].load(t_sxz + (jj + P::H) * P::BW, cl.c0);
-            dyz[r] = yfwd2<MIR, false, P, FDOH>(hc, t_syz, jj, cl.c0);
-            vz2[r] = lds2(pl + jj * kTileX + 2 * cl.lane);
-            rjp2[r] = lds2(pl + P::PLS + jj * kTileX + 2 * cl.lane);
+            for (int e = 0; e < V; e++) sxz_x[e] = xbwd(hc, w, e);
         }
+        ydiff_fs<true, EDGE, false, P>(hc, h + P::BOXS, q.jj, c0, g.free_surf && ti.j0 == 1, syz_y);
+        const float *in = pl + q.jj * kTileX + q.c;
+        const FV<V> vz = ldv<V>(in), rjp = ldv<V>(in + P::PLS);
         release_stage(empty);
-        const int slot = ti.slot;
-        const float DT = g.dt;
-#pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int j = ti.j0 + threadIdx.y * RT + r;
-            if (j > g.ny) break;
-            float o[2];
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                float sxz_x = xbwd<FDOH, P::HE>(hc, wxz[r], e), syz_y = pick(dyz[r], e);
-                if (PML && cl.valid(e)) {
-                    const int hx = cl.hx(e), ii = cl.i + e;
-                    if (hx) sxz_x = pml_x(g, M, S.psix[X_SXZ] + slot * S.psix_slot, j, hx, K_X, A_X, B_X, sxz_x);
-                    const int hy = strip_y(g, j);
-                    if (hy) syz_y = pml_y(g, M, S.psiy[Y_SYZ] + slot * S.psiy_slot, ii, hy, K_YH, A_YH, B_YH, syz_y);
-                }
-                o[e] = pick(vz2[r], e) + div_dh(g, pick(rjp2[r], e) * DT * (sxz_x + syz_y));
-            }
-            const RowOut out(g, S, so, slot, j, cl);
-            out.put(S.off[P_VZP1], vz2[r].x, vz2[r].y);
-            out.put(S.off[P_VZ], o[0], o[1]);
-            out.snap(so.n, tm.snap_comp[P_VZP1], vz2[r].x, vz2[r].y);
+        if (EDGE) {
+            cpml_x<V>(g, M, pt, S.psix[X_SXZ] + slot * S.psix_slot, pre.x0, q, false, sxz_x);
+            cpml_y<V>(g, pt, S.psiy[Y_SYZ] + slot * S.psiy_slot, pre.y0, q, true, syz_y);
         }
+        float f[V], o[V];
+#pragma unroll
+        for (int e = 0; e < V; e++) f[e] = rjp.v[e] * g.dt * (sxz_x[e] + syz_y[e]);
+        div_dh(g, f);
+#pragma unroll
+        for (int e = 0; e < V; e++) o[e] = vz.v[e] + f[e];
+        const RowOut<EDGE, V> out(g, S, slot, q);
+        out.put(S.off[P_VZP1], vz.v);
+        out.put(S.off[P_VZ], o);
+        if (so.base) snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_VZP1], vz.v);
     }
 };
 
@@ -1174,117 +1415,119 @@ struct OpVSh {
 // coefficients (elastic: uipjp f; visco: fipjp f mu muipjp); writes sxz syz [t o]
 template <int FDOH, int TY, int LL, int NST>
 struct OpSSh {
-    static constexpr int NH_ = 1, NP_ = LL ? 2 + 2 * LL + 4 : 4, NOUT = 2 + 2 * LL;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST>;
+    static constexpr int V = kCells;
+    static constexpr int NH_ = 1, NP_ = LL ? 2 + 2 * LL + 4 : 4, L1 = LL > 0 ? LL : 1;
+    static constexpr bool CPML = true, MIRROR = false;
+    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, LL ? 3 : sblocks(FDOH), V>;
     IFOS_OP_MEMBERS
-    __device__ void planes(const TileInfo &ti, int *hz, PlainSrc *pz) const {
-        const int zb = ti.slot * tm.planes_per_slot;
-        const int mb = ti.model * tm.model_planes;
-        hz[0] = zb + tm.pid[P_VZ];
-        pz[0] = {zb + tm.pid[P_SXZ], false};
-        pz[1] = {zb + tm.pid[P_SYZ], false};
-        if (LL == 0) {
-            pz[2] = {mb + tm.mid[M_UIPJP], true};
-            pz[3] = {mb + tm.mid[M_F], true};
-        } else {
-#pragma unroll
-            for (int l = 0; l < LL; l++) {
-                pz[(2 + l) % NP_] = {zb + tm.mem_pid[3] + l, false};       // t
-                pz[(2 + LL + l) % NP_] = {zb + tm.mem_pid[4] + l, false};  // o
-            }
-            pz[(2 + 2 * LL + 0) % NP_] = {mb + tm.mid[M_FIPJPV], true};
-            pz[(2 + 2 * LL + 1) % NP_] = {mb + tm.mid[M_FV], true};
-            pz[(2 + 2 * LL + 2) % NP_] = {mb + tm.mid[M_MUR], true};
-            pz[(2 + 2 * LL + 3) % NP_] = {mb + tm.mid[M_MUIPJPR], true};
-        }
+    // boxes of consecutive planes: their number, planes of box k, whether they are model planes
+    static constexpr int NG = LL ? 5 : 2;
+    __host__ __device__ static constexpr int gd(int k) { return k == 0 ? 2 : (!LL ? 2 : (k == 1 ? 2 * LL : (k == 2 ? 2 : 1))); }
+    __host__ __device__ static constexpr bool gm(int k) { return k >= (LL ? 2 : 1); }
+    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
+        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
+        hz = zb + tm.pid[P_VZ];
+        gz[0] = zb + tm.pid[P_SXZ];
+        gz[1] = LL ? zb + tm.mem_pid[3] : mb + tm.mid[M_UIPJP];
+        if (LL) gz[2 % NG] = mb + tm.mid[M_FIPJPV], gz[3 % NG] = mb + tm.mid[M_MUR], gz[4 % NG] = mb + tm.mid[M_MUIPJPR];
     }
-    IFOS_TILE_COMPUTE(false)
-    template <bool PML>
-    __device__ __forceinline__ void rows(const TileInfo &ti, const Cols &cl, const float *h, const float *pl,
-                                         uint64_t *empty) const {
-        constexpr int RT = P::RT;
-        const float *t_vz = h;
+    struct Pre {
+        Psi<V> x0, y0;
+    };
+    __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
+        if (!CPML) return;
+        const Lane q = Lane::of<true, V>(g, ti);
+        psi_x<V>(g, S.psix[X_VZX] + ti.slot * S.psix_slot, q, pre.x0);
+        psi_y<V>(g, S.psiy[Y_VZY] + ti.slot * S.psiy_slot, q, pre.y0);
+    }
+    template <bool EDGE>
+    __device__ __forceinline__ void rows(const TileInfo &ti, Pre &pre, const ProfTab &pt, const float *h,
+                                         const float *pl, uint64_t *empty) const {
+        const Lane q = Lane::of<EDGE, V>(g, ti);
+        const int c0 = P::XH + q.c, slot = ti.slot;
         const Hc<FDOH> hc(g);
-        XWin<P::HE> wz[RT];
-        float2 dzy[RT], in[RT][NP_];
-#pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int jj = threadIdx.y * RT + r;
-            wz[r].load(t_vz + (jj + P::H) * P::BW, cl.c0);
-            dzy[r] = ybwd2<false, false, P, FDOH>(hc, t_vz, jj, cl.c0);
-#pragma unroll
-            for (int q = 0; q < NP_; q++) in[r][q] = lds2(pl + q * P::PLS + jj * kTileX + 2 * cl.lane);
-        }
-        release_stage(empty);
-        const int slot = ti.slot;
-        const long long mo = (long long)ti.model * M.model_stride;
-        const float *ts_p = M.m[M_TAUS] ? M.m[M_TAUS] + mo : nullptr;
-        const float *tsij_p = M.m[M_TAUSIPJP] ? M.m[M_TAUSIPJP] + mo : nullptr;
         const float DT = g.dt, DH = g.dh;
         const float dhi = LL ? (float)(1.0 / (double)DH) : DT / DH, dthalbe = (float)((double)DT / 2.0);
-        constexpr int CO = 2 + 2 * LL;
+        float vzx[V], vzy[V];
+        {
+            XWin<FDOH, V> w;
+            w.load(h + (q.jj + P::H) * P::BW, c0);
 #pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int j = ti.j0 + threadIdx.y * RT + r;
-            if (j > g.ny) break;
-            float o[NOUT][2];
+            for (int e = 0; e < V; e++) vzx[e] = xfwd(hc, w, e) * dhi;
+        }
+        ydiff<false, false, false, P>(hc, h, q.jj, c0, vzy);
 #pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const float2 *v = in[r];
-                float vzx = xfwd<FDOH, P::HE>(hc, wz[r], e) * dhi, vzy = pick(dzy[r], e) * dhi;
-                const bool ok = cl.valid(e);
-                if (PML && ok) {
-                    const int hx = cl.hx(e), ii = cl.i + e;
-                    if (hx) vzx = pml_x(g, M, S.psix[X_VZX] + slot * S.psix_slot, j, hx, K_XH, A_XH, B_XH, vzx);
-                    const int hy = strip_y(g, j);
-                    if (hy) vzy = pml_y(g, M, S.psiy[Y_VZY] + slot * S.psiy_slot, ii, hy, K_Y, A_Y, B_Y, vzy);
-                }
-                if (LL == 0) {
-                    o[0][e] = pick(v[0], e) + (pick(v[2], e) * vzx);
-                    o[1][e] = pick(v[1], e) + (pick(v[3], e) * vzy);
-                    continue;
-                }
-                float sumo = 0, sumt = 0;
+        for (int e = 0; e < V; e++) vzy[e] *= dhi;
+        if (EDGE) {
+            cpml_x<V>(g, M, pt, S.psix[X_VZX] + slot * S.psix_slot, pre.x0, q, true, vzx);
+            cpml_y<V>(g, pt, S.psiy[Y_VZY] + slot * S.psiy_slot, pre.y0, q, false, vzy);
+        }
+        const float *in = pl + q.jj * kTileX + q.c;
+        auto ld = [&](int k) { return ldv<V>(in + k * P::PLS); };
+        const RowOut<EDGE, V> out(g, S, slot, q);
+        const FV<V> s0 = ld(0), s1 = ld(1);
+        float o[2][V];
+        if (LL == 0) {
+            const FV<V> fi = ld(2 % NP_), f = ld(3 % NP_);
+            release_stage(empty);
 #pragma unroll
-                for (int l = 0; l < LL; l++) {
-                    sumo += pick(v[(2 + LL + l) % NP_], e);
-                    sumt += pick(v[(2 + l) % NP_], e);
-                }
-                const float fipjp = pick(v[CO % NP_], e), f = pick(v[(CO + 1) % NP_], e);
-                const float mu = pick(v[(CO + 2) % NP_], e), muij = pick(v[(CO + 3) % NP_], e);
-                float ts = g.taus0, tsij = g.tausipjp0;
-                if (ok && (ts_p || tsij_p)) {
-                    const int c = (j - 1 + HY) * g.pitch + (cl.i + e - 1 + HX);
-                    if (ts_p) ts = ts_p[c];
-                    if (tsij_p) tsij = tsij_p[c];
-                }
-                const float s_xz = pick(v[0], e) + ((fipjp * vzx) + (dthalbe * sumo));
-                const float s_yz = pick(v[1], e) + ((f * vzy) + (dthalbe * sumt));
-                sumo = sumt = 0;
-#pragma unroll
-                for (int l = 0; l < LL; l++) {
-                    const float eta = g.eta[l + 1];
-                    const float dip = muij * eta * tsij, dd = mu * eta * ts;
-                    const float oo = g.bip[l + 1] * (pick(v[(2 + LL + l) % NP_], e) * g.cip[l + 1] - (dip * vzx));
-                    const float tt = g.bjm[l + 1] * (pick(v[(2 + l) % NP_], e) * g.cjm[l + 1] - (dd * vzy));
-                    o[(2 + LL + l) % NOUT][e] = oo;
-                    o[(2 + l) % NOUT][e] = tt;
-                    sumt += tt;
-                    sumo += oo;
-                }
-                o[0][e] = s_xz + (dthalbe * sumo);
-                o[1][e] = s_yz + (dthalbe * sumt);
+            for (int e = 0; e < V; e++) {
+                o[0][e] = s0.v[e] + (fi.v[e] * vzx[e]);
+                o[1][e] = s1.v[e] + (f.v[e] * vzy[e]);
             }
-            const RowOut out(g, S, so, slot, j, cl);
-            out.put(S.off[P_SXZ], o[0][0], o[0][1]);
-            out.put(S.off[P_SYZ], o[1][0], o[1][1]);
+        } else {
+            constexpr int CO = 2 + 2 * LL;
+            FV<V> mt[L1], mo[L1];
+#pragma unroll
+            for (int l = 0; l < LL; l++) mt[l] = ld(2 + l), mo[l] = ld(2 + LL + l);
+            const FV<V> fipjp = ld(CO), f = ld(CO + 1), mu = ld(CO + 2), muij = ld(CO + 3);
+            release_stage(empty);
+            FV<V> ts = FV<V>::of(g.taus0), tsij = FV<V>::of(g.tausipjp0);
+            if (M.m[M_TAUS]) {
+                const long long at = (long long)ti.model() * M.model_stride + (min(q.j, g.ny) - 1 + HY) * g.pitch +
+                                     (q.nv ? q.i - 1 + HX : 0);
+                ts = ldv<V>(M.m[M_TAUS] + at);
+                tsij = ldv<V>(M.m[M_TAUSIPJP] + at);
+            }
+            float sumo[V] = {}, sumt[V] = {};
+#pragma unroll
+            for (int e = 0; e < V; e++) {
+#pragma unroll
+                for (int l = 0; l < LL; l++) {
+                    sumo[e] += mo[l].v[e];
+                    sumt[e] += mt[l].v[e];
+                }
+                o[0][e] = s0.v[e] + ((fipjp.v[e] * vzx[e]) + (dthalbe * sumo[e]));
+                o[1][e] = s1.v[e] + ((f.v[e] * vzy[e]) + (dthalbe * sumt[e]));
+                sumo[e] = sumt[e] = 0;
+            }
 #pragma unroll
             for (int l = 0; l < LL; l++) {
-                out.put(S.mem_off[3] + l * g.plane, o[(2 + l) % NOUT][0], o[(2 + l) % NOUT][1]);
-                out.put(S.mem_off[4] + l * g.plane, o[(2 + LL + l) % NOUT][0], o[(2 + LL + l) % NOUT][1]);
+                const float eta = g.eta[l + 1];
+#pragma unroll
+                for (int e = 0; e < V; e++) {
+                    const float dip = muij.v[e] * eta * tsij.v[e], dd = mu.v[e] * eta * ts.v[e];
+                    const float oo = g.bip[l + 1] * (mo[l].v[e] * g.cip[l + 1] - (dip * vzx[e]));
+                    const float tt = g.bjm[l + 1] * (mt[l].v[e] * g.cjm[l + 1] - (dd * vzy[e]));
+                    mo[l].v[e] = oo;
+                    mt[l].v[e] = tt;
+                    sumt[e] += tt;
+                    sumo[e] += oo;
+                }
+                out.put(S.mem_off[3] + l * g.plane, mt[l].v);
+                out.put(S.mem_off[V] + l * g.plane, mo[l].v);
             }
-            out.snap(so.n, tm.snap_comp[P_SXZ], o[0][0], o[0][1]);
-            out.snap(so.n, tm.snap_comp[P_SYZ], o[1][0], o[1][1]);
+#pragma unroll
+            for (int e = 0; e < V; e++) {
+                o[0][e] = o[0][e] + (dthalbe * sumo[e]);
+                o[1][e] = o[1][e] + (dthalbe * sumt[e]);
+            }
+        }
+        out.put(S.off[P_SXZ], o[0]);
+        out.put(S.off[P_SYZ], o[1]);
+        if (so.base) {
+            snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SXZ], o[0]);
+            snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SYZ], o[1]);
         }
     }
 };
@@ -1293,65 +1536,67 @@ struct OpSSh {
 // halo: vx vy; plain: sp g (reference 10/12 branch: vp); writes sp
 template <int FDOH, int TY, int NST, bool QUIRK>
 struct OpPAc {
+    static constexpr int V = kCells;
     static constexpr int NH_ = 2, NP_ = 2;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST>;
+    static constexpr bool CPML = !QUIRK, MIRROR = false;
+    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, sblocks(FDOH), V>;
     IFOS_OP_MEMBERS
-    __device__ void planes(const TileInfo &ti, int *hz, PlainSrc *pz) const {
-        const int zb = ti.slot * tm.planes_per_slot;
-        const int mb = ti.model * tm.model_planes;
-        hz[0] = zb + tm.pid[P_VX];
-        hz[1] = zb + tm.pid[P_VY];
-        pz[0] = {zb + tm.pid[P_SP], false};
-        pz[1] = {mb + tm.mid[QUIRK ? M_VP : M_GAC], true};
+    // boxes of consecutive planes: their number, planes of box k, whether they are model planes
+    static constexpr int NG = 2;
+    __host__ __device__ static constexpr int gd(int k) { return 1 + 0 * k; }
+    __host__ __device__ static constexpr bool gm(int k) { return k == 1; }
+    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
+        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
+        hz = zb + tm.pid[P_VX];
+        gz[0] = zb + tm.pid[P_SP];
+        gz[1] = mb + tm.mid[QUIRK ? M_VP : M_GAC];
     }
-    IFOS_TILE_COMPUTE(QUIRK)
-    template <bool PML>
-    __device__ __forceinline__ void rows(const TileInfo &ti, const Cols &cl, const float *h, const float *pl,
-                                         uint64_t *empty) const {
-        constexpr int RT = P::RT;
-        const float *t_vx = h, *t_vy = h + P::BOXS;
+    struct Pre {
+        Psi<V> x0, y0;
+    };
+    __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
+        if (!CPML) return;
+        const Lane q = Lane::of<true, V>(g, ti);
+        psi_x<V>(g, S.psix[X_VXX] + ti.slot * S.psix_slot, q, pre.x0);
+        psi_y<V>(g, S.psiy[Y_VYY] + ti.slot * S.psiy_slot, q, pre.y0);
+    }
+    template <bool EDGE>
+    __device__ __forceinline__ void rows(const TileInfo &ti, Pre &pre, const ProfTab &pt, const float *h,
+                                         const float *pl, uint64_t *empty) const {
+        const Lane q = Lane::of<EDGE, V>(g, ti);
+        const int c0 = P::XH + q.c, slot = ti.slot;
         const Hc<FDOH> hc(g);
-        XWin<P::HE> wx[RT];
-        float2 dyy[RT], sp2[RT], g2[RT];
-#pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int jj = threadIdx.y * RT + r;
-            wx[r].load(t_vx + (jj + P::H) * P::BW, cl.c0);
-            dyy[r] = ybwd2<false, false, P, FDOH, QUIRK>(hc, t_vy, jj, cl.c0);
-            sp2[r] = lds2(pl + jj * kTileX + 2 * cl.lane);
-            g2[r] = lds2(pl + P::PLS + jj * kTileX + 2 * cl.lane);
-        }
-        release_stage(empty);
-        const int slot = ti.slot;
         const float DT = g.dt, DH = g.dh;
         const float dhi = DT / DH;
+        float vxx[V], vyy[V], o[V];
+        {
+            XWin<FDOH, V> w;
+            w.load(h + (q.jj + P::H) * P::BW, c0);
 #pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int j = ti.j0 + threadIdx.y * RT + r;
-            if (j > g.ny) break;
-            float o[2];
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                float vxx = xbwd<FDOH, P::HE, QUIRK>(hc, wx[r], e), vyy = pick(dyy[r], e);
-                if (QUIRK) {
-                    const float gg = pick(g2[r], e) * DT;
-                    o[e] = pick(sp2[r], e) + (gg * (vxx + vyy)) * dhi;
-                    continue;
-                }
-                vxx = vxx * dhi;
-                vyy = vyy * dhi;
-                if (PML && cl.valid(e)) {
-                    const int hx = cl.hx(e), ii = cl.i + e;
-                    if (hx) vxx = pml_x(g, M, S.psix[X_VXX] + slot * S.psix_slot, j, hx, K_X, A_X, B_X, vxx);
-                    const int hy = strip_y(g, j);
-                    if (hy) vyy = pml_y(g, M, S.psiy[Y_VYY] + slot * S.psiy_slot, ii, hy, K_Y, A_Y, B_Y, vyy);
-                }
-                o[e] = pick(sp2[r], e) + pick(g2[r], e) * (vxx + vyy);
-            }
-            const RowOut out(g, S, so, slot, j, cl);
-            out.put(S.off[P_SP], o[0], o[1]);
-            out.snap(so.n, tm.snap_comp[P_SP], o[0], o[1]);
+            for (int e = 0; e < V; e++) vxx[e] = xbwd<QUIRK>(hc, w, e);
         }
+        ydiff<false, false, false, P, QUIRK>(hc, h + P::BOXS, q.jj, c0, vyy);
+        const float *in = pl + q.jj * kTileX + q.c;
+        const FV<V> sp = ldv<V>(in), gg = ldv<V>(in + P::PLS);
+        release_stage(empty);
+        if (QUIRK) {
+#pragma unroll
+            for (int e = 0; e < V; e++) {
+                const float gd = gg.v[e] * DT;
+                o[e] = sp.v[e] + (gd * (vxx[e] + vyy[e])) * dhi;
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < V; e++) vxx[e] = vxx[e] * dhi, vyy[e] = vyy[e] * dhi;
+            if (EDGE) {
+                cpml_x<V>(g, M, pt, S.psix[X_VXX] + slot * S.psix_slot, pre.x0, q, false, vxx);
+                cpml_y<V>(g, pt, S.psiy[Y_VYY] + slot * S.psiy_slot, pre.y0, q, false, vyy);
+            }
+#pragma unroll
+            for (int e = 0; e < V; e++) o[e] = sp.v[e] + gg.v[e] * (vxx[e] + vyy[e]);
+        }
+        RowOut<EDGE, V>(g, S, slot, q).put(S.off[P_SP], o);
+        if (so.base) snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SP], o);
     }
 };
 // pressure, viscoacoustic with LL relaxation mechanisms
@@ -1361,101 +1606,103 @@ struct OpPAc {
 // read from HBM.
 template <int FDOH, int TY, int LL, int NST>
 struct OpPVisc {
-    static constexpr bool Z0 = FDOH != 1;
+    static constexpr int V = kCells;
+    static constexpr bool Z0 = FDOH != 1, CPML = !Z0, MIRROR = false;
     static constexpr int NH_ = 2, NP_ = 3 + LL;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST>;
+    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, 3, V>;
     IFOS_OP_MEMBERS
-    __device__ void planes(const TileInfo &ti, int *hz, PlainSrc *pz) const {
-        const int zb = ti.slot * tm.planes_per_slot;
-        const int mb = ti.model * tm.model_planes;
-        hz[0] = zb + tm.pid[P_VX];
-        hz[1] = zb + tm.pid[P_VY];
-        pz[0] = {zb + tm.pid[P_SP], false};
-#pragma unroll
-        for (int l = 0; l < LL; l++) pz[1 + l] = {zb + tm.mem_pid[1] + l, false};
-        pz[1 + LL] = {mb + tm.mid[M_GV], true};
-        pz[2 + LL] = {mb + tm.mid[M_PIR], true};
+    // boxes of consecutive planes: their number, planes of box k, whether they are model planes
+    static constexpr int NG = 3;
+    __host__ __device__ static constexpr int gd(int k) { return k == 0 ? 1 : (k == 1 ? LL : 2); }
+    __host__ __device__ static constexpr bool gm(int k) { return k == 2; }
+    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
+        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
+        hz = zb + tm.pid[P_VX];
+        gz[0] = zb + tm.pid[P_SP];
+        gz[1] = zb + tm.mem_pid[1];
+        gz[2] = mb + tm.mid[M_GV];
     }
-    IFOS_TILE_COMPUTE(Z0)
-    template <bool PML>
-    __device__ __forceinline__ void rows(const TileInfo &ti, const Cols &cl, const float *h, const float *pl,
-                                         uint64_t *empty) const {
-        constexpr int RT = P::RT;
-        const float *t_vx = h, *t_vy = h + P::BOXS;
+    struct Pre {
+        Psi<V> x0, y0;
+    };
+    __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
+        if (!CPML) return;
+        const Lane q = Lane::of<true, V>(g, ti);
+        psi_x<V>(g, S.psix[X_VXX] + ti.slot * S.psix_slot, q, pre.x0);
+        psi_y<V>(g, S.psiy[Y_VYY] + ti.slot * S.psiy_slot, q, pre.y0);
+    }
+    template <bool EDGE>
+    __device__ __forceinline__ void rows(const TileInfo &ti, Pre &pre, const ProfTab &pt, const float *h,
+                                         const float *pl, uint64_t *empty) const {
+        const Lane q = Lane::of<EDGE, V>(g, ti);
+        const int c0 = P::XH + q.c, slot = ti.slot;
         const Hc<FDOH> hc(g);
-        XWin<P::HE> wx[RT];
-        float2 dyy[RT], in[RT][NP_];
-#pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int jj = threadIdx.y * RT + r;
-            wx[r].load(t_vx + (jj + P::H) * P::BW, cl.c0);
-            dyy[r] = ybwd2<false, false, P, FDOH, Z0>(hc, t_vy, jj, cl.c0);
-#pragma unroll
-            for (int q = 0; q < NP_; q++) in[r][q] = lds2(pl + q * P::PLS + jj * kTileX + 2 * cl.lane);
-        }
-        release_stage(empty);
-        const int slot = ti.slot;
-        const float *tp_p = M.m[M_TAUP] ? M.m[M_TAUP] + (long long)ti.model * M.model_stride : nullptr;
         const float DT = g.dt, DH = g.dh;
         const float dhi = (float)(1.0 / (double)DH), dthalbe = (float)((double)DT / 2.0);
+        float vxx[V], vyy[V], o[V];
+        {
+            XWin<FDOH, V> w;
+            w.load(h + (q.jj + P::H) * P::BW, c0);
 #pragma unroll
-        for (int r = 0; r < RT; r++) {
-            const int j = ti.j0 + threadIdx.y * RT + r;
-            if (j > g.ny) break;
-            float o[1 + LL][2];
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const float2 *v = in[r];
-                float vxx = xbwd<FDOH, P::HE, Z0>(hc, wx[r], e) * dhi, vyy = pick(dyy[r], e) * dhi;
-                const bool ok = cl.valid(e);
-                if (PML && ok) {
-                    const int hx = cl.hx(e), ii = cl.i + e;
-                    if (hx) vxx = pml_x(g, M, S.psix[X_VXX] + slot * S.psix_slot, j, hx, K_X, A_X, B_X, vxx);
-                    const int hy = strip_y(g, j);
-                    if (hy) vyy = pml_y(g, M, S.psiy[Y_VYY] + slot * S.psiy_slot, ii, hy, K_Y, A_Y, B_Y, vyy);
-                }
-                float sump = 0;
-#pragma unroll
-                for (int l = 0; l < LL; l++) sump += pick(v[1 + l], e);
-                const float gg = pick(v[1 + LL], e), pi = pick(v[2 + LL], e);
-                float tp = g.taup0;
-                if (ok && tp_p) tp = tp_p[(j - 1 + HY) * g.pitch + (cl.i + e - 1 + HX)];
-                const float s = pick(v[0], e) + ((gg * (vxx + vyy)) + (dthalbe * sump));
-                sump = 0;
-#pragma unroll
-                for (int l = 0; l < LL; l++) {
-                    const float ee = pi * g.eta[l + 1] * tp;  // e of src/prepare_update_p.c:62
-                    const float pp = g.bjm[l + 1] * (pick(v[1 + l], e) * g.cjm[l + 1] - (ee * (vxx + vyy)));
-                    o[1 + l][e] = pp;
-                    sump += pp;
-                }
-                o[0][e] = s + (dthalbe * sump);
-            }
-            const RowOut out(g, S, so, slot, j, cl);
-            out.put(S.off[P_SP], o[0][0], o[0][1]);
-#pragma unroll
-            for (int l = 0; l < LL; l++) out.put(S.mem_off[1] + l * g.plane, o[1 + l][0], o[1 + l][1]);
-            out.snap(so.n, tm.snap_comp[P_SP], o[0][0], o[0][1]);
+            for (int e = 0; e < V; e++) vxx[e] = xbwd<Z0>(hc, w, e) * dhi;
         }
+        ydiff<false, false, false, P, Z0>(hc, h + P::BOXS, q.jj, c0, vyy);
+#pragma unroll
+        for (int e = 0; e < V; e++) vyy[e] *= dhi;
+        const float *in = pl + q.jj * kTileX + q.c;
+        auto ld = [&](int k) { return ldv<V>(in + k * P::PLS); };
+        FV<V> mp[LL];
+#pragma unroll
+        for (int l = 0; l < LL; l++) mp[l] = ld(1 + l);
+        const FV<V> sp = ld(0), gg = ld(1 + LL), pi = ld(2 + LL);
+        release_stage(empty);
+        if (EDGE && CPML) {
+            cpml_x<V>(g, M, pt, S.psix[X_VXX] + slot * S.psix_slot, pre.x0, q, false, vxx);
+            cpml_y<V>(g, pt, S.psiy[Y_VYY] + slot * S.psiy_slot, pre.y0, q, false, vyy);
+        }
+        FV<V> tp = FV<V>::of(g.taup0);
+        if (M.m[M_TAUP])
+            tp = ldv<V>(M.m[M_TAUP] + (long long)ti.model() * M.model_stride + (min(q.j, g.ny) - 1 + HY) * g.pitch +
+                      (q.nv ? q.i - 1 + HX : 0));
+        const RowOut<EDGE, V> out(g, S, slot, q);
+        float sump[V] = {};
+#pragma unroll
+        for (int e = 0; e < V; e++) {
+#pragma unroll
+            for (int l = 0; l < LL; l++) sump[e] += mp[l].v[e];
+            o[e] = sp.v[e] + ((gg.v[e] * (vxx[e] + vyy[e])) + (dthalbe * sump[e]));
+            sump[e] = 0;
+        }
+#pragma unroll
+        for (int l = 0; l < LL; l++) {
+#pragma unroll
+            for (int e = 0; e < V; e++) {
+                const float ee = pi.v[e] * g.eta[l + 1] * tp.v[e];  // e of src/prepare_update_p.c:62
+                const float pp = g.bjm[l + 1] * (mp[l].v[e] * g.cjm[l + 1] - (ee * (vxx[e] + vyy[e])));
+                mp[l].v[e] = pp;
+                sump[e] += pp;
+            }
+            out.put(S.mem_off[1] + l * g.plane, mp[l].v);
+        }
+#pragma unroll
+        for (int e = 0; e < V; e++) o[e] = o[e] + (dthalbe * sump[e]);
+        out.put(S.off[P_SP], o);
+        if (so.base) snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SP], o);
     }
 };
-#undef IFOS_TILE_COMPUTE
 #undef IFOS_OP_MEMBERS
 
 // Blocks per SM for the register budget: as many as the shared-memory ring
-// allows (227 KB per SM), at most 3, and no more than leave 64 registers a
-// thread.
+// allows (227 KB per SM), at most the op's BLOCK_CAP.
 template <typename P>
 constexpr int ring_blocks() {
-    constexpr int by_smem = (int)(232448 / (P::bytes() + 1024));
-    constexpr int by_regs = 65536 / (kBlockThreads * (P::BLOCK_CAP > 3 ? 56 : 64));
-    constexpr int b = by_smem < by_regs ? by_smem : by_regs;
+    constexpr int b = (int)(232448 / (P::bytes() + 1024 + 2 * kTileBatch * sizeof(TileInfo) + 6 * (kProfX + kProfY) * 4 + 128));
     return b < 1 ? 1 : (b > P::BLOCK_CAP ? P::BLOCK_CAP : b);
 }
 
 // the kernel: one Op per launch, persistent over all tiles of all slots
 template <typename Op>
-__global__ void __launch_bounds__(kBlockThreads, ring_blocks<typename Op::P>())
+__global__ void __launch_bounds__(Op::P::THREADS, ring_blocks<typename Op::P>())
     kp_stencil(const __grid_constant__ KMaps maps, const __grid_constant__ Op op, int nshots, int *err) {
     run_pipeline<typename Op::P>(op.g, maps, nshots, op, err);
 }
