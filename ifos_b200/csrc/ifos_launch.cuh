@@ -248,14 +248,14 @@ struct Launcher {
     KRec rec;
     dim3 blk{32, 8, 1}, grd;
     int nshots;
-    // the stress ops apply the explosive sources (fps) and the free surface
-    // (fsurf) of step nt_cur themselves: P-SV elastic and viscoelastic only
-    int nt_cur = 0, fsurf = 0, fps = 0;
+    // what the ops of the step being launched do beside the update (the
+    // members of the same names): P-SV, SH or acoustic alone on the pipelined path
+    int nt_cur = 0, fsurf = 0, fps = 0, fvs = 0;
+    int v_rec = 0, v_probe = 0, s_rec = 0;  // rec_mode and probe of the velocity ops, rec_mode of the pressure op
     int src_j0 = 1, src_j1 = 0;  // rows holding the slots' sources (empty range: none)
-    // the P-SV velocity ops sample (1) or inject (2) the receivers of rows
-    // rec_j0..rec_j1 themselves (the setting of the step being launched)
-    int rec_mode = 0, rec_j0 = 1, rec_j1 = 0;
-    bool seis_fused = false;  // the forward's velocity ops sample the receivers (no seismogram kernel)
+    int rec_j0 = 1, rec_j1 = 0;  // rows holding their receivers
+    bool surf_fused = false;  // the ops apply the explosive sources and the free surface (no surface kernel)
+    bool seis_fused = false;  // the forward's ops sample the receivers (no seismogram kernel)
     // rows holding the receivers of slots [0, nshots); false when a slot's
     // receivers do not fit its cell map
     bool receiver_rows() {
@@ -305,8 +305,15 @@ struct Launcher {
         using P = typename Op::P;
         Op op = op0;
         op.nt = nt_cur;
+        op.src = src;
+        op.src_j0 = src_j0;
+        op.src_j1 = src_j1;
         op.rec = rec;
-        op.rec_mode = rec_mode;
+        op.fsurf = Op::MIRROR ? 0 : fsurf;
+        op.fps = Op::MIRROR ? 0 : fps;
+        op.fvs = Op::MIRROR ? fvs : 0;
+        op.probe = Op::MIRROR ? v_probe : 0;
+        op.rec_mode = Op::MIRROR ? v_rec : s_rec;
         op.rec_j0 = rec_j0;
         op.rec_j1 = rec_j1;
         op.bad = (int *)c->bad.p;
@@ -328,11 +335,11 @@ struct Launcher {
         KMaps mp;
         mp.halo = *c->tensor_map(MAP_HALO, Op::NH_);
         for (int k = 0; k < Op::NG; k++) mp.grp[k] = *c->tensor_map(Op::gm(k) ? MAP_MODEL : MAP_PLAIN, Op::gd(k));
-        // A dependent launch pays while the grid leaves slots free: its start is
-        // then hidden.  A launch that fills the GPU can only take the slots that come free first and end unevenly spread
-        // over the SMs (4000 x 1200: 110 against 100 us a step; 300 x 100:
-        // 10 against 12 us).
-        const bool dep = c->pdl && grid < occ[d] * c->num_sms;
+        // A dependent launch hides the start of a kernel behind the end of the
+        // preceding one (the blocks may start when its last tiles have been
+        // issued): 2000 x 600 visco 14.3 to 13.0 ms a forward loop, 4000 x
+        // 1200 P-SV 16.6 to 15.1.  Op::DEP_TILES says where it does not pay.
+        const bool dep = c->pdl && ntiles <= (long long)Op::DEP_TILES * grid;
         launch_dep(c->st, dep, kern, dim3(grid), dim3(32, P::NCW + 1), P::bytes(), mp, op, nshots,
                    (int *)c->bad.p);
     }
@@ -374,14 +381,12 @@ struct Launcher {
             bool done = false;
             if constexpr (FD >= 5) {
                 if (g.quirk_hi) {
-                    pipelined(OpSVisc<FD, kTileY, LL, NST, true>{g, S, M, c->ktma, snap_out(hin), src, nt_cur, fsurf,
-                                                                 fps, src_j0, src_j1});
+                    pipelined(OpSVisc<FD, kTileY, LL, NST, true>{g, S, M, c->ktma, snap_out(hin)});
                     done = true;
                 }
             }
             if (!done)
-                pipelined(OpSVisc<FD, kTileY, LL, NST, false>{g, S, M, c->ktma, snap_out(hin), src, nt_cur, fsurf, fps, src_j0,
-                                                              src_j1});
+                pipelined(OpSVisc<FD, kTileY, LL, NST, false>{g, S, M, c->ktma, snap_out(hin)});
         }
         if (c->sh) pipelined(OpSSh<FD, kTileY, LL, ring_stages<FD, 1, 2 + 2 * LL + 4, 0, kTileY, 3>()>{g, S, M, c->ktma, snap_out(hin)});
     }
@@ -423,11 +428,11 @@ struct Launcher {
                     bool done = false;
                     if constexpr (FD >= 5) {
                         if (quirk) {
-                            pipelined(OpSEl<FD, kTileY, NST, true>{g, S, M, t, snap_out(hin), src, nt_cur, fsurf, fps, src_j0, src_j1});
+                            pipelined(OpSEl<FD, kTileY, NST, true>{g, S, M, t, snap_out(hin)});
                             done = true;
                         }
                     }
-                    if (!done) pipelined(OpSEl<FD, kTileY, NST, false>{g, S, M, t, snap_out(hin), src, nt_cur, fsurf, fps, src_j0, src_j1});
+                    if (!done) pipelined(OpSEl<FD, kTileY, NST, false>{g, S, M, t, snap_out(hin)});
                 }
                 if (c->sh) pipelined(OpSSh<FD, kTileY, 0, ring_stages<FD, 1, 4, 0, kTileY, sblocks(FD)>()>{g, S, M, t, snap_out(hin)});
                 break;
@@ -482,13 +487,13 @@ struct Launcher {
     // the explosive sources, free surface and receivers of a forward step
     void post_fwd(int nt, bool psource, const KSnapPatch &pt) {
         const KGrid &g = c->g;
-        if (!fps && (psource || c->p.free_surf)) {
+        if (!surf_fused && (psource || c->p.free_surf)) {
             const dim3 gs((unsigned)((c->p.nx + 127) / 128), (unsigned)nshots);
             DISPATCH_FDOH(g.fdoh, launch_dep(c->st, c->pdl, k_surface_src<T, FD>, gs, dim3(128), 0, g, S, M, src, nt,
                                              c->psv, c->sh, c->ac, psource ? 1 : 0, c->p.free_surf ? 1 : 0, pt));
             c->launches++;
         }
-        if (seis_fused) return;  // the velocity op sampled the receivers and probed for NaN
+        if (seis_fused) return;  // the ops sampled the receivers and probed for NaN
         const dim3 gr((unsigned)((std::max(1, c->p.max_rec) + 127) / 128), (unsigned)nshots);
         DISPATCH_FDOH(g.fdoh, launch_dep(c->st, c->pdl, k_seismo<T, FD>, gr, dim3(128), 0, g, S, M, rec, nt,
                                          c->p.seismo, c->psv, c->sh, c->ac, (int *)c->bad.p));
@@ -502,7 +507,7 @@ struct Launcher {
             launch_dep(c->st, c->pdl, k_psource_adj<T>, gr, dim3(128), 0, g, S, rec, nt, c->ac);
             c->launches++;
         }
-        if (c->p.free_surf && !fsurf) {
+        if (c->p.free_surf && !surf_fused) {
             const dim3 gs((unsigned)((c->p.nx + 127) / 128), (unsigned)nshots);
             DISPATCH_FDOH(g.fdoh, launch_dep(c->st, c->pdl, k_surface_src<T, FD>, gs, dim3(128), 0, g, S, M, src, nt,
                                              c->psv, c->sh, c->ac, 0, 1, KSnapPatch{}));

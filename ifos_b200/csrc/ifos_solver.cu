@@ -819,6 +819,19 @@ static int run_loop(ifos_ctx *c, LoopGraph &lg, const std::string &key, F &&enqu
     return IFOS_OK;
 }
 
+// Whether the SH and acoustic ops handle the receivers themselves.  That saves
+// launches of a few microseconds, but the tiles that hold receivers wait for
+// their scattered samples, so it pays while such tiles (a row of them per
+// shot, usually) fall to few of the blocks; in larger batches a receiver
+// kernel of its own is hidden behind the next launch's start.  Per step with
+// and without: SH 400 x 160 FDORDER 12, 1, 16 and 32 shots 7.6 / 8.2, 20.3 /
+// 22.1 and 36.4 / 36.7 us; acoustic 1500 x 500 FDORDER 8, 2, 4 and 8 shots 19.4
+// / 21.9, 35.6 / 34.9 and 70.8 / 63.4.  The P-SV ops always do.
+static bool rec_in_op(const ifos_ctx *c, int nshots) {
+    const long long tiles = (long long)nshots * ((c->p.nx + kTileX - 1) / kTileX);
+    return (c->psv && !c->ac) || 3 * tiles <= 2LL * c->num_sms;
+}
+
 static std::string loop_key(const ifos_ctx *c, std::initializer_list<long long> v) {
     std::string k;
     for (long long x : v) k += std::to_string(x) + ",";
@@ -846,16 +859,23 @@ static int forward_t(ifos_ctx *c, int nshots, int store, int nsteps) {
     // holding them are stored again after it
     const bool fused = snaps && c->pipe && c->fused_snap;
     const bool f16s = p.snap_format == IFOS_SNAP_F16S || p.snap_format == IFOS_SNAP_I16S;  // 16-bit segments
-    // P-SV elastic / viscoelastic: the stress kernel applies the explosive
-    // sources and the free surface, so nothing changes a stress after it
-    // (no surface kernel, no snapshot patches)
-    const bool in_stress = c->pipe && c->psv && !c->ac && !c->sh;
-    Lr.fps = in_stress ? 1 : 0;
+    // One wave type on the pipelined path: the stress (pressure) kernel applies
+    // the explosive sources and the free surface, so nothing changes a stress
+    // after it (no surface kernel, no snapshot patches), and the SH velocity
+    // kernel the force sources
+    const bool in_stress = c->pipe && !(c->psv && c->sh);
+    const bool sh_only = in_stress && c->sh;
+    Lr.surf_fused = in_stress;
+    Lr.fps = in_stress && c->psv ? 1 : 0;
     Lr.fsurf = (in_stress && p.free_surf) ? 1 : 0;
-    // P-SV without force sources, SEISMO 1: vx, vy are final when the velocity
-    // op stores them, so it samples the receivers itself (and probes for NaN)
+    Lr.fvs = sh_only ? 1 : 0;
+    // Without other force sources vx, vy (SEISMO 1, or vz) and the acoustic
+    // pressure (SEISMO 2) are final when their kernel stores them, so it
+    // samples the receivers itself (and the velocity kernel probes for NaN)
     const bool rec_ok = Lr.receiver_rows();
-    const bool seis_fused = std::is_same<T, float>::value && in_stress && !force && p.seismo == 1 && rec_ok;
+    const bool force_kernel = force && !sh_only;
+    const bool seis_fused = in_stress && !force_kernel && rec_ok && rec_in_op(c, nshots) &&
+                            (p.seismo == 1 || (c->ac && p.seismo == 2));
     Lr.seis_fused = seis_fused;
     {
         const int ms = std::max(1, p.max_src);
@@ -894,11 +914,12 @@ static int forward_t(ifos_ctx *c, int nshots, int store, int nsteps) {
         Lr.nt_cur = nt;
         {
             KTimer t(c, 0, sample);
-            Lr.rec_mode = seis_fused ? 1 : 0;
+            Lr.v_rec = seis_fused && p.seismo == 1 ? 1 : 0;
+            Lr.v_probe = seis_fused ? 1 : 0;
+            Lr.s_rec = seis_fused && p.seismo == 2 ? 1 : 0;
             Lr.v_step(0, snap_now ? 1 : 0, fhin);
-            Lr.rec_mode = 0;
         }
-        if (force) {
+        if (force_kernel) {
             launch_dep(c->st, c->pdl, k_inject_v_fwd<T>, dim3(nshots), dim3(32), 0, c->g, Lr.S, Lr.M, Lr.src, nt, c->psv && !c->ac ? 1 : (c->ac ? 1 : 0),
                                                         c->sh);
             c->launches++;
@@ -995,9 +1016,6 @@ template <typename T>
 static int adjoint_t(ifos_ctx *c, int nshots) {
     const ifos_params &p = c->p;
     Launcher<T> Lr(c, nshots);
-    // P-SV elastic / viscoelastic without the pressure residual source: the
-    // stress kernel applies the free surface (no surface kernel)
-    Lr.fsurf = (c->pipe && c->psv && !c->ac && !c->sh && p.free_surf && p.adjoint_type != 4) ? 1 : 0;
     if (int rc = zero_state<T>(c, nshots)) return rc;
     const long long N = (long long)p.nx * p.ny;
     CK(cudaMemsetAsync(c->gacc.p, 0, (size_t)nshots * 5 * N * 4, c->st));
@@ -1008,11 +1026,19 @@ static int adjoint_t(ifos_ctx *c, int nshots) {
     const int ntd = p.nt / p.dtinv;
     const int mr = std::max(1, p.max_rec);
     dim3 gr_rec((mr + 127) / 128, nshots);
-    // P-SV (elastic or viscoelastic) on the pipelined path: the velocity op
-    // adds the residual sources itself
-    const bool rec_ok = Lr.receiver_rows();
-    const bool inj_fused = std::is_same<T, float>::value && c->pipe && c->psv && !c->ac && !c->sh &&
-                           p.adjoint_type >= 1 && p.adjoint_type <= 3 && rec_ok;
+    // One wave type on the pipelined path: the velocity kernel adds the residual
+    // sources itself, the pressure kernel those of ADJOINT_TYPE 4, and the
+    // stress kernel applies the free surface (unless the pressure residual
+    // comes in between from its own kernel)
+    const bool one = c->pipe && !(c->psv && c->sh);
+    const bool rec_ok = Lr.receiver_rows() && rec_in_op(c, nshots);
+    const bool v_inj = c->sh || (p.adjoint_type >= 1 && p.adjoint_type <= 3);  // the velocities take residuals
+    const bool inj_fused = one && rec_ok && v_inj;
+    const bool p_inj = p.adjoint_type == 4, p_fused = one && rec_ok && p_inj && c->ac;
+    Lr.surf_fused = one && p.free_surf && (!p_inj || p_fused || c->sh);
+    Lr.fsurf = Lr.surf_fused ? 1 : 0;
+    Lr.v_rec = inj_fused ? 2 : 0;
+    Lr.s_rec = p_fused ? 2 : 0;
     CK(cudaEventRecord(c->ev0, c->st));
     auto enqueue = [&]() {
     int hin_a = 1;
@@ -1021,9 +1047,7 @@ static int adjoint_t(ifos_ctx *c, int nshots) {
         Lr.nt_cur = nt;
         {
             KTimer t(c, 0, sample);
-            Lr.rec_mode = inj_fused ? 2 : 0;
             Lr.v_step(1, 0);
-            Lr.rec_mode = 0;
         }
         if (!inj_fused && ((c->psv && p.adjoint_type >= 1 && p.adjoint_type <= 3) || c->sh)) {
             launch_dep(c->st, c->pdl, k_inject_v_adj<T>, dim3(gr_rec), dim3(128), 0, c->g, Lr.S, Lr.rec, nt, c->psv ? 1 : 0, c->sh && !c->ac);
@@ -1035,7 +1059,7 @@ static int adjoint_t(ifos_ctx *c, int nshots) {
             KTimer t(c, 1, sample);
             Lr.s_step();
         }
-        Lr.post_adj(nt, p.adjoint_type == 4);
+        Lr.post_adj(nt, p_inj && !p_fused);
         if (snap_step) {
             KTimer t(c, 3, sample);
             bool cells = false;
@@ -1051,7 +1075,7 @@ static int adjoint_t(ifos_ctx *c, int nshots) {
     launch_dep(c->st, c->pdl, k_assemble<T>, dim3(Lr.grd), dim3(Lr.blk), 0, c->g, Lr.M, gr, c->psv, c->sh, c->ac);
     c->launches++;
     };
-    if (int rc = run_loop(c, c->gadj, loop_key(c, {1, nshots, inj_fused, Lr.rec_j0, Lr.rec_j1}), enqueue))
+    if (int rc = run_loop(c, c->gadj, loop_key(c, {1, nshots, inj_fused, p_fused, Lr.rec_j0, Lr.rec_j1}), enqueue))
         return rc;
     CK(cudaEventRecord(c->ev1, c->st));
     CK(cudaGetLastError());

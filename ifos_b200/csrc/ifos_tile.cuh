@@ -18,6 +18,7 @@
 // and with the same float/double promotions as the one-thread-per-cell
 // kernels of ifos_kernels.cuh.
 #pragma once
+#include <limits.h>
 #include <type_traits>
 
 #include "ifos_kernels.cuh"
@@ -52,6 +53,14 @@ constexpr int kTileX = 64;
 // against 82), and in the P-SV velocity of the wide stencils (4000 x 1200,
 // FDORDER 8: 47.1 against 49.8).
 constexpr int kCells = 4, kCellsVisc = 2;
+// Tiles a block up to which a launch of the P-SV elastic FDORDER 2 and 4 ops
+// is a programmatic dependent one (the others always are).  Their four blocks
+// of 96 registers fill the register file, and while the blocks of the
+// preceding launch leave one by one the next one's do not pack: 15 tiles a
+// block (64 shots of 400 x 160) took 47 instead of 38 ms a forward loop, 21
+// tiles 14.9 instead of 13.4, 5.4 tiles 56.6 instead of 53.6; below that the
+// hidden start wins (2.2 tiles: 4.0 instead of 4.75 ms).
+constexpr int kDepTiles = 5;
 constexpr int cells_v(int fdoh) { return fdoh <= 2 ? 4 : 2; }
 
 using D = std::conditional<IFOS_EXACT != 0, double, float>::type;
@@ -213,8 +222,8 @@ __device__ __forceinline__ int edge_warps(const Op &op, const TileInfo &ti) {
         const int a = ti.j0 + P::ROWS * w, b = a + P::ROWS - 1;
         bool e = b > g.ny || (strips && ((!g.free_surf && a <= g.fw) || b >= g.ny - g.fw + 1));
         e = e || (op.rec_mode && a <= op.rec_j1 && b >= op.rec_j0);
-        e = e || (op.rec_mode == 1 && (a == g.ny / 2 || b == g.ny / 2));
-        e = e || (op.fps && a <= op.src_j1 && b >= op.src_j0) || (op.fsurf && a == 1);
+        e = e || (op.probe && (a == g.ny / 2 || b == g.ny / 2));
+        e = e || ((op.fps || op.fvs) && a <= op.src_j1 && b >= op.src_j0) || (op.fsurf && a == 1);
         m |= e ? 1 << w : 0;
     }
     return m;
@@ -831,10 +840,11 @@ __device__ __noinline__ SurfVals<LL, V> surface_row(const KGrid &g, const KState
 struct RecIdx {
     int l[4];
 };
-__device__ __forceinline__ RecIdx rec_lookup(const KGrid &g, const KRec &rec, int slot, const Lane &q) {
+__device__ __forceinline__ RecIdx rec_lookup(const KGrid &g, const KRec &rec, bool one_row, int slot, const Lane &q) {
     RecIdx r{{-1, -1, -1, -1}};
     const int *m = rec.map + (long long)slot * rec.map_stride;
-    const int rr = q.nv > 0 ? m[q.j - 1] : -1;
+    // with one receiver row its index is 0 and the row table need not be read
+    const int rr = q.nv <= 0 ? -1 : (one_row ? 0 : m[q.j - 1]);
     if (rr < 0) return r;
     const int *cells = m + g.ny + (long long)rr * g.nx + (q.i - 1);
 #pragma unroll
@@ -864,19 +874,83 @@ static __device__ __noinline__ SxxSyy rec_row(const KGrid &g, const KRec &rec, i
     return v;
 }
 
+// One value per cell: the SH velocity (plane 2 of the seismograms) and the
+// acoustic pressure (plane 3, -p); both take component 2 of the adjoint
+// sources (src/seismo_ssg.c, src/update_v_PML_SH.c, src/psource.c:61-74).
+struct Cells4 {
+    float v[4];
+};
+template <bool PRESSURE>
+__device__ __noinline__ Cells4 rec_row1(const KGrid &g, const KRec &rec, int mode, int slot, int nt, RecIdx r, Cells4 v) {
+    const long long cs = (long long)rec.max_rec * g.nt_total;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        if (r.l[e] < 0) continue;
+        const long long o = (long long)r.l[e] * g.nt_total + nt - 1;
+        if (mode == 2) v.v[e] += rec.adj[(long long)slot * 3 * cs + 2 * cs + o];
+        else rec.sec[(long long)slot * 6 * cs + (PRESSURE ? 3 : 2) * cs + o] = PRESSURE ? -v.v[e] : v.v[e];
+    }
+    return v;
+}
+__device__ __forceinline__ bool any_receiver(const RecIdx &r) {
+    return max(max(r.l[0], r.l[1]), max(r.l[2], r.l[3])) >= 0;
+}
+
+// Explosive sources on the acoustic pressure (psource_apply), in list order.
+static __device__ __noinline__ Cells4 psource_row_p(const KGrid &g, const KSrc &src, int slot, int nt, Lane q, Cells4 v) {
+    const float *pos = src.pos + (long long)slot * 8 * src.max_src;
+    const int n = src.nsrc[slot];
+    const float x0 = pos[0], y0 = pos[src.max_src], type0 = pos[7 * src.max_src];  // requested with the count
+    const float amp0 = psource_amp(src, slot, 0, nt, g.dh);
+    if (n <= 0 || (int)(n == 1 ? type0 : pos[7 * src.max_src + n - 1]) != 1) return v;  // psource_fires
+    for (int l = 0; l < n; l++) {
+        const int e = (int)(l ? pos[l] : x0) - q.i;
+        if ((int)(l ? pos[src.max_src + l] : y0) != q.j || e < 0 || e >= q.nv) continue;
+        const float amp = l ? psource_amp(src, slot, l, nt, g.dh) : amp0;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (e == k) v.v[k] += amp;
+    }
+    return v;
+}
+// Force sources on the SH velocity, as src/update_v_PML_SH.c:327-333 adds
+// them after the update, in list order; rjp: the cells' reciprocal densities.
+static __device__ __noinline__ Cells4 force_row_sh(const KGrid &g, const KSrc &src, int slot, int nt, Lane q, Cells4 rjp,
+                                                   Cells4 v) {
+    const float *pos = src.pos + (long long)slot * 8 * src.max_src;
+    const float *sig = src.sig + (long long)slot * src.max_src * src.nt_total + nt - 1;
+    const int n = src.nsrc[slot];
+    const float x0 = pos[0], y0 = pos[src.max_src], a0 = sig[0];  // requested with the count
+    const float DT = g.dt, DH = g.dh;
+    for (int l = 0; l < n; l++) {
+        const int e = (int)(l ? pos[l] : x0) - q.i;
+        if ((int)(l ? pos[src.max_src + l] : y0) != q.j || e < 0 || e >= q.nv) continue;
+        const float a = l ? sig[(long long)l * src.nt_total] : a0;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (e == k)
+                v.v[k] = (float)((double)v.v[k] + ((double)(rjp.v[k] * DT) * 1.0 * (double)a) / (double)(DH * DH));
+    }
+    return v;
+}
+
 // rows<true> runs on warps whose rows of the tile need anything beyond the
 // plain update (TileInfo::edge), rows<false> on the others.  prefetch starts
 // the loads of the CPML memories that rows<true> uses (Pre); they are written
 // by the op's own previous launch only, which has completed before this one
 // starts.
 // the common members of an op
-// src, nt, fsurf, fps: the stress ops apply the explosive sources of step nt
-// (fps; rows src_j0..src_j1 hold every slot's sources) and the free surface
-// of row 1 (fsurf) themselves
-// rec_mode (P-SV velocity ops): 1 the forward samples vx, vy at the
-// receivers into the seismograms (SEISMO 1) and probes the centre cell for
-// NaN, 2 the adjoint adds the residual sources at the receivers; rows
-// rec_j0..rec_j1 hold every slot's receivers.
+// nt: the time step.  What the ops do beside the update, so that a step needs
+// no other kernel:
+// fps: the stress and pressure ops apply the explosive sources of step nt,
+// fsurf: and the free surface of row 1;
+// fvs: the SH velocity op applies the force sources (rows src_j0..src_j1 hold
+// every slot's sources);
+// rec_mode 1: the op copies its new values at the receivers into the
+// seismograms (P-SV and acoustic velocity: vx, vy; SH velocity: vz; pressure:
+// -p), 2: it adds the adjoint sources there (rows rec_j0..rec_j1 hold every
+// slot's receivers);
+// probe: the velocity op checks the centre cell for NaN.
 #define IFOS_OP_MEMBERS \
     KGrid g;            \
     KState<float> S;    \
@@ -887,6 +961,8 @@ static __device__ __noinline__ SxxSyy rec_row(const KGrid &g, const KRec &rec, i
     int nt;             \
     int fsurf;          \
     int fps;            \
+    int fvs;            \
+    int probe;          \
     int src_j0, src_j1; \
     KRec rec;           \
     int rec_mode;       \
@@ -901,6 +977,7 @@ static __device__ __noinline__ SxxSyy rec_row(const KGrid &g, const KRec &rec, i
 template <int FDOH, int TY, int LL, int NST, bool QUIRK>
 struct OpSVisc {
     static constexpr int V = kCellsVisc;
+    static constexpr int DEP_TILES = INT_MAX;
     static constexpr int NH_ = 2, NP_ = 3 + 3 * LL + 6;
     static constexpr bool CPML = !QUIRK, MIRROR = false;
     using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, visc_blocks(LL), V>;
@@ -1070,6 +1147,7 @@ struct OpSVisc {
 template <int FDOH, int TY, int NST, bool QUIRK>
 struct OpSEl {
     static constexpr int V = kCells;
+    static constexpr int DEP_TILES = FDOH <= 2 ? kDepTiles : INT_MAX;
     static constexpr int NH_ = 2, NP_ = 6;
     static constexpr bool CPML = !QUIRK, MIRROR = false;
     using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, sblocks(FDOH), V>;
@@ -1194,6 +1272,7 @@ struct OpSEl {
 template <int FDOH, int TY, int NST, bool QUIRK, int SW, bool P1, bool AC>
 struct OpVPsv {
     static constexpr int V = cells_v(FDOH);
+    static constexpr int DEP_TILES = FDOH <= 2 && !AC ? kDepTiles : INT_MAX;
     static constexpr int NH_ = AC ? 1 : 3;
     static constexpr int NP_ = (SW == 1 && !QUIRK) ? 6 : 4;
     static constexpr bool CPML = !QUIRK, MIRROR = true;
@@ -1216,7 +1295,7 @@ struct OpVPsv {
     };
     __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
         const Lane q = Lane::of<true, V>(g, ti);
-        if (rec_mode && q.j >= rec_j0 && q.j <= rec_j1) pre.rec = rec_lookup(g, rec, ti.slot, q);
+        if (rec_mode && q.j >= rec_j0 && q.j <= rec_j1) pre.rec = rec_lookup(g, rec, rec_j0 == rec_j1, ti.slot, q);
         else pre.rec = RecIdx{{-1, -1, -1, -1}};
         if (!CPML) return;
         psi_x<V>(g, S.psix[X_SXX] + ti.slot * S.psix_slot, q, pre.x0);
@@ -1318,8 +1397,8 @@ struct OpVPsv {
                 o[1][e] = vyo.v[e] + fy[e];
             }
         }
-        if (EDGE && rec_mode && q.nv > 0) {
-            if (max(max(pre.rec.l[0], pre.rec.l[1]), max(pre.rec.l[2], pre.rec.l[3])) >= 0) {
+        if (EDGE && q.nv > 0) {
+            if (any_receiver(pre.rec)) {
                 SxxSyy v{};
 #pragma unroll
                 for (int e = 0; e < V; e++) v.xx[e] = o[0][e], v.yy[e] = o[1][e];
@@ -1327,7 +1406,7 @@ struct OpVPsv {
 #pragma unroll
                 for (int e = 0; e < V; e++) o[0][e] = v.xx[e], o[1][e] = v.yy[e];
             }
-            if (rec_mode == 1 && q.j == g.ny / 2) {  // the instability probe of the driver (src/IFOS2D.c:1660-1672)
+            if (probe && q.j == g.ny / 2) {  // the instability probe of the driver (src/IFOS2D.c:1660-1672)
                 const int at = g.nx / 2 - q.i;
 #pragma unroll
                 for (int e = 0; e < V; e++)
@@ -1353,6 +1432,7 @@ struct OpVPsv {
 template <int FDOH, int TY, int NST>
 struct OpVSh {
     static constexpr int V = kCells;
+    static constexpr int DEP_TILES = INT_MAX;
     static constexpr int NH_ = 2, NP_ = 2;
     static constexpr bool CPML = true, MIRROR = true;
     using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, vblocks(FDOH), V>;
@@ -1369,10 +1449,13 @@ struct OpVSh {
     }
     struct Pre {
         Psi<V> x0, y0;
+        RecIdx rec;
     };
     __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
-        if (!CPML) return;
         const Lane q = Lane::of<true, V>(g, ti);
+        if (rec_mode && q.j >= rec_j0 && q.j <= rec_j1) pre.rec = rec_lookup(g, rec, rec_j0 == rec_j1, ti.slot, q);
+        else pre.rec = RecIdx{{-1, -1, -1, -1}};
+        if (!CPML) return;
         psi_x<V>(g, S.psix[X_SXZ] + ti.slot * S.psix_slot, q, pre.x0);
         psi_y<V>(g, S.psiy[Y_SYZ] + ti.slot * S.psiy_slot, q, pre.y0);
     }
@@ -1403,6 +1486,24 @@ struct OpVSh {
         div_dh(g, f);
 #pragma unroll
         for (int e = 0; e < V; e++) o[e] = vz.v[e] + f[e];
+        if (EDGE && q.nv > 0) {
+            const bool force = fvs && q.j >= src_j0 && q.j <= src_j1;
+            if (force || any_receiver(pre.rec)) {
+                Cells4 v{}, r{};
+#pragma unroll
+                for (int e = 0; e < V; e++) v.v[e] = o[e], r.v[e] = rjp.v[e];
+                if (force) v = force_row_sh(g, src, slot, nt, q, r, v);
+                if (any_receiver(pre.rec)) v = rec_row1<false>(g, rec, rec_mode, slot, nt, pre.rec, v);
+#pragma unroll
+                for (int e = 0; e < V; e++) o[e] = v.v[e];
+            }
+            if (probe && q.j == g.ny / 2) {
+                const int at = g.nx / 2 - q.i;
+#pragma unroll
+                for (int e = 0; e < V; e++)
+                    if (e == at && e < q.nv && isnan(o[e])) atomicExch(bad, 1);
+            }
+        }
         const RowOut<EDGE, V> out(g, S, slot, q);
         out.put(S.off[P_VZP1], vz.v);
         out.put(S.off[P_VZ], o);
@@ -1416,6 +1517,7 @@ struct OpVSh {
 template <int FDOH, int TY, int LL, int NST>
 struct OpSSh {
     static constexpr int V = kCells;
+    static constexpr int DEP_TILES = INT_MAX;
     static constexpr int NH_ = 1, NP_ = LL ? 2 + 2 * LL + 4 : 4, L1 = LL > 0 ? LL : 1;
     static constexpr bool CPML = true, MIRROR = false;
     using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, LL ? 3 : sblocks(FDOH), V>;
@@ -1523,6 +1625,10 @@ struct OpSSh {
                 o[1][e] = o[1][e] + (dthalbe * sumt[e]);
             }
         }
+        if (EDGE && fsurf && q.j == 1) {  // src/surface_elastic_PML.c, SH: syz = 0
+#pragma unroll
+            for (int e = 0; e < V; e++) o[1][e] = 0.0f;
+        }
         out.put(S.off[P_SXZ], o[0]);
         out.put(S.off[P_SYZ], o[1]);
         if (so.base) {
@@ -1537,6 +1643,7 @@ struct OpSSh {
 template <int FDOH, int TY, int NST, bool QUIRK>
 struct OpPAc {
     static constexpr int V = kCells;
+    static constexpr int DEP_TILES = INT_MAX;
     static constexpr int NH_ = 2, NP_ = 2;
     static constexpr bool CPML = !QUIRK, MIRROR = false;
     using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, sblocks(FDOH), V>;
@@ -1553,10 +1660,13 @@ struct OpPAc {
     }
     struct Pre {
         Psi<V> x0, y0;
+        RecIdx rec;
     };
     __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
-        if (!CPML) return;
         const Lane q = Lane::of<true, V>(g, ti);
+        if (rec_mode && q.j >= rec_j0 && q.j <= rec_j1) pre.rec = rec_lookup(g, rec, rec_j0 == rec_j1, ti.slot, q);
+        else pre.rec = RecIdx{{-1, -1, -1, -1}};
+        if (!CPML) return;
         psi_x<V>(g, S.psix[X_VXX] + ti.slot * S.psix_slot, q, pre.x0);
         psi_y<V>(g, S.psiy[Y_VYY] + ti.slot * S.psiy_slot, q, pre.y0);
     }
@@ -1595,6 +1705,21 @@ struct OpPAc {
 #pragma unroll
             for (int e = 0; e < V; e++) o[e] = sp.v[e] + gg.v[e] * (vxx[e] + vyy[e]);
         }
+        if (EDGE && q.nv > 0) {
+            // sources or adjoint sources, then the free surface, then the receivers
+            const bool source = fps && q.j >= src_j0 && q.j <= src_j1, surface = fsurf && q.j == 1;
+            if (source || surface || any_receiver(pre.rec)) {
+                Cells4 v{};
+#pragma unroll
+                for (int e = 0; e < V; e++) v.v[e] = o[e];
+                if (source) v = psource_row_p(g, src, slot, nt, q, v);
+                if (rec_mode == 2 && any_receiver(pre.rec)) v = rec_row1<true>(g, rec, 2, slot, nt, pre.rec, v);
+                if (surface) v = Cells4{};
+                if (rec_mode == 1 && any_receiver(pre.rec)) v = rec_row1<true>(g, rec, 1, slot, nt, pre.rec, v);
+#pragma unroll
+                for (int e = 0; e < V; e++) o[e] = v.v[e];
+            }
+        }
         RowOut<EDGE, V>(g, S, slot, q).put(S.off[P_SP], o);
         if (so.base) snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SP], o);
     }
@@ -1607,6 +1732,7 @@ struct OpPAc {
 template <int FDOH, int TY, int LL, int NST>
 struct OpPVisc {
     static constexpr int V = kCells;
+    static constexpr int DEP_TILES = INT_MAX;
     static constexpr bool Z0 = FDOH != 1, CPML = !Z0, MIRROR = false;
     static constexpr int NH_ = 2, NP_ = 3 + LL;
     using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, 3, V>;
@@ -1624,10 +1750,13 @@ struct OpPVisc {
     }
     struct Pre {
         Psi<V> x0, y0;
+        RecIdx rec;
     };
     __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
-        if (!CPML) return;
         const Lane q = Lane::of<true, V>(g, ti);
+        if (rec_mode && q.j >= rec_j0 && q.j <= rec_j1) pre.rec = rec_lookup(g, rec, rec_j0 == rec_j1, ti.slot, q);
+        else pre.rec = RecIdx{{-1, -1, -1, -1}};
+        if (!CPML) return;
         psi_x<V>(g, S.psix[X_VXX] + ti.slot * S.psix_slot, q, pre.x0);
         psi_y<V>(g, S.psiy[Y_VYY] + ti.slot * S.psiy_slot, q, pre.y0);
     }
@@ -1686,6 +1815,21 @@ struct OpPVisc {
         }
 #pragma unroll
         for (int e = 0; e < V; e++) o[e] = o[e] + (dthalbe * sump[e]);
+        if (EDGE && q.nv > 0) {
+            // sources or adjoint sources, then the free surface, then the receivers
+            const bool source = fps && q.j >= src_j0 && q.j <= src_j1, surface = fsurf && q.j == 1;
+            if (source || surface || any_receiver(pre.rec)) {
+                Cells4 v{};
+#pragma unroll
+                for (int e = 0; e < V; e++) v.v[e] = o[e];
+                if (source) v = psource_row_p(g, src, slot, nt, q, v);
+                if (rec_mode == 2 && any_receiver(pre.rec)) v = rec_row1<true>(g, rec, 2, slot, nt, pre.rec, v);
+                if (surface) v = Cells4{};
+                if (rec_mode == 1 && any_receiver(pre.rec)) v = rec_row1<true>(g, rec, 1, slot, nt, pre.rec, v);
+#pragma unroll
+                for (int e = 0; e < V; e++) o[e] = v.v[e];
+            }
+        }
         out.put(S.off[P_SP], o);
         if (so.base) snap<EDGE, V>(g, so, slot, q, tm.snap_comp[P_SP], o);
     }

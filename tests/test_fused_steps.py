@@ -1,0 +1,62 @@
+"""Sources, receivers and the free surface inside the SH and acoustic
+kernels: receiver layouts that fit the cell map and ones that do not, sources
+that share a cell or a row with receivers, both seismogram and adjoint types.
+Bit-identical to the oracle."""
+import numpy as np
+import pytest
+
+from ifos_b200 import workloads as W
+from tests.golden.cases import build_case
+from tests.gpu_helpers import bit_equal, forward_fields_mask, gpu_shot, oracle_shot
+
+pytestmark = pytest.mark.gpu
+
+
+def _receivers(p, layout):
+    if layout == "three_rows":
+        xs = np.concatenate([np.arange(10, 55, 4), np.arange(12, 50, 5), np.arange(9, 57, 6)])
+        ys = np.concatenate([np.full(12, 3), np.full(8, 11), np.full(8, 20)])
+    elif layout == "vertical_line":  # more rows than the cell map holds: the separate receiver kernels
+        ys = np.arange(3, 36, 3)
+        xs = np.full(ys.shape, 30)
+    elif layout == "surface":
+        xs, ys = np.arange(5, 60, 7), np.full(8, 1)
+    else:  # the probe's cell, and the last cells of a row
+        xs, ys = np.array([p.nx // 2, p.nx, p.nx - 1, 1]), np.array([p.ny // 2, 3, 3, 3])
+    return np.stack([xs, ys]).astype(np.int32)
+
+
+@pytest.mark.parametrize("layout", ["three_rows", "vertical_line", "surface", "centre"])
+@pytest.mark.parametrize("name,seismo,adjoint_type", [("sh_el_o6", 1, 1), ("sh_visc_o4", 1, 1), ("acoustic_o4_p", 2, 4),
+                                                      ("acoustic_o4_p", 1, 1), ("acoustic_o4_p", 1, 2),
+                                                      ("acoustic_o4_p", 5, 4), ("ac_visc_o4_p", 2, 4),
+                                                      ("ac_visc_o2_nofs", 2, 4)])
+def test_receivers(name, seismo, adjoint_type, layout):
+    p, model, g, sig, _ = build_case(name, nt=60)
+    p.seismo, p.adjoint_type = seismo, adjoint_type
+    rec = _receivers(p, layout)
+    g = W.Geometry(g.srcpos, rec)
+    adj = (np.random.default_rng(5).standard_normal((3, rec.shape[1], p.nt)) * 1e-3).astype(np.float32)
+    gpu, ref = gpu_shot(p, model, g, sig, adj), oracle_shot(p, model, g, sig, adj)
+    m = forward_fields_mask()
+    for key in ("sections", "grads", "adj_fields"):
+        assert bit_equal(gpu[key], ref[key]), key
+    assert bit_equal(gpu["fields"][m], ref["fields"][m]), "fields"
+    if layout != "surface":  # the pressure of row 1 is zero
+        assert np.abs(ref["sections"]).max() > 0 and np.abs(ref["grads"]).max() > 0
+
+
+@pytest.mark.parametrize("cells", [[(30, 3), (30, 3)], [(30, 1), (31, 1), (33, 2)], [(64, 40), (1, 1), (17, 9), (18, 9)]])
+@pytest.mark.parametrize("name", ["sh_el_o6", "sh_visc_o4", "acoustic_o4_p", "ac_visc_o4_p", "psv_el_o4", "psv_visc_o4"])
+def test_several_sources(name, cells):
+    p, model, g, sig, adj = build_case(name, nt=60)
+    src = np.repeat(g.srcpos, len(cells), axis=1)
+    for k, (i, j) in enumerate(cells):
+        src[0, k], src[1, k] = i, j
+    sig = np.concatenate([sig * np.float32(1.0 + 0.3 * k) for k in range(len(cells))])
+    g = W.Geometry(np.ascontiguousarray(src), g.recpos)
+    gpu, ref = gpu_shot(p, model, g, sig, adj), oracle_shot(p, model, g, sig, adj)
+    m = forward_fields_mask()
+    for key in ("sections", "grads"):
+        assert bit_equal(gpu[key], ref[key]), key
+    assert bit_equal(gpu["fields"][m], ref["fields"][m]), "fields"
