@@ -336,10 +336,7 @@ struct Vec {
     float v[V];
     __device__ __forceinline__ static Vec load(const float *p) {
         Vec r;
-        if constexpr (V == 4) {
-            const float4 a = *reinterpret_cast<const float4 *>(p);
-            r.v[0] = a.x, r.v[1] = a.y, r.v[2] = a.z, r.v[3] = a.w;
-        } else if constexpr (V == 2) {
+        if constexpr (V == 2) {
             const float2 a = *reinterpret_cast<const float2 *>(p);
             r.v[0] = a.x, r.v[1] = a.y;
         } else {
@@ -348,18 +345,13 @@ struct Vec {
         return r;
     }
     __device__ __forceinline__ void store(float *p) const {
-        if constexpr (V == 4) *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-        else if constexpr (V == 2) *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+        if constexpr (V == 2) *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
         else *p = v[0];
     }
     // 16-bit segment values times the segment's scale
     __device__ __forceinline__ static Vec load16(const unsigned short *p, float sc, bool i16) {
         unsigned short h[V];
-        if constexpr (V == 4) {
-            const uint2 a = *reinterpret_cast<const uint2 *>(p);
-            h[0] = (unsigned short)a.x, h[1] = (unsigned short)(a.x >> 16), h[2] = (unsigned short)a.y,
-            h[3] = (unsigned short)(a.y >> 16);
-        } else if constexpr (V == 2) {
+        if constexpr (V == 2) {
             const unsigned a = *reinterpret_cast<const unsigned *>(p);
             h[0] = (unsigned short)a, h[1] = (unsigned short)(a >> 16);
         } else {
@@ -374,8 +366,9 @@ struct Vec {
 
 // Zero-lag correlation for fp32 state and fp32 or 16-bit-segment snapshots:
 // the arithmetic of k_correlate per cell, V adjacent cells of a row per thread
-// (V the largest of 4, 2, 1 that divides NX: rows of the snapshots and sums
-// then start V-aligned, and no group straddles a 64-cell segment).  Threads
+// (V = 2 for an even NX, else 1: rows of the snapshots and sums then start
+// V-aligned, and no group straddles a 64-cell segment; four cells a thread
+// were no faster, 44.5 against 43.5 us on 64 shots of 400 x 160).  Threads
 // walk the groups of a slot row by row without gaps; grid: x over groups, y =
 // slot.  SEG: 0 fp32 snapshots, 1 fp16 segments, 2 int16 segments; ACC64: the
 // sums in double (gr.acc64).

@@ -991,17 +991,9 @@ static void correlate_physics(ifos_ctx *c, const Launcher<float> &L, const KSnap
 }
 template <int SEG>
 static void correlate_width(ifos_ctx *c, const Launcher<float> &L, const KSnap &sn, const KGrad &gr, int snap, int ns) {
-    const int v = c->p.nx % 4 == 0 ? 4 : (c->p.nx % 2 == 0 ? 2 : 1);
-    if (gr.acc64) {  // even NX only
-        if (v == 4) correlate_physics<SEG, 4, true>(c, L, sn, gr, snap, ns);
-        else correlate_physics<SEG, 2, true>(c, L, sn, gr, snap, ns);
-    } else if (v == 4) {
-        correlate_physics<SEG, 4, false>(c, L, sn, gr, snap, ns);
-    } else if (v == 2) {
-        correlate_physics<SEG, 2, false>(c, L, sn, gr, snap, ns);
-    } else {
-        correlate_physics<SEG, 1, false>(c, L, sn, gr, snap, ns);
-    }
+    if (gr.acc64) correlate_physics<SEG, 2, true>(c, L, sn, gr, snap, ns);  // even NX only
+    else if (c->p.nx % 2 == 0) correlate_physics<SEG, 2, false>(c, L, sn, gr, snap, ns);
+    else correlate_physics<SEG, 1, false>(c, L, sn, gr, snap, ns);
 }
 static bool correlate_cells(ifos_ctx *c, const Launcher<float> &L, const KSnap &sn, const KGrad &gr, int snap, int ns) {
     switch (c->p.snap_format) {
