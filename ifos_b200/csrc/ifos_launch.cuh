@@ -373,22 +373,32 @@ struct Launcher {
         }
         if (c->sh) pipelined(OpVSh<FD, kTileY, ring_stages<FD, 2, 2, 0, kTileY, vblocks(FD)>()>{c->g, S, M, c->ktma, snap_out(hin)});
     }
+    template <int FD, int LL, bool SHARED>
+    void s_visc_psv(int hin) {
+        const KGrid &g = c->g;
+        constexpr int NST = ring_stages<FD, 2, 3 + 3 * LL + (SHARED ? 0 : 6), 0, kTileY, visc_blocks(LL)>();
+        if constexpr (FD >= 5) {
+            if (g.quirk_hi) {
+                pipelined(OpSVisc<FD, kTileY, LL, NST, true, SHARED>{g, S, M, c->ktma, snap_out(hin)});
+                return;
+            }
+        }
+        pipelined(OpSVisc<FD, kTileY, LL, NST, false, SHARED>{g, S, M, c->ktma, snap_out(hin)});
+    }
     template <int FD, int LL>
     void s_visc_pipe(int hin) {
-        const KGrid &g = c->g;
-        constexpr int NST = ring_stages<FD, 2, 3 + 3 * LL + 6, 0, kTileY, visc_blocks(LL)>();
         if (c->psv) {
-            bool done = false;
-            if constexpr (FD >= 5) {
-                if (g.quirk_hi) {
-                    pipelined(OpSVisc<FD, kTileY, LL, NST, true>{g, S, M, c->ktma, snap_out(hin)});
-                    done = true;
-                }
-            }
-            if (!done)
-                pipelined(OpSVisc<FD, kTileY, LL, NST, false>{g, S, M, c->ktma, snap_out(hin)});
+            // OpSVisc's SHARED form pays when the state streams from HBM
+            // (above about twice the L2) and few tiles hold strip cells.  A
+            // forward step with and without: 2000 x 600, 2, 4, 6 and 12 shots 81
+            // / 80, 153 / 157, 220 / 234 and 439 / 500 us; 1300 x 400, 4, 8 and 24
+            // shots 69 / 67, 131 / 134 and 403 / 416; 593 x 246, 8 and 24 shots
+            // 46.0 / 44.5 and 134 / 136 (adjoint 150 / 145).
+            const long long cells = (long long)c->p.nx * c->p.ny;
+            if ((c->g.tile_order & 1) && cells >= 300000 && cells * nshots >= 4000000) s_visc_psv<FD, LL, true>(hin);
+            else s_visc_psv<FD, LL, false>(hin);
         }
-        if (c->sh) pipelined(OpSSh<FD, kTileY, LL, ring_stages<FD, 1, 2 + 2 * LL + 4, 0, kTileY, 3>()>{g, S, M, c->ktma, snap_out(hin)});
+        if (c->sh) pipelined(OpSSh<FD, kTileY, LL, ring_stages<FD, 1, 2 + 2 * LL + 4, 0, kTileY, 3>()>{c->g, S, M, c->ktma, snap_out(hin)});
     }
     template <int FD, int LL>
     void p_visc_pipe(int hin) {

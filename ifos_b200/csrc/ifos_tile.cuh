@@ -383,6 +383,10 @@ __device__ __forceinline__ void run_pipeline(const KGrid &g, const KMaps &mp, in
         const bool edge = ti.edge(warp);
         typename Op::Pre pre;
         if (edge) op.prefetch(ti, pre);
+        if constexpr (Op::EARLY) {
+            if (edge) op.template early<true>(ti, pre);
+            else op.template early<false>(ti, pre);
+        }
         bool landed = false;
         for (long it = 0; it < (1L << 16) && !landed; it++) {
             landed = mbar_try_wait(&full[st], parity);
@@ -974,16 +978,21 @@ static __device__ __noinline__ Cells4 force_row_sh(const KGrid &g, const KSrc &s
 // reference 10/12 default :615-660 has no CPML and zero-started sums: QUIRK)
 // halo: vx vy; plain: sxx syy sxy, r[LL] p[LL] q[LL], fipjp f g mu pi muipjp;
 // writes sxx syy sxy r p q.  Non-uniform tau planes are read from HBM.
-template <int FDOH, int TY, int LL, int NST, bool QUIRK>
+// SHARED: the shots of the launch walk the same tile side by side, so that all
+// but one of them find the model's coefficients in L2; they are then loaded
+// into registers before the wait for the stage instead of through the ring,
+// whose stages shrink from 46 to 34 KB and are three instead of two.
+template <int FDOH, int TY, int LL, int NST, bool QUIRK, bool SHARED>
 struct OpSVisc {
     static constexpr int V = kCellsVisc;
+    static constexpr bool EARLY = SHARED;
     static constexpr int DEP_TILES = INT_MAX;
-    static constexpr int NH_ = 2, NP_ = 3 + 3 * LL + 6;
+    static constexpr int NH_ = 2, NP_ = 3 + 3 * LL + (SHARED ? 0 : 6);
     static constexpr bool CPML = !QUIRK, MIRROR = false;
     using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, visc_blocks(LL), V>;
     IFOS_OP_MEMBERS
     // boxes of consecutive planes: their number, planes of box k, whether they are model planes
-    static constexpr int NG = 3;
+    static constexpr int NG = SHARED ? 2 : 3;
     __host__ __device__ static constexpr int gd(int k) { return k == 0 ? 3 : (k == 1 ? 3 * LL : 6); }
     __host__ __device__ static constexpr bool gm(int k) { return k == 2; }
     __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
@@ -991,11 +1000,20 @@ struct OpSVisc {
         hz = zb + tm.pid[P_VX];
         gz[0] = zb + tm.pid[P_SXX];
         gz[1] = zb + tm.mem_pid[0];
-        gz[2] = mb + tm.mid[M_FIPJPV];
+        if (!SHARED) gz[2 % NG] = mb + tm.mid[M_FIPJPV];
     }
+    // SHARED: fipjp f g mu pi muipjp of the thread's cells, loaded before the wait
     struct Pre {
+        FV<V> c[SHARED ? 6 : 1];
         Psi<V> x0, x1, y0, y1;
     };
+    template <bool EDGE>
+    __device__ __forceinline__ void early(const TileInfo &ti, Pre &pre) const {
+        const Lane q = Lane::of<EDGE, V>(g, ti);
+        const float *p = M.m[M_FIPJPV] + (long long)ti.model() * M.model_stride + (q.j - 1 + HY) * g.pitch + (q.i - 1 + HX);
+#pragma unroll
+        for (int k = 0; k < 6; k++) pre.c[k] = !EDGE || q.nv > 0 ? ldv<V>(p + k * g.plane) : FV<V>::of(0.0f);
+    }
     __device__ __forceinline__ void prefetch(const TileInfo &ti, Pre &pre) const {
         if (!CPML) return;
         const Lane q = Lane::of<true, V>(g, ti);
@@ -1042,9 +1060,11 @@ struct OpSVisc {
         }
         const float *in = pl + q.jj * kTileX + q.c;
         auto ld = [&](int k) { return ldv<V>(in + k * P::PLS); };
-        constexpr int CO = 3 + 3 * LL;  // first coefficient plane
-        const FV<V> s0 = ld(0), s1 = ld(1), s2 = ld(2), fipjp = ld(CO), f = ld(CO + 1), gg = ld(CO + 2);
-        const FV<V> mu = ld(CO + 3), pi = ld(CO + 4), muij = ld(CO + 5);
+        const FV<V> s0 = ld(0), s1 = ld(1), s2 = ld(2);
+        FV<V> co[6];
+#pragma unroll
+        for (int k = 0; k < 6; k++) co[k] = SHARED ? pre.c[SHARED ? k : 0] : ld(3 + 3 * LL + k);
+        const FV<V> &fipjp = co[0], &f = co[1], &gg = co[2], &mu = co[3], &pi = co[4], &muij = co[5];
         FV<V> mr[LL], mp[LL], mq[LL];
 #pragma unroll
         for (int l = 0; l < LL; l++) mr[l] = ld(3 + l), mp[l] = ld(3 + LL + l), mq[l] = ld(3 + 2 * LL + l);
@@ -1147,6 +1167,7 @@ struct OpSVisc {
 template <int FDOH, int TY, int NST, bool QUIRK>
 struct OpSEl {
     static constexpr int V = kCells;
+    static constexpr bool EARLY = false;
     static constexpr int DEP_TILES = FDOH <= 2 ? kDepTiles : INT_MAX;
     static constexpr int NH_ = 2, NP_ = 6;
     static constexpr bool CPML = !QUIRK, MIRROR = false;
@@ -1272,6 +1293,7 @@ struct OpSEl {
 template <int FDOH, int TY, int NST, bool QUIRK, int SW, bool P1, bool AC>
 struct OpVPsv {
     static constexpr int V = cells_v(FDOH);
+    static constexpr bool EARLY = false;
     static constexpr int DEP_TILES = FDOH <= 2 && !AC ? kDepTiles : INT_MAX;
     static constexpr int NH_ = AC ? 1 : 3;
     static constexpr int NP_ = (SW == 1 && !QUIRK) ? 6 : 4;
@@ -1432,6 +1454,7 @@ struct OpVPsv {
 template <int FDOH, int TY, int NST>
 struct OpVSh {
     static constexpr int V = kCells;
+    static constexpr bool EARLY = false;
     static constexpr int DEP_TILES = INT_MAX;
     static constexpr int NH_ = 2, NP_ = 2;
     static constexpr bool CPML = true, MIRROR = true;
@@ -1517,6 +1540,7 @@ struct OpVSh {
 template <int FDOH, int TY, int LL, int NST>
 struct OpSSh {
     static constexpr int V = kCells;
+    static constexpr bool EARLY = false;
     static constexpr int DEP_TILES = INT_MAX;
     static constexpr int NH_ = 1, NP_ = LL ? 2 + 2 * LL + 4 : 4, L1 = LL > 0 ? LL : 1;
     static constexpr bool CPML = true, MIRROR = false;
@@ -1643,6 +1667,7 @@ struct OpSSh {
 template <int FDOH, int TY, int NST, bool QUIRK>
 struct OpPAc {
     static constexpr int V = kCells;
+    static constexpr bool EARLY = false;
     static constexpr int DEP_TILES = INT_MAX;
     static constexpr int NH_ = 2, NP_ = 2;
     static constexpr bool CPML = !QUIRK, MIRROR = false;
@@ -1732,6 +1757,7 @@ struct OpPAc {
 template <int FDOH, int TY, int LL, int NST>
 struct OpPVisc {
     static constexpr int V = kCells;
+    static constexpr bool EARLY = false;
     static constexpr int DEP_TILES = INT_MAX;
     static constexpr bool Z0 = FDOH != 1, CPML = !Z0, MIRROR = false;
     static constexpr int NH_ = 2, NP_ = 3 + LL;

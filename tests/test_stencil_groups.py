@@ -116,3 +116,30 @@ def test_correlation_of_segment_snapshots(name, snap, nx):
         want = {0: (f[2] + f[3]) * (a[2] + a[3]), 2: a[5] * f[0] + a[6] * f[1]}
     for plane, w in want.items():
         assert bit_equal(grads[plane] + 0.0, w.astype(np.float32) + np.float32(0.0)), plane
+
+
+def test_shared_coefficients_match_single_shots():
+    """A batch large enough that the viscoelastic stress takes the model's
+    coefficients past its ring (two models, ragged rows): every slot equals
+    the same shot alone."""
+    nx, ny, n = 703, 431, 14  # 303 000 cells, 4.2 million in the batch
+    p, model, g, sig, adj = build_case("psv_visc_o8_holberg", nx=nx, ny=ny, nt=12, fw=20)
+    p.dtinv = 3
+    ntr = g.recpos.shape[1]
+    models = [model, {k: (v * np.float32(1.01) if k != "rho" else v) for k, v in model.items()}]
+    alone = []
+    for m in models:
+        with ShotSolver(p, max_rec=ntr) as s:
+            s.upload_model(m)
+            s.setup_shot(0, g.srcpos, sig, g.recpos)
+            alone.append((s.forward(1)[0], s.adjoint(adj[None])[0]))
+    with ShotSolver(p, max_shots=n, max_models=2, max_rec=ntr) as s:
+        s.set_options(tile_order=3)
+        for k, m in enumerate(models):
+            s.upload_model(m, k)
+        for k in range(n):
+            s.setup_shot(k, g.srcpos, sig, g.recpos, model=k % 2)
+        sec = s.forward(n)
+        grads = s.adjoint(np.stack([adj] * n), n)
+    for k in range(n):
+        assert bit_equal(sec[k], alone[k % 2][0]) and bit_equal(grads[k], alone[k % 2][1]), k
