@@ -355,12 +355,14 @@ __device__ __forceinline__ void run_pipeline(const KGrid &g, const KMaps &mp, in
         return;
     }
     ProfTab pt{op.M.profx, op.M.prof + 6 * (2 * g.fw + 1), g.psy, 2 * g.fw + 1, false};
-    if (Op::CPML && op.M.proftab) {
-        constexpr int n = 6 * (kProfX + kProfY) / 4;
-        for (int k = warp * 32 + lane; k < n; k += 32 * P::NCW)
-            reinterpret_cast<float4 *>(sprof)[k] = reinterpret_cast<const float4 *>(op.M.proftab)[k];
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * P::NCW) : "memory");
-        pt = ProfTab{sprof, sprof + 6 * kProfX, kProfX, kProfY, true};
+    if constexpr (Op::CPML) {
+        if (op.M.proftab) {
+            constexpr int n = 6 * (kProfX + kProfY) / 4;
+            for (int k = warp * 32 + lane; k < n; k += 32 * P::NCW)
+                reinterpret_cast<float4 *>(sprof)[k] = reinterpret_cast<const float4 *>(op.M.proftab)[k];
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * P::NCW) : "memory");
+            pt = ProfTab{sprof, sprof + 6 * kProfX, kProfX, kProfY, true};
+        }
     }
     int st = -1;
     uint32_t parity = 1;

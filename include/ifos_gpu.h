@@ -306,7 +306,8 @@ enum {
      * later call with the same shot count; 0: launched step by step. */
     IFOS_OPT_GRAPHS = 0,
     /* 1 (default): the loop's kernels are programmatic dependent launches
-     * (each starts its independent loads while its predecessor drains). */
+     * (each starts its independent loads while its predecessor drains), save
+     * the ones the launcher has been measured to run faster plainly. */
     IFOS_OPT_PDL = 1,
     /* persistent stencil CTAs per SM; 0 (default): as many as fit. */
     IFOS_OPT_BLOCKS_PER_SM = 2,
