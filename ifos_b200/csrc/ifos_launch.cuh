@@ -291,6 +291,14 @@ struct Launcher {
         }
         return so;
     }
+    // P-SV elastic launches of FDORDER 2 and 4 with at most a tile per SM: two
+    // cells a thread, twice the warps on the SM's only tile, and registers for
+    // both (400 x 160, one
+    // shot: 44.8 to 35.7 ms a gradient pass; 300 x 100: 8.2 to 7.2 ms a forward one)
+    bool small() const {
+        const long long tiles = (long long)((c->p.nx + kTileX - 1) / kTileX) * ((c->p.ny + kTileY - 1) / kTileY) * nshots;
+        return tiles <= c->num_sms;
+    }
     // the pipelined launches of half width FD: defined where ifos_pipe.cu is
     // compiled for that width, so that their kernels are compiled once
     // hin: snapshot index stored by this step's kernels (-1 none)
@@ -354,6 +362,13 @@ struct Launcher {
         }
         if (c->psv) {
             constexpr int NP = (SW == 1 && !Q) ? 6 : 4;
+            if constexpr (FD <= 2) {
+                if (small()) {
+                    pipelined(OpVPsv<FD, kTileY, ring_stages<FD, 3, NP, 0, kTileY, vblocks(FD)>(), Q, SW, P1, false, true>{
+                        g, S, M, t, snap_out(hin)});
+                    return;
+                }
+            }
             pipelined(OpVPsv<FD, kTileY, ring_stages<FD, 3, NP, 0, kTileY, vblocks(FD)>(), Q, SW, P1, false>{g, S, M, t, snap_out(hin)});
         }
     }
@@ -439,6 +454,12 @@ struct Launcher {
                     if constexpr (FD >= 5) {
                         if (quirk) {
                             pipelined(OpSEl<FD, kTileY, NST, true>{g, S, M, t, snap_out(hin)});
+                            done = true;
+                        }
+                    }
+                    if constexpr (FD <= 2) {
+                        if (small()) {
+                            pipelined(OpSEl<FD, kTileY, NST, false, true>{g, S, M, t, snap_out(hin)});
                             done = true;
                         }
                     }

@@ -1166,14 +1166,15 @@ struct OpSVisc {
 // stress, P-SV elastic (src/update_s_elastic_PML.c:151-241; 10/12: :442-535)
 // halo: vx vy; plain: sxx syy sxy uipjp f g (reference 10/12 branch: uipjp vs vp);
 // writes sxx syy sxy
-template <int FDOH, int TY, int NST, bool QUIRK>
+// SMALL: see Launcher::small
+template <int FDOH, int TY, int NST, bool QUIRK, bool SMALL = false>
 struct OpSEl {
-    static constexpr int V = kCells;
+    static constexpr int V = SMALL ? 2 : kCells;
     static constexpr bool EARLY = false;
     static constexpr int DEP_TILES = FDOH <= 2 ? kDepTiles : INT_MAX;
     static constexpr int NH_ = 2, NP_ = 6;
     static constexpr bool CPML = !QUIRK, MIRROR = false;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, sblocks(FDOH), V>;
+    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, SMALL ? 2 : sblocks(FDOH), V>;
     IFOS_OP_MEMBERS
     // boxes of consecutive planes: their number, planes of box k, whether they are model planes
     static constexpr int NG = QUIRK ? 4 : 2;
@@ -1292,15 +1293,15 @@ struct OpSEl {
 // plain: vx vy rip rjp [+ vxp1 vyp1 in the adjoint].  SW: 0 forward,
 // 1 adjoint; P1: this forward step forms vxp1/vyp1 for a snapshot (written to
 // the snapshot when the launch stores one, else to the state).
-template <int FDOH, int TY, int NST, bool QUIRK, int SW, bool P1, bool AC>
+template <int FDOH, int TY, int NST, bool QUIRK, int SW, bool P1, bool AC, bool SMALL = false>
 struct OpVPsv {
-    static constexpr int V = cells_v(FDOH);
+    static constexpr int V = SMALL ? 2 : cells_v(FDOH);
     static constexpr bool EARLY = false;
     static constexpr int DEP_TILES = FDOH <= 2 && !AC ? kDepTiles : INT_MAX;
     static constexpr int NH_ = AC ? 1 : 3;
     static constexpr int NP_ = (SW == 1 && !QUIRK) ? 6 : 4;
     static constexpr bool CPML = !QUIRK, MIRROR = true;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, vblocks(FDOH), V>;
+    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, SMALL ? 2 : vblocks(FDOH), V>;
     IFOS_OP_MEMBERS
     // boxes of consecutive planes: their number, planes of box k, whether they are model planes
     static constexpr int NG = NP_ / 2;

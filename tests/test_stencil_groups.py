@@ -143,3 +143,22 @@ def test_shared_coefficients_match_single_shots():
         grads = s.adjoint(np.stack([adj] * n), n)
     for k in range(n):
         assert bit_equal(sec[k], alone[k % 2][0]) and bit_equal(grads[k], alone[k % 2][1]), k
+
+
+@pytest.mark.parametrize("nx", [129, 130, 131, 132])
+@pytest.mark.parametrize("name", ["psv_el_o4", "psv_el_o2_nofs"])
+def test_batches_match_single_shots_of_a_tile_per_sm(name, nx):
+    """FDORDER 2 and 4 elastic launches of at most a tile per SM use two cells
+    a thread, larger ones four: a batch of 12 (180 tiles) equals the single
+    shot (15 tiles), which equals the oracle."""
+    p, model, g, sig, adj = build_case(name, nx=nx, ny=33, nt=40, fw=9)
+    ntr, n = g.recpos.shape[1], 12
+    ref = oracle_shot(p, model, g, sig, adj)
+    with ShotSolver(p, max_shots=n, max_rec=ntr) as s:
+        s.upload_model(model)
+        for k in range(n):
+            s.setup_shot(k, g.srcpos, sig, g.recpos)
+        sec = s.forward(n)
+        grads = s.adjoint(np.stack([adj] * n), n)
+    for k in range(n):
+        assert bit_equal(sec[k], ref["sections"]) and bit_equal(grads[k], ref["grads"]), k
