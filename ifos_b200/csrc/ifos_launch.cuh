@@ -88,6 +88,11 @@ struct LoopGraph {
     std::vector<TimedPair> pairs;
 };
 
+// tau of a model as it was last uploaded: the values of a uniform one
+struct ModelTau {
+    bool uploaded = false, uniform = false;
+    float taus = 0, taup = 0, tausipjp = 0;
+};
 enum { MAP_HALO = 0, MAP_PLAIN, MAP_MODEL };
 struct ifos_ctx {
     ifos_params p{};
@@ -110,7 +115,8 @@ struct ifos_ctx {
     long long mem_off[5];
     bool mplane[NM_PLANE];
     long long moff[NM_PLANE];
-    bool tau_planes = false;
+    bool tau_planes = false;                  // the kernels read the tau planes (else the scalars of g)
+    std::vector<ModelTau> model_tau;          // per model
     ViscoScalars vsc{};
     // snapshots
     bool with_snap = false;

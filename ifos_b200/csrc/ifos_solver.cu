@@ -578,6 +578,7 @@ extern "C" int ifos_ctx_create(const ifos_params *pp, int device, int with_snaps
     c->rec_row_hi.assign(S, 0);
     c->rec_mapped.assign(S, 1);
     c->slot_model_h.assign(S, 0);
+    c->model_tau.assign(p.max_models, ModelTau{});
     c->srcpos_h.assign((size_t)S * 8 * ms, 0.0f);
     setup_pipeline(c, L);
     if (const char *e = std::getenv("IFOS_PDL")) c->pdl = std::atoi(e) != 0;
@@ -653,17 +654,23 @@ extern "C" int ifos_model_upload(ifos_ctx *c, int model, const float *vp, const 
             return fail(c, IFOS_ERR_ARG, "model has non-finite values or non-positive density");
     if (cudaSetDevice(c->device) != cudaSuccess) return fail(c, IFOS_ERR_CUDA, "cudaSetDevice failed");
     if (c->p.L) {
-        // all models of a context share the tau representation of the first upload
-        if (!mp.tau_uniform) c->tau_planes = true;
-        c->g.taus0 = mp.taus0;
-        c->g.taup0 = mp.taup0;
-        c->g.tausipjp0 = mp.tausipjp0;
-        if (mp.tau_uniform) {
-            // planes stay in the table but are ignored (the kernels read the scalars)
+        // The kernels take tau from the scalars of KGrid while the context's
+        // models are all uniform with the same values, else from the tau
+        // planes, which every upload fills.
+        const bool uniform = mp.tau_uniform;
+        if (uniform) {
             mp.taus.assign(mp.rho.size(), mp.taus0);
             mp.taup.assign(mp.rho.size(), mp.taup0);
             mp.tausipjp.assign(mp.rho.size(), mp.tausipjp0);
         }
+        c->model_tau[model] = {true, uniform, mp.taus0, mp.taup0, mp.tausipjp0};
+        c->tau_planes = false;
+        for (const ModelTau &t : c->model_tau)
+            if (t.uploaded && !(t.uniform && t.taus == mp.taus0 && t.taup == mp.taup0 && t.tausipjp == mp.tausipjp0))
+                c->tau_planes = true;
+        c->g.taus0 = mp.taus0;
+        c->g.taup0 = mp.taup0;
+        c->g.tausipjp0 = mp.tausipjp0;
     }
     c->snaps_valid = false;
     return c->dbl ? model_upload_t<double>(c, model, mp) : model_upload_t<float>(c, model, mp);
@@ -837,7 +844,13 @@ static std::string loop_key(const ifos_ctx *c, std::initializer_list<long long> 
     for (long long x : v) k += std::to_string(x) + ",";
     k += std::to_string(c->prof_stride) + "," + std::to_string(c->pdl) + "," + std::to_string(c->blocks_per_sm) + "," +
          std::to_string(c->g.tile_order) + "," + std::to_string(c->g.prod_polls);
-    return k;
+    // the tau scalars and the choice of the tau planes are launch parameters too (ifos_model_upload sets them)
+    for (const float t : {c->g.taus0, c->g.taup0, c->g.tausipjp0}) {
+        unsigned bits;
+        std::memcpy(&bits, &t, 4);
+        k += "," + std::to_string(bits);
+    }
+    return k + "," + std::to_string(c->tau_planes);
 }
 
 template <typename T>
