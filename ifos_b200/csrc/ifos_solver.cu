@@ -1039,8 +1039,9 @@ static int adjoint_t(ifos_ctx *c, int nshots) {
     const bool rec_ok = Lr.receiver_rows() && rec_in_op(c, nshots);
     const bool v_inj = c->sh || (p.adjoint_type >= 1 && p.adjoint_type <= 3);  // the velocities take residuals
     const bool inj_fused = one && rec_ok && v_inj;
-    const bool p_inj = p.adjoint_type == 4, p_fused = one && rec_ok && p_inj && c->ac;
-    Lr.surf_fused = one && p.free_surf && (!p_inj || p_fused || c->sh);
+    // the pressure residual needs a pressure: SH alone takes its residuals in vz whatever ADJOINT_TYPE says
+    const bool p_inj = p.adjoint_type == 4 && c->psv, p_fused = one && rec_ok && p_inj && c->ac;
+    Lr.surf_fused = one && p.free_surf && (!p_inj || p_fused);
     Lr.fsurf = Lr.surf_fused ? 1 : 0;
     Lr.v_rec = inj_fused ? 2 : 0;
     Lr.s_rec = p_fused ? 2 : 0;

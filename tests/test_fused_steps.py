@@ -60,3 +60,21 @@ def test_several_sources(name, cells):
     for key in ("sections", "grads"):
         assert bit_equal(gpu[key], ref[key]), key
     assert bit_equal(gpu["fields"][m], ref["fields"][m]), "fields"
+
+
+@pytest.mark.parametrize("name", ["sh_el_o6", "sh_visc_o4"])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("layout", ["three_rows", "vertical_line"])
+def test_sh_has_no_pressure_residual(name, precision, layout):
+    """An SH run takes its residuals in vz under every ADJOINT_TYPE: the
+    pressure residual of type 4 has no plane to go to."""
+    p, model, g, sig, _ = build_case(name, nt=60)
+    rec = _receivers(p, layout)
+    g = W.Geometry(g.srcpos, rec)
+    adj = (np.random.default_rng(6).standard_normal((3, rec.shape[1], p.nt)) * 1e-3).astype(np.float32)
+    got = []
+    for p.adjoint_type in (1, 4):
+        got.append(gpu_shot(p, model, g, sig, adj, precision=precision))
+    for key in ("sections", "grads", "adj_fields"):
+        assert bit_equal(got[0][key], got[1][key]), key
+    assert np.abs(got[0]["grads"]).max() > 0
