@@ -342,8 +342,8 @@ struct Launcher {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, P::THREADS, P::bytes());
             occ[d] = o > 0 ? o : 1;
         }
-        const long long ntiles =
-            (long long)((c->p.nx + kTileX - 1) / kTileX) * ((c->p.ny + P::TILE_Y - 1) / P::TILE_Y) * nshots;
+        const TileWalk walk = TileWalk::of(op, nshots);
+        const long long ntiles = walk.ntiles;
         const int bps = c->blocks_per_sm > 0 ? std::min(c->blocks_per_sm, occ[d]) : occ[d];
         const int grid = (int)std::min<long long>(ntiles, (long long)bps * c->num_sms);
         KMaps mp;
@@ -354,7 +354,7 @@ struct Launcher {
         // issued): 2000 x 600 visco 14.3 to 13.0 ms a forward loop, 4000 x
         // 1200 P-SV 16.6 to 15.1.  Op::DEP_TILES says where it does not pay.
         const bool dep = c->pdl && ntiles <= (long long)Op::DEP_TILES * grid;
-        launch_dep(c->st, dep, kern, dim3(grid), dim3(32, P::NCW + 1), P::bytes(), mp, op, nshots,
+        launch_dep(c->st, dep, kern, dim3(grid), dim3(32, P::NCW + 1), P::bytes(), mp, walk, op,
                    (int *)c->bad.p);
     }
     template <int FD, bool Q, int SW, bool P1>

@@ -19,6 +19,7 @@
 // kernels of ifos_kernels.cuh.
 #pragma once
 #include <limits.h>
+#include <algorithm>
 #include <type_traits>
 
 #include "ifos_kernels.cuh"
@@ -154,80 +155,131 @@ __device__ __forceinline__ int div_small(int a, int b, float rb, int &rem) {
 // over the persistent CTAs hands each CTA the same number of them (within
 // one), so the CTAs finish together instead of the ones that drew the strip
 // columns finishing last.  A bijection on [0, ntx*nty).
+//
+// The launcher makes the struct (Launcher::pipelined) with everything the
+// producer warp needs before its first loads, in a few adjacent words of the
+// parameters.  Worked out on the device from the members of the op, the first
+// tile's indices took 2600-3200 cycles in front of every launch's first loads,
+// twice what the whole producer start had taken with one lane and no classes of
+// warps; so they take 1100-1300 (400 x 160, FDORDER 4, no dependent launches:
+// 9.8 to 7.5 us a forward step; with them acoustic 777 x 259 8.2 to 7.6, 1010 x
+// 336 viscoelastic, two shots, 23.7 to 22.6).
 struct TileWalk {
-    int ntx, nty, nshots, ntiles;
+    int ntx, per, nshots, ntiles;  // tile columns, tiles of a slot, slots, all tiles
     float r_ntx, r_shots, r_per;
-    // CPML-first regions: rows in a top y strip, first row of the bottom one,
-    // rows in y strips; left x-strip columns, first right one, x-strip columns
-    int rt, yb0, nys, cl, xr0, ce;
-    float r_ce, r_w;
-    __device__ __forceinline__ TileWalk(const KGrid &g, int TY, int shots) {
-        ntx = (g.nx + kTileX - 1) / kTileX, nty = (g.ny + TY - 1) / TY;
-        nshots = shots, ntiles = ntx * nty * shots;
-        r_ntx = 1.0f / ntx, r_shots = 1.0f / shots, r_per = 1.0f / (ntx * nty);
-        cl = min(ntx, (g.fw - 1) / kTileX + 1);  // tile columns with i0 <= FW
-        const int vx = g.nx - g.fw + 1 - kTileX;  // right strip: min(i0+63, NX) >= NX-FW+1
-        xr0 = max(cl, vx <= 0 ? 0 : (vx + kTileX - 1) / kTileX);
-        rt = g.free_surf ? 0 : min(nty, (g.fw - 1) / TY + 1);  // tile rows with j0 <= FW
-        const int vy = g.ny - g.fw + 1 - TY;                   // bottom strip: j0+TY-1 >= NY-FW+1
-        yb0 = min(nty, max(rt, vy <= 0 ? 0 : (vy + TY - 1) / TY));
-        nys = rt + (nty - yb0);
-        ce = cl + (ntx - xr0);
-        r_ce = 1.0f / ce, r_w = 1.0f / (ntx - ce);
+    // tile order (slot-minor, CPML first) and its CPML-first regions: rows in a
+    // top y strip, first row of the bottom one, tiles in y-strip rows; left
+    // x-strip columns, first right one, x-strip columns and their tiles in the
+    // other rows, columns between
+    int minor, cpml;
+    int rt, yb0, ny_tiles, cl, xr0, ce, nx_tiles, mid;
+    float r_ce, r_mid;
+    // Compute warps whose rows need more than the plain update: all of a tile
+    // outside the tile columns px0..px1-1 (an x strip, cells outside the grid)
+    // or of the top tiles if `top` (rows imaged at the free surface, velocity);
+    // else those with a row of the ranges lo..hi: top y strip or the surface
+    // itself, bottom y strip and rows outside the grid, the probe's row,
+    // receiver rows, source rows
+    enum { R_TOP, R_BOTTOM, R_PROBE, R_REC, R_SRC, NR };
+    int px0, px1, top;
+    int lo[NR], hi[NR];
+    // TMA z coordinates: planes of a slot and of a model, the halo box's first plane, the groups'
+    int slot_planes, model_planes, zh, zg[kMaxGroups];
+
+    template <typename Op>
+    static TileWalk of(const Op &op, int shots) {
+        using std::max;
+        using std::min;
+        const KGrid &g = op.g;
+        constexpr int TY = Op::P::TILE_Y;
+        TileWalk w{};
+        const int nty = (g.ny + TY - 1) / TY;
+        w.ntx = (g.nx + kTileX - 1) / kTileX;
+        w.per = w.ntx * nty;
+        w.nshots = shots;
+        w.ntiles = w.per * shots;
+        w.r_ntx = 1.0f / w.ntx, w.r_shots = 1.0f / shots, w.r_per = 1.0f / w.per;
+        w.minor = g.tile_order & 1;
+        w.cpml = (g.tile_order & 2) && g.fw > 0;
+        w.cl = min(w.ntx, (g.fw - 1) / kTileX + 1);  // tile columns with i0 <= FW
+        const int vx = g.nx - g.fw + 1 - kTileX;     // right strip: min(i0+63, NX) >= NX-FW+1
+        w.xr0 = max(w.cl, vx <= 0 ? 0 : (vx + kTileX - 1) / kTileX);
+        w.rt = g.free_surf ? 0 : min(nty, (g.fw - 1) / TY + 1);  // tile rows with j0 <= FW
+        const int vy = g.ny - g.fw + 1 - TY;                     // bottom strip: j0+TY-1 >= NY-FW+1
+        w.yb0 = min(nty, max(w.rt, vy <= 0 ? 0 : (vy + TY - 1) / TY));
+        w.ny_tiles = (w.rt + nty - w.yb0) * w.ntx;
+        w.ce = w.cl + (w.ntx - w.xr0);
+        w.nx_tiles = (w.yb0 - w.rt) * w.ce;
+        w.mid = w.ntx - w.ce;
+        w.r_ce = 1.0f / w.ce, w.r_mid = w.mid > 0 ? 1.0f / w.mid : 0.0f;
+
+        const bool ystrips = Op::CPML && g.fw > 0, xstrips = ystrips && !g.boundary;
+        w.px0 = xstrips ? (g.fw - 1) / kTileX + 1 : 0;
+        w.px1 = (g.nx - (xstrips ? g.fw : 0)) / kTileX;
+        w.top = Op::MIRROR && g.free_surf;
+        auto range = [&](int k, bool on, int a, int b) { w.lo[k] = on ? a : 1, w.hi[k] = on ? b : 0; };
+        range(R_TOP, g.free_surf ? op.fsurf != 0 : ystrips, 1, g.free_surf ? 1 : g.fw);
+        range(R_BOTTOM, true, ystrips ? g.ny - g.fw + 1 : g.ny + 1, INT_MAX);
+        range(R_PROBE, op.probe, g.ny / 2, g.ny / 2);
+        range(R_REC, op.rec_mode, op.rec_j0, op.rec_j1);
+        range(R_SRC, op.fps || op.fvs, op.src_j0, op.src_j1);
+
+        int z[Op::NG];
+        op.planes(w.zh, z);
+        for (int k = 0; k < Op::NG; k++) w.zg[k] = z[k];
+        w.slot_planes = op.tm.planes_per_slot;
+        w.model_planes = op.tm.model_planes;
+        return w;
     }
     // tile row and column of a spatial rank in CPML-first order
     __device__ __forceinline__ int first(int rank, int &tx) const {
-        if (rank < nys * ntx) {
+        if (rank < ny_tiles) {
             const int r = div_small(rank, ntx, r_ntx, tx);
             return r < rt ? r : yb0 + (r - rt);
         }
-        rank -= nys * ntx;
-        const int mid = nty - nys;  // rows between the y strips: rt .. yb0-1
+        rank -= ny_tiles;
         int c;
-        if (rank < mid * ce) {
+        if (rank < nx_tiles) {  // rows between the y strips: rt .. yb0-1
             const int r = div_small(rank, ce, r_ce, c);
             tx = c < cl ? c : xr0 + (c - cl);
             return rt + r;
         }
-        rank -= mid * ce;
-        const int r = div_small(rank, ntx - ce, r_w, c);  // ce < ntx here: the regions above hold every tile when it is not
+        rank -= nx_tiles;
+        const int r = div_small(rank, mid, r_mid, c);  // mid > 0 here: the regions above hold every tile when it is not
         tx = cl + c;
         return rt + r;
     }
-    __device__ __forceinline__ void tile(int t, int TY, int order, int fw, TileInfo &r) const {
+    // Tile t of the launch: slot, first cell, and the bits of the compute warps
+    // of ROWS rows each that need more than the plain update
+    template <int TY, int ROWS>
+    __device__ __forceinline__ TileInfo tile(int t) const {
+        TileInfo r;
         int rem, tx;
         if (nshots == 1) r.slot = 0, rem = t;
-        else if (order & 1) rem = div_small(t, nshots, r_shots, r.slot);
-        else r.slot = div_small(t, ntx * nty, r_per, rem);
-        const int ty = (order & 2) && fw > 0 ? first(rem, tx) : div_small(rem, ntx, r_ntx, tx);
+        else if (minor) rem = div_small(t, nshots, r_shots, r.slot);
+        else r.slot = div_small(t, per, r_per, rem);
+        const int ty = cpml ? first(rem, tx) : div_small(rem, ntx, r_ntx, tx);
         r.i0 = tx * kTileX + 1;
         r.j0 = ty * TY + 1;
+        unsigned rows = tx < px0 || tx >= px1 || (top && ty == 0) ? (1u << TY) - 1 : 0u;
+#pragma unroll
+        for (int k = 0; k < NR; k++) {
+            const int a = max(lo[k] - r.j0, 0), b = min(hi[k] - r.j0, TY - 1);
+            if (a <= b) rows |= (2u << b) - (1u << a);
+        }
+        r.bits = warps_of_rows<ROWS>(rows);
+        return r;
+    }
+    // bit w: one of the rows of compute warp w
+    template <int ROWS>
+    static __device__ __forceinline__ int warps_of_rows(unsigned rows) {
+        static_assert(ROWS == 1 || ROWS == 2, "rows of a compute warp");
+        if (ROWS == 1) return (int)rows;
+        unsigned m = (rows | rows >> 1) & 0x55u;
+        m = (m | m >> 1) & 0x33u;
+        return (int)((m | m >> 2) & 0x0fu);
     }
 };
-
-// Compute warps of a tile whose rows need more than the plain update of whole
-// rows: a CPML strip, the imaged rows of the free surface (velocity), the
-// surface itself, a source, receiver or probe row, or cells outside the grid.
-template <typename Op>
-__device__ __forceinline__ int edge_warps(const Op &op, const TileInfo &ti) {
-    const KGrid &g = op.g;
-    using P = typename Op::P;
-    constexpr int all = (1 << P::NCW) - 1;
-    const bool strips = Op::CPML && g.fw > 0;
-    if (ti.i0 + kTileX - 1 > g.nx || (Op::MIRROR && g.free_surf && ti.j0 == 1)) return all;
-    if (strips && !g.boundary && (ti.i0 <= g.fw || ti.i0 + kTileX - 1 >= g.nx - g.fw + 1)) return all;
-    int m = 0;
-#pragma unroll
-    for (int w = 0; w < P::NCW; w++) {
-        const int a = ti.j0 + P::ROWS * w, b = a + P::ROWS - 1;
-        bool e = b > g.ny || (strips && ((!g.free_surf && a <= g.fw) || b >= g.ny - g.fw + 1));
-        e = e || (op.rec_mode && a <= op.rec_j1 && b >= op.rec_j0);
-        e = e || (op.probe && (a == g.ny / 2 || b == g.ny / 2));
-        e = e || ((op.fps || op.fvs) && a <= op.src_j1 && b >= op.src_j0) || (op.fsurf && a == 1);
-        m |= e ? 1 << w : 0;
-    }
-    return m;
-}
 
 // The profiles a block reads: in shared memory (staged once per block) when
 // the strips are no wider than kProfX columns and kProfY rows, else the global
@@ -263,7 +315,7 @@ constexpr int kTileBatch = 32;
 // wait for every tile it issued (so that no copy into the ring is in flight
 // when the block exits), compute none of them, and leave at k_stop.
 template <typename P, typename Op>
-__device__ __forceinline__ void run_pipeline(const KGrid &g, const KMaps &mp, int nshots, const Op &op, int *err) {
+__device__ __forceinline__ void run_pipeline(const KGrid &g, const KMaps &mp, const TileWalk &walk, const Op &op, int *err) {
     constexpr int NST = P::STAGES, TY = P::TILE_Y;
     extern __shared__ __align__(1024) unsigned char sm_raw[];
     __shared__ __align__(8) uint64_t full[NST], empty[NST], filled;
@@ -271,7 +323,7 @@ __device__ __forceinline__ void run_pipeline(const KGrid &g, const KMaps &mp, in
     __shared__ __align__(16) float sprof[Op::CPML ? 6 * (kProfX + kProfY) : 4];
     __shared__ int stop_at;  // -1 while the producer runs, else the first tile it did not issue
     float *smem = reinterpret_cast<float *>(sm_raw);
-    const int ntiles = ((g.nx + kTileX - 1) / kTileX) * ((g.ny + TY - 1) / TY) * nshots;
+    const int ntiles = walk.ntiles;
     const int warp = threadIdx.y, lane = threadIdx.x;
     if (warp == P::NCW && lane == 0) {
         for (int s = 0; s < NST; s++) {
@@ -287,13 +339,11 @@ __device__ __forceinline__ void run_pipeline(const KGrid &g, const KMaps &mp, in
     if (warp == P::NCW) {
         // tiles k0 .. k0+31 of this block; the entries they replace belong to
         // tiles the compute warps have left (they are at most NST behind)
-        const TileWalk walk(g, TY, nshots);
         auto fill = [&](int k0) {
             const int k = k0 + lane, t = blockIdx.x + k * gridDim.x;
             if (t < ntiles) {
-                TileInfo ti;
-                walk.tile(t, TY, g.tile_order, g.fw, ti);
-                ti.bits = (op.M.one_model ? 0 : op.M.slot_model[ti.slot] * 256) + edge_warps(op, ti);
+                TileInfo ti = walk.tile<TY, P::ROWS>(t);
+                if (!op.M.one_model) ti.bits += op.M.slot_model[ti.slot] * 256;
                 tq[k % (2 * kTileBatch)] = ti;
             }
             __syncwarp();
@@ -303,17 +353,16 @@ __device__ __forceinline__ void run_pipeline(const KGrid &g, const KMaps &mp, in
             const TileInfo ti = tq[k % (2 * kTileBatch)];
             float *stage = smem + st * P::STAGE;
             uint64_t *bar = &full[st];
-            int hz, gz[Op::NG];
-            op.planes(ti, hz, gz);
+            const int zs = ti.slot * walk.slot_planes, zm = ti.model() * walk.model_planes;
             if (plain) mbar_expect_tx(bar, P::TXB);
             if (halo)
-                tma_load_3d(stage, &mp.halo, HX + ti.i0 - 1 - P::XH, HY + ti.j0 - 1 - P::H, hz, bar);
+                tma_load_3d(stage, &mp.halo, HX + ti.i0 - 1 - P::XH, HY + ti.j0 - 1 - P::H, zs + walk.zh, bar);
             if (plain) {
                 const int px = HX + ti.i0 - 1, py = HY + ti.j0 - 1;
                 int q = 0;
 #pragma unroll
                 for (int k = 0; k < Op::NG; k++) {
-                    tma_load_3d(stage + P::HALO + q * P::PLS, &mp.grp[k], px, py, gz[k], bar);
+                    tma_load_3d(stage + P::HALO + q * P::PLS, &mp.grp[k], px, py, (Op::gm(k) ? zm : zs) + walk.zg[k], bar);
                     q += Op::gd(k);
                 }
             }
@@ -997,12 +1046,11 @@ struct OpSVisc {
     static constexpr int NG = SHARED ? 2 : 3;
     __host__ __device__ static constexpr int gd(int k) { return k == 0 ? 3 : (k == 1 ? 3 * LL : 6); }
     __host__ __device__ static constexpr bool gm(int k) { return k == 2; }
-    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
-        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
-        hz = zb + tm.pid[P_VX];
-        gz[0] = zb + tm.pid[P_SXX];
-        gz[1] = zb + tm.mem_pid[0];
-        if (!SHARED) gz[2 % NG] = mb + tm.mid[M_FIPJPV];
+    void planes(int &hz, int (&gz)[NG]) const {  // first planes of the boxes, in slot 0 and model 0
+        hz = tm.pid[P_VX];
+        gz[0] = tm.pid[P_SXX];
+        gz[1] = tm.mem_pid[0];
+        if (!SHARED) gz[2 % NG] = tm.mid[M_FIPJPV];
     }
     // SHARED: fipjp f g mu pi muipjp of the thread's cells, loaded before the wait
     struct Pre {
@@ -1180,12 +1228,11 @@ struct OpSEl {
     static constexpr int NG = QUIRK ? 4 : 2;
     __host__ __device__ static constexpr int gd(int k) { return k == 0 || !QUIRK ? 3 : 1; }
     __host__ __device__ static constexpr bool gm(int k) { return k > 0; }
-    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
-        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
-        hz = zb + tm.pid[P_VX];
-        gz[0] = zb + tm.pid[P_SXX];
-        gz[1] = mb + tm.mid[M_UIPJP];
-        if (QUIRK) gz[2 % NG] = mb + tm.mid[M_VS], gz[3 % NG] = mb + tm.mid[M_VP];
+    void planes(int &hz, int (&gz)[NG]) const {  // first planes of the boxes, in slot 0 and model 0
+        hz = tm.pid[P_VX];
+        gz[0] = tm.pid[P_SXX];
+        gz[1] = tm.mid[M_UIPJP];
+        if (QUIRK) gz[2 % NG] = tm.mid[M_VS], gz[3 % NG] = tm.mid[M_VP];
     }
     struct Pre {
         Psi<V> x0, x1, y0, y1;
@@ -1307,12 +1354,11 @@ struct OpVPsv {
     static constexpr int NG = NP_ / 2;
     __host__ __device__ static constexpr int gd(int k) { return 2 + 0 * k; }
     __host__ __device__ static constexpr bool gm(int k) { return k == 1; }
-    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
-        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
-        hz = zb + tm.pid[AC ? P_SP : P_SXX];
-        gz[0] = zb + tm.pid[P_VX];
-        gz[1] = mb + tm.mid[M_RIP];
-        if (NG > 2) gz[2 % NG] = zb + tm.pid[P_VXP1];
+    void planes(int &hz, int (&gz)[NG]) const {  // first planes of the boxes, in slot 0 and model 0
+        hz = tm.pid[AC ? P_SP : P_SXX];
+        gz[0] = tm.pid[P_VX];
+        gz[1] = tm.mid[M_RIP];
+        if (NG > 2) gz[2 % NG] = tm.pid[P_VXP1];
     }
     struct Pre {
         Psi<V> x0, x1, y0, y1;
@@ -1467,11 +1513,10 @@ struct OpVSh {
     static constexpr int NG = 2;
     __host__ __device__ static constexpr int gd(int k) { return 1 + 0 * k; }
     __host__ __device__ static constexpr bool gm(int k) { return k == 1; }
-    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
-        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
-        hz = zb + tm.pid[P_SXZ];
-        gz[0] = zb + tm.pid[P_VZ];
-        gz[1] = mb + tm.mid[M_RJP];
+    void planes(int &hz, int (&gz)[NG]) const {  // first planes of the boxes, in slot 0 and model 0
+        hz = tm.pid[P_SXZ];
+        gz[0] = tm.pid[P_VZ];
+        gz[1] = tm.mid[M_RJP];
     }
     struct Pre {
         Psi<V> x0, y0;
@@ -1553,12 +1598,11 @@ struct OpSSh {
     static constexpr int NG = LL ? 5 : 2;
     __host__ __device__ static constexpr int gd(int k) { return k == 0 ? 2 : (!LL ? 2 : (k == 1 ? 2 * LL : (k == 2 ? 2 : 1))); }
     __host__ __device__ static constexpr bool gm(int k) { return k >= (LL ? 2 : 1); }
-    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
-        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
-        hz = zb + tm.pid[P_VZ];
-        gz[0] = zb + tm.pid[P_SXZ];
-        gz[1] = LL ? zb + tm.mem_pid[3] : mb + tm.mid[M_UIPJP];
-        if (LL) gz[2 % NG] = mb + tm.mid[M_FIPJPV], gz[3 % NG] = mb + tm.mid[M_MUR], gz[4 % NG] = mb + tm.mid[M_MUIPJPR];
+    void planes(int &hz, int (&gz)[NG]) const {  // first planes of the boxes, in slot 0 and model 0
+        hz = tm.pid[P_VZ];
+        gz[0] = tm.pid[P_SXZ];
+        gz[1] = LL ? tm.mem_pid[3] : tm.mid[M_UIPJP];
+        if (LL) gz[2 % NG] = tm.mid[M_FIPJPV], gz[3 % NG] = tm.mid[M_MUR], gz[4 % NG] = tm.mid[M_MUIPJPR];
     }
     struct Pre {
         Psi<V> x0, y0;
@@ -1680,11 +1724,10 @@ struct OpPAc {
     static constexpr int NG = 2;
     __host__ __device__ static constexpr int gd(int k) { return 1 + 0 * k; }
     __host__ __device__ static constexpr bool gm(int k) { return k == 1; }
-    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
-        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
-        hz = zb + tm.pid[P_VX];
-        gz[0] = zb + tm.pid[P_SP];
-        gz[1] = mb + tm.mid[QUIRK ? M_VP : M_GAC];
+    void planes(int &hz, int (&gz)[NG]) const {  // first planes of the boxes, in slot 0 and model 0
+        hz = tm.pid[P_VX];
+        gz[0] = tm.pid[P_SP];
+        gz[1] = tm.mid[QUIRK ? M_VP : M_GAC];
     }
     struct Pre {
         Psi<V> x0, y0;
@@ -1770,12 +1813,11 @@ struct OpPVisc {
     static constexpr int NG = 3;
     __host__ __device__ static constexpr int gd(int k) { return k == 0 ? 1 : (k == 1 ? LL : 2); }
     __host__ __device__ static constexpr bool gm(int k) { return k == 2; }
-    __device__ __forceinline__ void planes(const TileInfo &ti, int &hz, int (&gz)[NG]) const {
-        const int zb = ti.slot * tm.planes_per_slot, mb = ti.model() * tm.model_planes;
-        hz = zb + tm.pid[P_VX];
-        gz[0] = zb + tm.pid[P_SP];
-        gz[1] = zb + tm.mem_pid[1];
-        gz[2] = mb + tm.mid[M_GV];
+    void planes(int &hz, int (&gz)[NG]) const {  // first planes of the boxes, in slot 0 and model 0
+        hz = tm.pid[P_VX];
+        gz[0] = tm.pid[P_SP];
+        gz[1] = tm.mem_pid[1];
+        gz[2] = tm.mid[M_GV];
     }
     struct Pre {
         Psi<V> x0, y0;
@@ -1876,8 +1918,9 @@ constexpr int ring_blocks() {
 // the kernel: one Op per launch, persistent over all tiles of all slots
 template <typename Op>
 __global__ void __launch_bounds__(Op::P::THREADS, ring_blocks<typename Op::P>())
-    kp_stencil(const __grid_constant__ KMaps maps, const __grid_constant__ Op op, int nshots, int *err) {
-    run_pipeline<typename Op::P>(op.g, maps, nshots, op, err);
+    kp_stencil(const __grid_constant__ KMaps maps, const __grid_constant__ TileWalk walk, const __grid_constant__ Op op,
+               int *err) {
+    run_pipeline<typename Op::P>(op.g, maps, walk, op, err);
 }
 
 }  // namespace ifos
