@@ -297,13 +297,24 @@ struct Launcher {
         }
         return so;
     }
-    // P-SV elastic launches of FDORDER 2 and 4 with at most a tile per SM: two
-    // cells a thread, twice the warps on the SM's only tile, and registers for
-    // both (400 x 160, one
-    // shot: 44.8 to 35.7 ms a gradient pass; 300 x 100: 8.2 to 7.2 ms a forward one)
-    bool small() const {
+    // Whether a launch of the P-SV elastic stress, or of the P-SV velocity of
+    // FDORDER 2 and 4, takes two cells a thread with twice the warps and two
+    // blocks' registers, instead of four cells: launches of a few tiles per SM
+    // are bound by the latency of a tile, whose straight-line code and register
+    // use four cells double.  Up to four tiles per SM for FDORDER 2 and 4 and
+    // for the reference's 10/12 form, up to one for the others.  A forward and
+    // an adjoint step of 400 x 160, FW 20, with four cells and with two (us):
+    //   FDORDER 4, 2, 3, 4, 6 and 8 shots (1.9, 2.8, 3.8, 5.7 and 7.6 tiles per SM):
+    //     11.4 + 14.1 and 8.8 + 10.8, 11.5 + 15.4 and 11.0 + 12.4, 11.8 + 16.0 and
+    //     10.5 + 12.8, 14.2 + 17.9 and 15.0 + 18.3, 15.0 + 20.7 and 17.0 + 19.8;
+    //   the same with K above 1, 4 shots: 18.1 + 19.4 and 13.3 + 14.4;
+    //   FDORDER 8 (stress only), 1 and 3 shots: 9.0 + 10.3 and 8.2 + 9.9, 10.9 +
+    //     13.4 and 11.0 + 12.9;
+    //   FDORDER 10 form (stress only), 1 and 3: 6.9 + 9.0 and 6.4 + 8.5, 8.4 + 11.6
+    //     and 8.2 + 10.8.
+    bool small(int tiles_per_sm) const {
         const long long tiles = (long long)((c->p.nx + kTileX - 1) / kTileX) * ((c->p.ny + kTileY - 1) / kTileY) * nshots;
-        return tiles <= c->num_sms;
+        return tiles <= (long long)tiles_per_sm * c->num_sms;
     }
     // the pipelined launches of half width FD: defined where ifos_pipe.cu is
     // compiled for that width, so that their kernels are compiled once
@@ -369,7 +380,7 @@ struct Launcher {
         if (c->psv) {
             constexpr int NP = (SW == 1 && !Q) ? 6 : 4;
             if constexpr (FD <= 2) {
-                if (small()) {
+                if (small(4)) {
                     pipelined(OpVPsv<FD, kTileY, ring_stages<FD, 3, NP, 0, kTileY, vblocks(FD)>(), Q, SW, P1, false, true>{
                         g, S, M, t, snap_out(hin)});
                     return;
@@ -459,15 +470,14 @@ struct Launcher {
                     bool done = false;
                     if constexpr (FD >= 5) {
                         if (quirk) {
-                            pipelined(OpSEl<FD, kTileY, NST, true>{g, S, M, t, snap_out(hin)});
+                            if (small(4)) pipelined(OpSEl<FD, kTileY, NST, true, true>{g, S, M, t, snap_out(hin)});
+                            else pipelined(OpSEl<FD, kTileY, NST, true>{g, S, M, t, snap_out(hin)});
                             done = true;
                         }
                     }
-                    if constexpr (FD <= 2) {
-                        if (small()) {
-                            pipelined(OpSEl<FD, kTileY, NST, false, true>{g, S, M, t, snap_out(hin)});
-                            done = true;
-                        }
+                    if (!done && small(FD <= 2 ? 4 : 1)) {
+                        pipelined(OpSEl<FD, kTileY, NST, false, true>{g, S, M, t, snap_out(hin)});
+                        done = true;
                     }
                     if (!done) pipelined(OpSEl<FD, kTileY, NST, false>{g, S, M, t, snap_out(hin)});
                 }

@@ -162,3 +162,24 @@ def test_batches_match_single_shots_of_a_tile_per_sm(name, nx):
         grads = s.adjoint(np.stack([adj] * n), n)
     for k in range(n):
         assert bit_equal(sec[k], ref["sections"]) and bit_equal(grads[k], ref["grads"]), k
+
+
+@pytest.mark.parametrize("nx", [130, 131])
+@pytest.mark.parametrize("name,n", [("psv_el_o4", 42), ("psv_el_o2_nofs", 42), ("psv_el_o8_holberg", 12),
+                                    ("psv_el_o12_ref", 12), ("psv_el_o12_ref", 42)])
+def test_batches_of_few_and_more_tiles_per_sm(name, n, nx):
+    """The P-SV launches change from two to four cells a thread above one or
+    four tiles per SM (by FDORDER): batches on both sides (12 and 42 shots, 180
+    and 630 tiles) and the single shot (15 tiles) equal the oracle."""
+    p, model, g, sig, adj = build_case(name, nx=nx, ny=33, nt=40, fw=9)
+    ntr = g.recpos.shape[1]
+    ref = oracle_shot(p, model, g, sig, adj)
+    for shots in (1, n):
+        with ShotSolver(p, max_shots=shots, max_rec=ntr) as s:
+            s.upload_model(model)
+            for k in range(shots):
+                s.setup_shot(k, g.srcpos, sig, g.recpos)
+            sec = s.forward(shots)
+            grads = s.adjoint(np.stack([adj] * shots), shots)
+        for k in range(shots):
+            assert bit_equal(sec[k], ref["sections"]) and bit_equal(grads[k], ref["grads"]), k
