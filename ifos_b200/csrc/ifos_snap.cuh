@@ -435,18 +435,18 @@ __global__ void __launch_bounds__(128) k_correlate_cells(KGrid g, KState<float> 
     };
     if constexpr (ACC64) {
         double *acd = gr.acc64 + (long long)slot * 5 * n + q;
+        static_assert(V == 2, "double sums: two cells a thread (NX even), 16-byte accesses");
+        double2 w[5] = {};
 #pragma unroll
-        for (int e = 0; e < V; e++) {
-            double w[5] = {};
+        for (int k = 0; k < 5; k++)
+            if (use[k]) w[k] = *reinterpret_cast<const double2 *>(acd + k * n);
+        correlate_cell<PSV, SH, AC, double>(cell(0), mm.v[0], ll.v[0], rho.v[0], u.v[0], w[0].x, w[1].x, w[2].x, w[3].x,
+                                            w[4].x, g.mu_fix != 0);
+        correlate_cell<PSV, SH, AC, double>(cell(1), mm.v[1], ll.v[1], rho.v[1], u.v[1], w[0].y, w[1].y, w[2].y, w[3].y,
+                                            w[4].y, g.mu_fix != 0);
 #pragma unroll
-            for (int k = 0; k < 5; k++)
-                if (use[k]) w[k] = acd[k * n + e];
-            correlate_cell<PSV, SH, AC, double>(cell(e), mm.v[e], ll.v[e], rho.v[e], u.v[e], w[0], w[1], w[2], w[3],
-                                                w[4], g.mu_fix != 0);
-#pragma unroll
-            for (int k = 0; k < 5; k++)
-                if (use[k]) acd[k * n + e] = w[k];
-        }
+        for (int k = 0; k < 5; k++)
+            if (use[k]) *reinterpret_cast<double2 *>(acd + k * n) = w[k];
     } else {
         float *acc = gr.acc + (long long)slot * 5 * n + q;
         Vec<V> w[5] = {};
