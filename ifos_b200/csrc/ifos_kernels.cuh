@@ -36,6 +36,8 @@ enum : int {
     M_MUIPJPR, M_TAUS, M_TAUP, M_TAUSIPJP, M_MM, M_LL, NM_PLANE
 };
 // CPML strip ids: x strips (NY x 2FW), y strips (2FW x NX)
+// groups of memory variables (L planes each): r, p, q of P-SV (p alone acoustic), t, o of SH
+enum : int { MEM_R = 0, MEM_P, MEM_Q, MEM_T, MEM_O, N_MEM };
 enum : int { X_SXX = 0, X_SXY, X_VXX, X_VYX, X_VXXS, X_SXZ, X_VZX, NX_STRIP };
 enum : int { Y_SYY = 0, Y_SXY, Y_VYY, Y_VXY, Y_SYZ, Y_VZY, NY_STRIP };
 // profile ids (arrays of 2FW+1, 1-based)
@@ -70,7 +72,7 @@ struct KState {
     T *base;                  // slot 0
     long long slot_stride;    // elements between slots
     long long off[NP_FIELD];  // plane offsets within a slot (-1 absent)
-    long long mem_off[5];     // first plane of r,p,q,t,o (L planes each), -1 absent
+    long long mem_off[N_MEM]; // first plane of a group of memory variables (L planes each)
     T *psix[NX_STRIP];        // slot 0 strip, NY rows of KGrid::psx
     T *psiy[NY_STRIP];        // slot 0 strip, 2FW rows of KGrid::psy
     long long psix_slot, psiy_slot;  // elements between slots of one strip
@@ -405,9 +407,9 @@ __global__ void k_s_psv_visc(KGrid g, KState<T> S, KModel<T> M) {
     const int L = g.L;
     T sumr = 0, sump = 0, sumq = 0;
     for (int l = 1; l <= L; l++) {
-        sumr += memp(S, g, slot, 0, l)[c];
-        sump += memp(S, g, slot, 1, l)[c];
-        sumq += memp(S, g, slot, 2, l)[c];
+        sumr += memp(S, g, slot, MEM_R, l)[c];
+        sump += memp(S, g, slot, MEM_P, l)[c];
+        sumq += memp(S, g, slot, MEM_Q, l)[c];
     }
     const T fipjp = modelp(M, slot, M_FIPJPV)[c], f = modelp(M, slot, M_FV)[c], gg = modelp(M, slot, M_GV)[c];
     sxy[c] += (fipjp * (vxy + vyx)) + (dthalbe * sumr);
@@ -421,7 +423,7 @@ __global__ void k_s_psv_visc(KGrid g, KState<T> S, KModel<T> M) {
         const T eta = g.eta[l];
         // dip, d, e of src/prepare_update_s.c:57-59, formed in the same order
         const T dip = muij * eta * tsij, d = mu * eta * ts, e = pi * eta * tp;
-        T *rr = memp(S, g, slot, 0, l) + c, *pp = memp(S, g, slot, 1, l) + c, *qq = memp(S, g, slot, 2, l) + c;
+        T *rr = memp(S, g, slot, MEM_R, l) + c, *pp = memp(S, g, slot, MEM_P, l) + c, *qq = memp(S, g, slot, MEM_Q, l) + c;
         T r = (T)g.bip[l] * (*rr * (T)g.cip[l] - (dip * (vxy + vyx)));
         T p = (T)((double)g.bjm[l] * ((double)(*pp * (T)g.cjm[l] - (e * (vxx + vyy))) + (2.0 * (double)d * (double)vyy)));
         T q = (T)((double)g.bjm[l] * ((double)(*qq * (T)g.cjm[l] - (e * (vxx + vyy))) + (2.0 * (double)d * (double)vxx)));
@@ -468,8 +470,8 @@ __global__ void k_s_sh(KGrid g, KState<T> S, KModel<T> M) {
     }
     T sumo = 0, sumt = 0;
     for (int l = 1; l <= L; l++) {
-        sumo += memp(S, g, slot, 4, l)[c];
-        sumt += memp(S, g, slot, 3, l)[c];
+        sumo += memp(S, g, slot, MEM_O, l)[c];
+        sumt += memp(S, g, slot, MEM_T, l)[c];
     }
     sxz[c] += (modelp(M, slot, M_FIPJPV)[c] * vzx) + (dthalbe * sumo);
     syz[c] += (modelp(M, slot, M_FV)[c] * vzy) + (dthalbe * sumt);
@@ -480,7 +482,7 @@ __global__ void k_s_sh(KGrid g, KState<T> S, KModel<T> M) {
     for (int l = 1; l <= L; l++) {
         const T eta = g.eta[l];
         const T dip = muij * eta * tsij, d = mu * eta * ts;
-        T *oo = memp(S, g, slot, 4, l) + c, *tt = memp(S, g, slot, 3, l) + c;
+        T *oo = memp(S, g, slot, MEM_O, l) + c, *tt = memp(S, g, slot, MEM_T, l) + c;
         T o = (T)g.bip[l] * (*oo * (T)g.cip[l] - (dip * vzx));
         T t = (T)g.bjm[l] * (*tt * (T)g.cjm[l] - (d * vzy));
         *oo = o;
@@ -551,7 +553,7 @@ __global__ void k_p_visc(KGrid g, KState<T> S, KModel<T> M) {
     }
     const int L = g.L;
     T sump = 0;
-    for (int l = 1; l <= L; l++) sump += memp(S, g, slot, 1, l)[c];
+    for (int l = 1; l <= L; l++) sump += memp(S, g, slot, MEM_P, l)[c];
     const T gg = modelp(M, slot, M_GV)[c], pi = modelp(M, slot, M_PIR)[c];
     const T *tpp = modelp(M, slot, M_TAUP);
     const T tp = tpp ? tpp[c] : (T)g.taup0;
@@ -559,7 +561,7 @@ __global__ void k_p_visc(KGrid g, KState<T> S, KModel<T> M) {
     sump = 0;
     for (int l = 1; l <= L; l++) {
         const T e = pi * (T)g.eta[l] * tp;  // e of src/prepare_update_p.c:62, formed in the same order
-        T *pp = memp(S, g, slot, 1, l) + c;
+        T *pp = memp(S, g, slot, MEM_P, l) + c;
         const T p = (T)g.bjm[l] * (*pp * (T)g.cjm[l] - (e * (vxx + vyy)));
         *pp = p;
         sump += p;
@@ -799,7 +801,7 @@ __device__ void surface_cell(const KGrid &g, const KState<T> &S, const KModel<T>
     syy[c] = 0;
     const int L = g.L;
     if (L)
-        for (int l = 1; l <= L; l++) memp(S, g, slot, 2, l)[c] = 0;
+        for (int l = 1; l <= L; l++) memp(S, g, slot, MEM_Q, l)[c] = 0;
     T vxx = 0, vyy = 0;
 #pragma unroll
     for (int m = 1; m <= FDOH; m++) {
@@ -818,11 +820,11 @@ __device__ void surface_cell(const KGrid &g, const KState<T> &S, const KModel<T>
     }
     const T djm = srf[2 * g.nx + i - 1], e = srf[3 * g.nx + i - 1];
     T sump = 0;
-    for (int l = 1; l <= L; l++) sump += memp(S, g, slot, 1, l)[c];
+    for (int l = 1; l <= L; l++) sump += memp(S, g, slot, MEM_P, l)[c];
     sxx[c] += -(DT * (gg - fjm) * (gg - fjm) * vxx / gg) - (DT * (gg - fjm) * vyy) - (dthalbe * sump);
     sump = 0;
     for (int l = 1; l <= L; l++) {
-        T *pp = memp(S, g, slot, 1, l) + c;
+        T *pp = memp(S, g, slot, MEM_P, l) + c;
         const T bjm = g.bjm_srf[l];
         *pp = (T)((double)*pp + (double)bjm * (((double)(djm - e) * ((double)(fjm / gg) - 1.0) * (double)vxx) -
                                                 (double)((djm - e) * vyy)));

@@ -112,7 +112,7 @@ struct ifos_ctx {
     long long profx_off = 0;  // elements from prof to the x profiles by grid column
     long long slot_stride = 0, psix_len = 0, psiy_len = 0, psi_slot = 0, model_stride = 0;
     long long off[NP_FIELD];
-    long long mem_off[5];
+    long long mem_off[N_MEM];
     bool mplane[NM_PLANE];
     long long moff[NM_PLANE];
     bool tau_planes = false;                  // the kernels read the tau planes (else the scalars of g)
@@ -170,7 +170,7 @@ inline KState<T> kstate(const ifos_ctx *c) {
     s.base = (T *)c->state.p;
     s.slot_stride = c->slot_stride;
     for (int k = 0; k < NP_FIELD; k++) s.off[k] = c->off[k] < 0 ? 0 : c->off[k];
-    for (int k = 0; k < 5; k++) s.mem_off[k] = c->mem_off[k] < 0 ? 0 : c->mem_off[k];
+    for (int k = 0; k < N_MEM; k++) s.mem_off[k] = c->mem_off[k] < 0 ? 0 : c->mem_off[k];
     T *psi = (T *)c->psi.p;
     for (int k = 0; k < NX_STRIP; k++) s.psix[k] = psi + k * c->psix_len;
     for (int k = 0; k < NY_STRIP; k++) s.psiy[k] = psi + NX_STRIP * c->psix_len + k * c->psiy_len;

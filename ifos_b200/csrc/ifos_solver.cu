@@ -293,7 +293,7 @@ static void setup_pipeline(ifos_ctx *c, const Layout &L) {
     KTma &t = c->ktma;
     t.planes_per_slot = (int)(L.slot_elems / L.plane);
     for (int k = 0; k < NP_FIELD; k++) t.pid[k] = c->off[k] < 0 ? 0 : (int)(c->off[k] / L.plane);
-    for (int k = 0; k < 5; k++) t.mem_pid[k] = c->mem_off[k] < 0 ? 0 : (int)(c->mem_off[k] / L.plane);
+    for (int k = 0; k < N_MEM; k++) t.mem_pid[k] = c->mem_off[k] < 0 ? 0 : (int)(c->mem_off[k] / L.plane);
     t.model_planes = (int)(L.model_elems / L.plane);
     for (int m = 0; m < NM_PLANE; m++) t.mid[m] = c->moff[m] < 0 ? 0 : (int)(c->moff[m] / L.plane);
     const int fdoh = c->g.fdoh, xh = ((fdoh + 3) / 4) * 4;
@@ -414,13 +414,13 @@ extern "C" int ifos_ctx_create(const ifos_params *pp, int device, int with_snaps
     }
     if (p.L) {
         if (c->psv)
-            for (int w = 0; w < 3; w++) {
-                if (c->ac && w != 1) continue;  // viscoacoustic: the pressure memories only
+            for (int w = MEM_R; w <= MEM_Q; w++) {
+                if (c->ac && w != MEM_P) continue;  // viscoacoustic: the pressure memories only
                 c->mem_off[w] = k * L.plane;
                 k += p.L;
             }
         if (c->sh)
-            for (int w = 3; w < 5; w++) {
+            for (int w = MEM_T; w <= MEM_O; w++) {
                 c->mem_off[w] = k * L.plane;
                 k += p.L;
             }

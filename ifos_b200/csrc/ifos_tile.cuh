@@ -72,7 +72,7 @@ using D = std::conditional<IFOS_EXACT != 0, double, float>::type;
 struct KTma {
     int planes_per_slot;
     int pid[NP_FIELD];
-    int mem_pid[5];
+    int mem_pid[N_MEM];
     int model_planes;
     int mid[NM_PLANE];
     int snap_ntd, snap_ncomp;
@@ -1049,7 +1049,7 @@ struct OpSVisc {
     void planes(int &hz, int (&gz)[NG]) const {  // first planes of the boxes, in slot 0 and model 0
         hz = tm.pid[P_VX];
         gz[0] = tm.pid[P_SXX];
-        gz[1] = tm.mem_pid[0];
+        gz[1] = tm.mem_pid[MEM_R];
         if (!SHARED) gz[2 % NG] = tm.mid[M_FIPJPV];
     }
     // SHARED: fipjp f g mu pi muipjp of the thread's cells, loaded before the wait
@@ -1160,9 +1160,9 @@ struct OpSVisc {
                 sump[e] += mp[l].v[e];
                 sumq[e] += mq[l].v[e];
             }
-            out.put(S.mem_off[0] + l * g.plane, mr[l].v);
-            out.put(S.mem_off[1] + l * g.plane, mp[l].v);
-            out.put(S.mem_off[2] + l * g.plane, mq[l].v);
+            out.put(S.mem_off[MEM_R] + l * g.plane, mr[l].v);
+            out.put(S.mem_off[MEM_P] + l * g.plane, mp[l].v);
+            out.put(S.mem_off[MEM_Q] + l * g.plane, mq[l].v);
         }
 #pragma unroll
         for (int e = 0; e < V; e++) {
@@ -1187,7 +1187,7 @@ struct OpSVisc {
                 for (int l = 0; l < LL; l++)
 #pragma unroll
                     for (int e = 0; e < V; e++) {
-                        r.p[l][e] = e < q.nv ? out.st[S.mem_off[1] + l * g.plane + e] : 0.0f;
+                        r.p[l][e] = e < q.nv ? out.st[S.mem_off[MEM_P] + l * g.plane + e] : 0.0f;
                         r.q[l][e] = 0.0f;
                     }
                 r = surface_row<LL, V>(g, S, M, pt, q, slot, ti.model(), r);
@@ -1195,8 +1195,8 @@ struct OpSVisc {
                 for (int e = 0; e < V; e++) o[0][e] = r.xx[e], o[1][e] = r.yy[e];
 #pragma unroll
                 for (int l = 0; l < LL; l++) {
-                    out.put(S.mem_off[1] + l * g.plane, r.p[l]);
-                    out.put(S.mem_off[2] + l * g.plane, r.q[l]);
+                    out.put(S.mem_off[MEM_P] + l * g.plane, r.p[l]);
+                    out.put(S.mem_off[MEM_Q] + l * g.plane, r.q[l]);
                 }
             }
         }
@@ -1601,7 +1601,7 @@ struct OpSSh {
     void planes(int &hz, int (&gz)[NG]) const {  // first planes of the boxes, in slot 0 and model 0
         hz = tm.pid[P_VZ];
         gz[0] = tm.pid[P_SXZ];
-        gz[1] = LL ? tm.mem_pid[3] : tm.mid[M_UIPJP];
+        gz[1] = LL ? tm.mem_pid[MEM_T] : tm.mid[M_UIPJP];
         if (LL) gz[2 % NG] = tm.mid[M_FIPJPV], gz[3 % NG] = tm.mid[M_MUR], gz[4 % NG] = tm.mid[M_MUIPJPR];
     }
     struct Pre {
@@ -1687,8 +1687,8 @@ struct OpSSh {
                     sumt[e] += tt;
                     sumo[e] += oo;
                 }
-                out.put(S.mem_off[3] + l * g.plane, mt[l].v);
-                out.put(S.mem_off[V] + l * g.plane, mo[l].v);
+                out.put(S.mem_off[MEM_T] + l * g.plane, mt[l].v);
+                out.put(S.mem_off[MEM_O] + l * g.plane, mo[l].v);
             }
 #pragma unroll
             for (int e = 0; e < V; e++) {
@@ -1816,7 +1816,7 @@ struct OpPVisc {
     void planes(int &hz, int (&gz)[NG]) const {  // first planes of the boxes, in slot 0 and model 0
         hz = tm.pid[P_VX];
         gz[0] = tm.pid[P_SP];
-        gz[1] = tm.mem_pid[1];
+        gz[1] = tm.mem_pid[MEM_P];
         gz[2] = tm.mid[M_GV];
     }
     struct Pre {
@@ -1882,7 +1882,7 @@ struct OpPVisc {
                 mp[l].v[e] = pp;
                 sump[e] += pp;
             }
-            out.put(S.mem_off[1] + l * g.plane, mp[l].v);
+            out.put(S.mem_off[MEM_P] + l * g.plane, mp[l].v);
         }
 #pragma unroll
         for (int e = 0; e < V; e++) o[e] = o[e] + (dthalbe * sump[e]);
