@@ -494,6 +494,17 @@ __device__ __forceinline__ FV<V> ldv(const float *p) {
         return {{a.x, a.y}};
     }
 }
+// the same from L2, past this SM's L1
+template <int V>
+__device__ __forceinline__ FV<V> ldv_l2(const float *p) {
+    if constexpr (V == 4) {
+        const float4 a = __ldcg(reinterpret_cast<const float4 *>(p));
+        return {{a.x, a.y, a.z, a.w}};
+    } else {
+        const float2 a = __ldcg(reinterpret_cast<const float2 *>(p));
+        return {{a.x, a.y}};
+    }
+}
 template <int V>
 __device__ __forceinline__ void stv(float *p, const float (&v)[V]) {
     if constexpr (V == 4) *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
@@ -600,6 +611,13 @@ struct Lane {
 // (KGrid::psx, psy); cells of the group outside the strip have zero factors
 // and keep their difference.  The memory values are loaded before the wait
 // for the stage (Op::prefetch) and used after the differences.
+//
+// These loads may run before the preceding kernel has completed, in warps that
+// never wait for it.  Their values were stored two launches back or earlier, and
+// the launch between has waited for that one (griddepcontrol.wait, after which
+// its stores are performed) before it let this one start, so they are in L2.
+// They are read from there: a dependent launch may find lines of earlier
+// launches in L1.  No line is read twice in a launch, so nothing is lost by it.
 template <int V>
 struct Psi {
     int at;  // index of the group in its strip (-1: in no strip)
@@ -612,7 +630,7 @@ __device__ __forceinline__ void psi_x(const KGrid &g, const float *strip, const 
     const bool right = q.i + V - 1 >= g.nx - g.fw + 1;
     if (q.i > g.fw && !right) return;
     s.at = (q.j - 1) * g.psx + (right ? q.i - 1 - g.psx_rs + g.psx_lw : q.i - 1);
-    s.v = ldv<V>(strip + s.at);
+    s.v = ldv_l2<V>(strip + s.at);
 }
 template <int V>
 __device__ __forceinline__ void psi_y(const KGrid &g, const float *strip, const Lane &q, Psi<V> &s) {
@@ -620,7 +638,7 @@ __device__ __forceinline__ void psi_y(const KGrid &g, const float *strip, const 
     const int hy = q.nv == 0 ? 0 : strip_y(g, q.j);
     if (!hy) return;
     s.at = (hy - 1) * g.psy + (q.i - 1);
-    s.v = ldv<V>(strip + s.at);
+    s.v = ldv_l2<V>(strip + s.at);
 }
 // cells lo..hi of the group lie in the strip
 template <int V>
