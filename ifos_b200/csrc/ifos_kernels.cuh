@@ -643,6 +643,8 @@ struct KSrc {
     const float *sig;    // slot * max_src * NT
     const int *nsrc;     // per slot
     int max_src, nt_total;
+    const unsigned char *rows;  // per slot row_bytes bytes: bit r of byte b is set when row 8 b + r + 1 holds a source
+    int row_bytes;
 };
 struct KRec {
     const int *pos;      // slot * 2 * max_rec
@@ -658,6 +660,8 @@ struct KRec {
     const int *map;
     long long map_stride;
     int rmax;
+    const unsigned char *rows;  // rows that hold receivers, as KSrc::rows
+    int row_bytes;
 };
 
 template <typename T>

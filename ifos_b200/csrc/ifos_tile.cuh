@@ -183,6 +183,16 @@ struct TileWalk {
     enum { R_TOP, R_BOTTOM, R_PROBE, R_REC, R_SRC, NR };
     int px0, px1, top;
     int lo[NR], hi[NR];
+    // The receiver and source ranges span all slots.  Where one holds more than
+    // one row, the slot's own rows are looked up (KRec::rows, KSrc::rows; NULL:
+    // the range says it all), so that shots at several depths, or receivers in
+    // a shallow and a deep row, do not put all rows between on the longer path.
+    // A forward step with the ranges alone, with the lookup, and with one row
+    // (us): six viscoelastic shots of 2000 x 600 at six depths 261, 217 and 215;
+    // four acoustic shots of 1500 x 500 at four depths 47.2, 34.9 and 32.2; a
+    // P-SV shot of 4000 x 1200 with two receiver rows 88.5, 73.9 and 71.9.
+    const unsigned char *own[2];
+    int own_stride;
     // TMA z coordinates: planes of a slot and of a model, the halo box's first plane, the groups'
     int slot_planes, model_planes, zh, zg[kMaxGroups];
 
@@ -223,6 +233,10 @@ struct TileWalk {
         range(R_PROBE, op.probe, g.ny / 2, g.ny / 2);
         range(R_REC, op.rec_mode, op.rec_j0, op.rec_j1);
         range(R_SRC, op.fps || op.fvs, op.src_j0, op.src_j1);
+        static_assert(TY == 8, "a tile's rows are one byte of the row tables");
+        w.own[0] = w.hi[R_REC] > w.lo[R_REC] ? op.rec.rows : nullptr;
+        w.own[1] = w.hi[R_SRC] > w.lo[R_SRC] ? op.src.rows : nullptr;
+        w.own_stride = op.rec.row_bytes;
 
         int z[Op::NG];
         op.planes(w.zh, z);
@@ -265,7 +279,9 @@ struct TileWalk {
 #pragma unroll
         for (int k = 0; k < NR; k++) {
             const int a = max(lo[k] - r.j0, 0), b = min(hi[k] - r.j0, TY - 1);
-            if (a <= b) rows |= (2u << b) - (1u << a);
+            if (a > b) continue;
+            const unsigned char *p = k >= R_REC ? own[k - R_REC] : nullptr;
+            rows |= p ? p[(long long)r.slot * own_stride + ty] : (2u << b) - (1u << a);
         }
         r.bits = warps_of_rows<ROWS>(rows);
         return r;
