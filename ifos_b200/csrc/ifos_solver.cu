@@ -844,17 +844,36 @@ static int run_loop(ifos_ctx *c, LoopGraph &lg, const std::string &key, F &&enqu
     return IFOS_OK;
 }
 
-// Whether the SH and acoustic ops handle the receivers themselves.  That saves
-// launches of a few microseconds, but the tiles that hold receivers wait for
-// their scattered samples, so it pays while such tiles (a row of them per
-// shot, usually) fall to few of the blocks; in larger batches a receiver
-// kernel of its own is hidden behind the next launch's start.  Per step with
-// and without: SH 400 x 160 FDORDER 12, 1, 16 and 32 shots 7.6 / 8.2, 20.3 /
-// 22.1 and 36.4 / 36.7 us; acoustic 1500 x 500 FDORDER 8, 2, 4 and 8 shots 19.4
-// / 21.9, 35.6 / 34.9 and 70.8 / 63.4.  The P-SV ops always do.
+// Whether the ops handle the receivers themselves.  In the SH and acoustic ops
+// that saves launches of a few microseconds, but the tiles that hold receivers
+// wait for their scattered samples; in large launches a receiver kernel of its
+// own is hidden behind the next launch's start.  The line lies at 24 tiles per
+// SM: every point measured below it is faster with the receivers in the op.
+// Forward + adjoint step without and with them (us):
+//   SH 400 x 160 FDORDER 12, 1, 4, 16, 24, 32 and 64 shots (0.9 to 61 tiles per
+//     SM): 8.1 + 7.7 and 7.4 + 7.2, 10.9 + 11.4 and 8.9 + 10.3, 18.8 + 21.5 and
+//     17.2 + 20.2, 24.9 + 28.8 and 23.2 + 27.8 (23), 30.6 + 36.5 and 31.3 + 36.9
+//     (30), 55.5 + 69.7 and 62.7 + 74.2;
+//   acoustic 400 x 160 FDORDER 4, 16, 32 and 64 shots: 16.4 + 19.9 and 16.1 + 19.1
+//     (15), 25.6 + 31.6 and 28.8 + 33.7 (30), 44.6 + 61.9 and 52.8 + 67.2;
+//   1500 x 500 FDORDER 8, 2, 4 and 8 shots: SH 17.7 + 18.9 and 15.8 + 17.1 (20),
+//     27.9 + 31.5 and 26.7 + 30.4 (41), 52.5 + 60.5 and 54.6 + 61.7 (82); acoustic
+//     18.4 + 21.2 and 16.6 + 18.5, 29.6 + 35.3 and 30.5 + 33.8, 54.4 + 73.6 and
+//     61.5 + 73.7;
+//   acoustic 777 x 259 FDORDER 6, 8 and 16 shots: 23.3 + 30.2 and 22.8 + 30.2 (23),
+//     39.5 + 52.7 and 37.9 + 52.1 (46); 4000 x 1200, one shot (64): SH 48.9 + 53.9
+//     and 50.1 + 55.2, acoustic 49.6 + 61.2 and 51.0 + 60.6.
+// Above the line either form wins, the op by up to 4 %, the separate kernel by up
+// to 18 %.
+//
+// The P-SV ops always do: 4000 x 1200 FDORDER 8 78.0 + 97.8 without and 73.7 + 93.1
+// with, 1500 x 500, 4 shots, 45.2 + 59.7 and 43.3 + 55.4; viscoelastic 2000 x 600, 1
+// and 6 shots, 42.9 + 46.5 and 39.8 + 43.2, 203.5 + 232.2 and 203.6 + 231.0; 400 x
+// 160 FDORDER 4, 1 and 64 shots, 10.5 + 10.7 and 8.0 + 9.6, 88.3 + 113.5 and 85.9 +
+// 113.4.  (The adjoint of 16 such shots is the exception: 32.6 without, 35.2 with.)
 static bool rec_in_op(const ifos_ctx *c, int nshots) {
-    const long long tiles = (long long)nshots * ((c->p.nx + kTileX - 1) / kTileX);
-    return (c->psv && !c->ac) || 3 * tiles <= 2LL * c->num_sms;
+    const long long tiles = (long long)((c->p.nx + kTileX - 1) / kTileX) * ((c->p.ny + kTileY - 1) / kTileY) * nshots;
+    return (c->psv && !c->ac) || tiles <= 24LL * c->num_sms;
 }
 
 static std::string loop_key(const ifos_ctx *c, std::initializer_list<long long> v) {
