@@ -409,30 +409,35 @@ struct Launcher {
         }
         if (c->sh) pipelined(OpVSh<FD, kTileY, ring_stages<FD, 2, 2, 0, kTileY, vblocks(FD)>()>{c->g, S, M, c->ktma, snap_out(hin)});
     }
-    template <int FD, int LL, bool SHARED>
+    template <int FD, int LL, bool DIRECT>
     void s_visc_psv(int hin) {
         const KGrid &g = c->g;
-        constexpr int NST = ring_stages<FD, 2, 3 + 3 * LL + (SHARED ? 0 : 6), 0, kTileY, visc_blocks(LL)>();
+        constexpr int NST = ring_stages<FD, 2, 3 + 3 * LL + (DIRECT ? 0 : 6), 0, kTileY, visc_blocks(LL)>();
         if constexpr (FD >= 5) {
             if (g.quirk_hi) {
-                pipelined(OpSVisc<FD, kTileY, LL, NST, true, SHARED>{g, S, M, c->ktma, snap_out(hin)});
+                pipelined(OpSVisc<FD, kTileY, LL, NST, true, DIRECT>{g, S, M, c->ktma, snap_out(hin)});
                 return;
             }
         }
-        pipelined(OpSVisc<FD, kTileY, LL, NST, false, SHARED>{g, S, M, c->ktma, snap_out(hin)});
+        pipelined(OpSVisc<FD, kTileY, LL, NST, false, DIRECT>{g, S, M, c->ktma, snap_out(hin)});
     }
     template <int FD, int LL>
     void s_visc_pipe(int hin) {
         if (c->psv) {
-            // OpSVisc's SHARED form pays when the state streams from HBM
-            // (above about twice the L2) and few tiles hold strip cells.  A
-            // forward step with and without: 2000 x 600, 2, 4, 6 and 12 shots 81
-            // / 80, 153 / 157, 220 / 234 and 439 / 500 us; 1300 x 400, 4, 8 and 24
-            // shots 69 / 67, 131 / 134 and 403 / 416; 593 x 246, 8 and 24 shots
-            // 46.0 / 44.5 and 134 / 136 (adjoint 150 / 145).
+            // OpSVisc's DIRECT form (visc_direct) pays when the state streams
+            // from HBM (above about twice the L2) and few tiles hold strip
+            // cells.  Forward + adjoint step without and with it at L 3,
+            // FDORDER 8 (us): 2000 x 600, 1, 2, 4 and 6 shots 39.4 + 43.0 / 41.3 +
+            // 46.3, 73.9 + 83.8 / 74.1 + 85.6, 147 + 163 / 141 + 160 and 220 + 239 /
+            // 203 + 228; 1300 x 400, 4, 8 and 24 shots 64.5 + 70.9 / 64.8 + 73.2, 130 +
+            // 142 / 126 + 140 and 415 + 443 / 402 + 451; 593 x 246, 24 shots 125 + 132 /
+            // 124 + 136.
             const long long cells = (long long)c->p.nx * c->p.ny;
-            if ((c->g.tile_order & 1) && cells >= 300000 && cells * nshots >= 4000000) s_visc_psv<FD, LL, true>(hin);
-            else s_visc_psv<FD, LL, false>(hin);
+            const bool large = (c->g.tile_order & 1) && cells >= 300000 && cells * nshots >= 4000000;
+            if constexpr (visc_direct(FD, LL)) {
+                if (large) s_visc_psv<FD, LL, true>(hin);
+            }
+            if (!(visc_direct(FD, LL) && large)) s_visc_psv<FD, LL, false>(hin);
         }
         if (c->sh) pipelined(OpSSh<FD, kTileY, LL, ring_stages<FD, 1, 2 + 2 * LL + 4, 0, kTileY, 3>()>{c->g, S, M, c->ktma, snap_out(hin)});
     }

@@ -44,6 +44,26 @@ namespace ifos {
 constexpr int sblocks(int fdoh) { return fdoh <= 2 ? 4 : 3; }
 constexpr int vblocks(int fdoh) { return fdoh <= 2 ? 4 : 3; }
 constexpr int visc_blocks(int LL) { return LL <= 1 ? 3 : 2; }
+// Half widths and memory variables for which the viscoelastic stress's DIRECT
+// form is faster on large batches (Launcher::s_visc_pipe), 4 shots of 2000 x
+// 600, forward + adjoint step without and with it (us), with one model, and
+// with a model per shot:
+//   L 3, FDORDER 2, 4, 6, 8 and 12: 144 + 161 and 140 + 158, 144 + 165 and 139 + 161,
+//     145 + 161 and 140 + 160, 147 + 163 and 141 + 160, 140 + 145 and 133 + 138; models
+//     160 + 178 and 157 + 176, 160 + 183 and 156 + 179, 160 + 179 and 156 + 176, 163 +
+//     181 and 156 + 176, 157 + 162 and 149 + 155;
+//   L 4, FDORDER 4, 8 and 12: 171 + 192 and 167 + 184, 174 + 192 and 162 + 185, 161 +
+//     168 and 160 + 166; models 187 + 209 and 182 + 202, 190 + 210 and 178 + 201, 167 +
+//     174 and 174 + 181 (24 shots of 1300 x 400: 436 + 451 and 544 + 558);
+//   L 1, FDORDER 2, 4, 6, 8, 10 and 12: 98 + 116 and 129 + 115, 100 + 145 and 126 +
+//     123 (24 of 1300 x 400: 243 + 334 and 327 + 325), 124 + 135 and 101 + 153, 130 +
+//     143 and 107 + 142, 103 + 111 and 105 + 112, 103 + 111 and 91 + 102;
+//   L 2, FDORDER 4, 8 and 12: 115 + 138 and 122 + 144, 118 + 134 and 124 + 142, 111 +
+//     116 and 111 + 117; L 5: 183 + 204 and 195 + 214, 187 + 202 and 194 + 217, 176 + 183
+//     and 188 + 195.
+constexpr bool visc_direct(int fdoh, int LL) {
+    return LL == 3 || (LL == 4 && fdoh <= 4) || (LL == 1 && (fdoh == 3 || fdoh == 4 || fdoh == 6));
+}
 constexpr int kTileX = 64;
 // Cells per thread.  Four halve the loads, addresses and bookkeeping per cell;
 // two leave room for twice the warps.  Four win where instructions bound the
@@ -1063,32 +1083,31 @@ static __device__ __noinline__ Cells4 force_row_sh(const KGrid &g, const KSrc &s
 // reference 10/12 default :615-660 has no CPML and zero-started sums: QUIRK)
 // halo: vx vy; plain: sxx syy sxy, r[LL] p[LL] q[LL], fipjp f g mu pi muipjp;
 // writes sxx syy sxy r p q.  Non-uniform tau planes are read from HBM.
-// SHARED: the shots of the launch walk the same tile side by side, so that all
-// but one of them find the model's coefficients in L2; they are then loaded
-// into registers before the wait for the stage instead of through the ring,
-// whose stages shrink from 46 to 34 KB and are three instead of two.
-template <int FDOH, int TY, int LL, int NST, bool QUIRK, bool SHARED>
+// DIRECT: the model's coefficients are loaded into registers before the wait
+// for the stage instead of through the ring, whose stages shrink (L 3: from 46
+// to 34 KB, three instead of two).
+template <int FDOH, int TY, int LL, int NST, bool QUIRK, bool DIRECT>
 struct OpSVisc {
     static constexpr int V = kCellsVisc;
-    static constexpr bool EARLY = SHARED;
+    static constexpr bool EARLY = DIRECT;
     static constexpr int DEP_TILES = INT_MAX;
-    static constexpr int NH_ = 2, NP_ = 3 + 3 * LL + (SHARED ? 0 : 6);
+    static constexpr int NH_ = 2, NP_ = 3 + 3 * LL + (DIRECT ? 0 : 6);
     static constexpr bool CPML = !QUIRK, MIRROR = false;
     using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, visc_blocks(LL), V>;
     IFOS_OP_MEMBERS
     // boxes of consecutive planes: their number, planes of box k, whether they are model planes
-    static constexpr int NG = SHARED ? 2 : 3;
+    static constexpr int NG = DIRECT ? 2 : 3;
     __host__ __device__ static constexpr int gd(int k) { return k == 0 ? 3 : (k == 1 ? 3 * LL : 6); }
     __host__ __device__ static constexpr bool gm(int k) { return k == 2; }
     void planes(int &hz, int (&gz)[NG]) const {  // first planes of the boxes, in slot 0 and model 0
         hz = tm.pid[P_VX];
         gz[0] = tm.pid[P_SXX];
         gz[1] = tm.mem_pid[MEM_R];
-        if (!SHARED) gz[2 % NG] = tm.mid[M_FIPJPV];
+        if (!DIRECT) gz[2 % NG] = tm.mid[M_FIPJPV];
     }
-    // SHARED: fipjp f g mu pi muipjp of the thread's cells, loaded before the wait
+    // DIRECT: fipjp f g mu pi muipjp of the thread's cells, loaded before the wait
     struct Pre {
-        FV<V> c[SHARED ? 6 : 1];
+        FV<V> c[DIRECT ? 6 : 1];
         Psi<V> x0, x1, y0, y1;
     };
     template <bool EDGE>
@@ -1147,7 +1166,7 @@ struct OpSVisc {
         const FV<V> s0 = ld(0), s1 = ld(1), s2 = ld(2);
         FV<V> co[6];
 #pragma unroll
-        for (int k = 0; k < 6; k++) co[k] = SHARED ? pre.c[SHARED ? k : 0] : ld(3 + 3 * LL + k);
+        for (int k = 0; k < 6; k++) co[k] = DIRECT ? pre.c[DIRECT ? k : 0] : ld(3 + 3 * LL + k);
         const FV<V> &fipjp = co[0], &f = co[1], &gg = co[2], &mu = co[3], &pi = co[4], &muij = co[5];
         FV<V> mr[LL], mp[LL], mq[LL];
 #pragma unroll

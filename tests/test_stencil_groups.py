@@ -183,3 +183,29 @@ def test_batches_of_few_and_more_tiles_per_sm(name, n, nx):
             grads = s.adjoint(np.stack([adj] * shots), shots)
         for k in range(shots):
             assert bit_equal(sec[k], ref["sections"]) and bit_equal(grads[k], ref["grads"]), k
+
+
+@pytest.mark.parametrize("fdorder,L", [(2, 3), (4, 3), (6, 1), (8, 1), (12, 1), (12, 3), (4, 4), (8, 4), (8, 2), (10, 3)])
+def test_large_viscoelastic_batches_by_order_and_mechanisms(fdorder, L):
+    """Each form that a large viscoelastic batch takes by FDORDER and L
+    (coefficients in registers or through the ring, with and without CPML in
+    the stress): every slot equals the same shot alone, which takes the ring."""
+    nx, ny, n = 703, 431, 14  # 303 000 cells, 4.2 million in the batch
+    p, model, g, sig, adj = build_case("psv_visc_o4", nx=nx, ny=ny, nt=9, fw=20)
+    p.dtinv, p.fdorder = 3, fdorder
+    p.L, p.fl = L, [5.0 * 2 ** k for k in range(L)]
+    ntr = g.recpos.shape[1]
+    with ShotSolver(p, max_rec=ntr) as s:
+        s.upload_model(model)
+        s.setup_shot(0, g.srcpos, sig, g.recpos)
+        alone = s.forward(1)[0], s.adjoint(adj[None])[0]
+    with ShotSolver(p, max_shots=n, max_rec=ntr) as s:
+        s.set_options(tile_order=3)
+        s.upload_model(model)
+        for k in range(n):
+            s.setup_shot(k, g.srcpos, sig, g.recpos)
+        sec = s.forward(n)
+        grads = s.adjoint(np.stack([adj] * n), n)
+    for k in range(n):
+        assert bit_equal(sec[k], alone[0]) and bit_equal(grads[k], alone[1]), k
+    assert np.abs(alone[1]).max() > 0
