@@ -219,9 +219,10 @@ class Clocks:
 
 # ---------------------------------------------------------------------------
 def _ref_sample(args):
-    """One bounded sample of the workload through the reference's own C code
-    (oracle/_ref): forward + adjoint of `ns` steps on the full grid."""
-    ns, seed = args
+    """One bounded sample of the workload through an oracle library (`kind`:
+    the reference's own C code, or the restatement where that is not built):
+    forward + adjoint of `ns` steps on the full grid."""
+    kind, ns, seed = args
     from oracle import oracle as O
     from ifos_b200 import workloads as W
     p, model, geoms = workload(ns)
@@ -230,7 +231,7 @@ def _ref_sample(args):
     rng = np.random.default_rng(seed)
     adj = (rng.standard_normal((3, g.recpos.shape[1], p.nt)) * 1e-6).astype(np.float32)
     t0 = time.perf_counter()
-    O.run_shot("ref", p, model, g.srcpos, sig, g.recpos, run_adjoint=True, adj=adj, want_fields=False)
+    O.run_shot(kind, p, model, g.srcpos, sig, g.recpos, run_adjoint=True, adj=adj, want_fields=False)
     return time.perf_counter() - t0
 
 
@@ -242,6 +243,7 @@ def cpu_baseline(full_nt, procs=None, ns=30):
     sample to the full NT."""
     from oracle import oracle as O
     kind = "reference" if O.available("ref") else "port"
+    lib = "ref" if kind == "reference" else "restate"
     ncpu = os.cpu_count() or 1
     try:
         import psutil
@@ -253,7 +255,7 @@ def cpu_baseline(full_nt, procs=None, ns=30):
     ctx = mp.get_context("spawn")
     with ctx.Pool(procs) as pool:
         t0 = time.perf_counter()
-        times = pool.map(_ref_sample, [(ns, k) for k in range(procs)])
+        times = pool.map(_ref_sample, [(lib, ns, k) for k in range(procs)])
         wall = time.perf_counter() - t0
     value = procs / wall * (ns / full_nt)
     return {"value": value, "unit": METRIC, "cores": procs, "host_cores": ncpu,
@@ -588,6 +590,12 @@ def reference_arm(args):
     time steps of one shot on the full grid, a few seconds), and the value is
     the work of all timed steps over their total time, scaled to whole
     shot-gradients."""
+    from oracle import oracle as O
+    if not O.available("ref"):
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "oracle/_ref/libifosref.so is not built: the reference's sources are not on this machine"}),
+              flush=True)
+        return
     p, model, geoms = workload(args.nt)
     for _ in range(max(0, args.warmup)):
         cpu_baseline(p.nt)
@@ -853,7 +861,10 @@ def main():
                 extra[name] = {"error": repr(exc)}
     cpu = None
     if not args.no_cpu and world == 1:
-        cpu = cpu_baseline(p.nt)
+        try:
+            cpu = cpu_baseline(p.nt)
+        except Exception as exc:  # the device's results stand without it
+            cpu = {"error": repr(exc)}
     lat = sorted(step_ms)
     line = {
         "metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": args.steps,
