@@ -20,8 +20,9 @@ never what they compute (every setting is bit-identical):
 
 ``tune()`` times a short forward + adjoint (a few snapshot intervals of the
 same grid, physics and FDORDER) for each candidate on the device and returns
-the fastest; results are cached per key in a JSON file (``IFOS_TUNE_CACHE``,
-default ``~/.cache/ifos_b200/tune.json``).
+the fastest; results are cached per key (device, library build, grid, physics,
+batch) in a JSON file (``IFOS_TUNE_CACHE``, default
+``~/.cache/ifos_b200/tune.json``).
 """
 from __future__ import annotations
 
@@ -51,8 +52,19 @@ def _device_name(device: int) -> str:
         return f"cuda:{device}"
 
 
+def _library_stamp() -> str:
+    """The digest of the library's sources and flags (build.py writes it beside
+    the library): options measured with other kernels are not reused."""
+    from . import build
+    try:
+        with open(build.LIB + ".stamp") as fh:
+            return fh.read().strip()[:16]
+    except OSError:
+        return "unstamped"
+
+
 def tune_key(p: ShotParams, nshots: int, snap_format: str, device: int = 0) -> str:
-    return "|".join(str(x) for x in (_device_name(device), p.wavetype, p.acoustic, p.L, p.fdorder, p.nx, p.ny,
+    return "|".join(str(x) for x in (_device_name(device), _library_stamp(), p.wavetype, p.acoustic, p.L, p.fdorder, p.nx, p.ny,
                                      p.fw, p.free_surf, nshots, snap_format))
 
 

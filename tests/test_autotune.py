@@ -86,3 +86,23 @@ def test_best_batch_tries_three_times_powers_of_two(monkeypatch):
     best = A.best_batch(p, {}, free_bytes=int(151e9), max_batch=8)
     assert tried == [1, 2, 3, 4, 6]  # 8 shots need 200 GB
     assert best["nshots"] == 6
+
+
+def test_options_of_another_library_build_are_not_reused(tmp_path, monkeypatch):
+    """The cache key holds the library's stamp: new kernels are timed anew."""
+    from ifos_b200 import build
+    monkeypatch.setenv("IFOS_TUNE_CACHE", str(tmp_path / "tune.json"))
+    monkeypatch.setattr(A, "_device_name", lambda d: "fake")
+    monkeypatch.setattr(build, "LIB", str(tmp_path / "lib.so"))
+    calls = []
+
+    def fake_time(p, model, nshots, options, snap_format="fp32", device=0, reps=3):
+        calls.append(1)
+        return [(1.0, o) for o in options]
+
+    monkeypatch.setattr(A, "time_options", fake_time)
+    p = ShotParams(nx=64, ny=40, nt=90, dtinv=3)
+    for stamp, timed in (("a" * 64, 1), ("a" * 64, 1), ("b" * 64, 2)):
+        (tmp_path / "lib.so.stamp").write_text(stamp + "\n")
+        A.tune(p, {}, nshots=2)
+        assert len(calls) == timed
