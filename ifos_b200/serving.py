@@ -113,13 +113,18 @@ class GpuBackend:
 
     def create(self, p: ShotParams, kind: str, nshots: int, max_models: int, max_src: int, max_rec: int,
                snap_format: str, model: Optional[dict] = None):
-        """A context for the batch.  Its execution options are the ones the
-        autotuner picked on the measured workloads (graph replay, no PDL,
-        slot-minor tiles for several shots, CPML strip tiles first for one);
-        with ``tune`` they are timed
-        once per shape (at two shots, then cached) instead."""
+        """A context for the batch.  Its execution options are the fastest of
+        the measured ones: graph replay, dependent launches (a forward and an
+        adjoint step of contexts alone, without and with them: 777 x 259
+        acoustic, one shot, 19.4 and 15.0 us; 1010 x 336 viscoelastic, one and
+        eight, 40.4 and 33.9, 198.6 and 195.4; 300 x 100 elastic, one, 20.0 and
+        15.8), strip tiles first for one shot, slot-minor tiles for several
+        (three lanes at once, 64 requests of the scaled stream, three runs
+        each: 38.9-40.9 requests/s at saturation; with the strips first as well
+        30.7-37.8; without dependent launches 30.8-39.2).  With ``tune`` they are
+        timed once per shape (at two shots, then cached) instead."""
         from .solver import ShotSolver
-        opts = dict(graphs=1, pdl=0, tile_order=1 if nshots > 1 else 2)
+        opts = dict(graphs=1, pdl=1, tile_order=1 if nshots > 1 else 2)
         if self.tune and model is not None and kind == GRADIENT:
             from . import autotune
             opts = autotune.tune(p, model, 2, snap_format, self.device)
