@@ -43,6 +43,7 @@ def test_slots_and_components_in_one_launch(case, planes):
     obs = (rng.standard_normal((2, 3, ntr, p.nt)) * 1e-6).astype(np.float32)
     kill = np.zeros((2, ntr), np.int32)
     kill[1, ntr // 2] = 1
+    adj = np.zeros((2, 3, ntr, p.nt), np.float32)
     with ShotSolver(p, max_shots=2, max_rec=ntr) as s:
         s.upload_model(model)
         s.setup_shot(0, g.srcpos, sig, g.recpos)
@@ -52,6 +53,13 @@ def test_slots_and_components_in_one_launch(case, planes):
         for slot, live in ((0, np.arange(ntr)), (1, np.delete(np.arange(ntr - 1), ntr // 2))):
             want = np.zeros(2)
             for k in planes:
-                _, a, b = s.calc_res(obs[slot, k][live], sec[slot, sec_plane[k]][live])
+                diff, a, b = s.calc_res(obs[slot, k][live], sec[slot, sec_plane[k]][live])
                 want += (a, b)
+                adj[slot, k, live] = diff
             np.testing.assert_allclose((l2[slot], en[slot]), want, rtol=1e-13)
+        # the residual traces: the adjoint of the staged ones equals that of the single calls' traces
+        s.forward(2, store=True, fetch=False)
+        s.residual_adjoint(obs, 2, kill=kill)
+        staged = s.adjoint(None, 2)
+        assert bit_equal(staged, s.adjoint(adj, 2))
+        assert all(np.abs(staged[slot]).max() > 0 for slot in range(2))
