@@ -63,7 +63,7 @@ struct KGrid {
     // a right-strip profile index (psx_roff).  Four cells of a group whose
     // first column is a multiple of 4 are 16-byte aligned in every strip.
     int psx, psy, psx_lw, psx_rs, psx_roff;
-    float div_lo, div_hi;  // |x| for which div_dh4 uses the reciprocal
+    float div_lo, div_hi;  // |x| for which div_dh uses the reciprocal
     int lame;        // PARAMETERIZATION 3: the model planes hold lambda and mu, the assembly stops at the moduli
 };
 
@@ -569,10 +569,6 @@ __global__ void k_p_visc(KGrid g, KState<T> S, KModel<T> M) {
     sp[c] += (dthalbe * sump);
 }
 
-// Cells of a snapshot that the stencil kernels stored and a later kernel of
-// the same step changes (explosive sources, the free surface): base of the
-// snapshot of slot 0 being stored (NULL: nothing to patch), floats between
-// slots, NX*NY, and the component index of every patched field (-1 absent).
 // fp16 snapshot segments (IFOS_SNAP_F16S).  The 64 consecutive cells of a
 // row that one pipelined tile covers share one fp32 scale: the segment's
 // absolute maximum m is mapped to kSegTop, just below fp16's largest finite
@@ -621,11 +617,16 @@ __device__ __forceinline__ float seg_unpack(unsigned short u, bool i16) {
     return i16 ? (float)(short)u : __half2float(__ushort_as_half(u));
 }
 
+// Cells of a snapshot that the stencil kernels stored and a later kernel of
+// the same step changes (the explosive sources and the free surface of P-SV and
+// SH together): base of the snapshot of slot 0 being stored (NULL: nothing to
+// patch), floats between slots, NX*NY, and the component index of every
+// patched field (-1 absent).
 struct KSnapPatch {
     float *base;
     long long slot_floats;
     long long n;
-    int c_sxx, c_syy, c_sp, c_syz;
+    int c_sxx, c_syy, c_syz;
 };
 __device__ __forceinline__ void snap_patch(const KSnapPatch &pt, int slot, int comp, const KGrid &g, int j, int i,
                                            float v) {
@@ -655,11 +656,10 @@ struct KRec {
     // the cell -> receiver map the velocity ops use to sample or inject the
     // receivers in place: per slot map_stride ints, first NY row entries
     // (-1: no receiver in the row, else the row's index among the slot's
-    // receiver rows), then rmax rows of NX cell entries (-1 or the index of
+    // receiver rows), then kRecMapRows rows of NX cell entries (-1 or the index of
     // the receiver in the cell)
     const int *map;
     long long map_stride;
-    int rmax;
     const unsigned char *rows;  // rows that hold receivers, as KSrc::rows
     int row_bytes;
 };
@@ -758,7 +758,6 @@ __device__ void psource_apply(const KGrid &g, const KState<T> &S, const KSrc &sr
     } else {
         T *sp = fieldp(S, slot, P_SP);
         sp[c] += (T)amp;
-        snap_patch(pt, slot, pt.c_sp, g, j, i, (float)sp[c]);
     }
 }
 
@@ -789,7 +788,6 @@ __device__ void surface_cell(const KGrid &g, const KState<T> &S, const KModel<T>
     const long long c = pidx(g, j, i);
     if (acoustic) {
         fieldp(S, slot, P_SP)[c] = 0;
-        snap_patch(pt, slot, pt.c_sp, g, j, i, 0.0f);
         return;
     }
     if (sh) {

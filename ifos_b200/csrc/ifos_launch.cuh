@@ -36,9 +36,9 @@ constexpr int kBlockSmem = 1024 + 2 * kTileBatch * (int)sizeof(TileInfo) + 6 * (
 
 // Stages of an op's shared-memory ring: as many as fit when `blocks` blocks
 // share an SM's 227 KB (1..6).
-template <int FD, int NH, int NP, int NO, int TY, int RB>
+template <int FD, int NH, int NP, int TY, int RB>
 constexpr int ring_stages() {
-    constexpr size_t stage = Pipe<FD, TY, NH, NP, NO, 1>::bytes();
+    constexpr size_t stage = Pipe<FD, TY, NH, NP, 1>::bytes();
     constexpr int n = (int)((232448 / RB - kBlockSmem) / stage);
     return n < 1 ? 1 : (n > 6 ? 6 : n);
 }
@@ -218,7 +218,6 @@ inline KRec krec(const ifos_ctx *c) {
     r.row_bytes = (c->p.ny + 7) / 8;
     r.map = (const int *)c->rec_map.p;
     r.map_stride = (long long)c->p.ny + (long long)kRecMapRows * c->p.nx;
-    r.rmax = kRecMapRows;
     return r;
 }
 inline KSnap ksnap(const ifos_ctx *c) {
@@ -378,19 +377,19 @@ struct Launcher {
         const KTma &t = c->ktma;
         if (c->ac) {
             constexpr int NP = (SW == 1 && !Q) ? 6 : 4;
-            pipelined(OpVPsv<FD, kTileY, ring_stages<FD, 1, NP, 0, kTileY, vblocks(FD)>(), Q, SW, P1, true>{g, S, M, t, snap_out(hin)});
+            pipelined(OpVPsv<FD, kTileY, ring_stages<FD, 1, NP, kTileY, vblocks(FD)>(), Q, SW, P1, true>{g, S, M, t, snap_out(hin)});
             return;
         }
         if (c->psv) {
             constexpr int NP = (SW == 1 && !Q) ? 6 : 4;
             if constexpr (FD <= 2) {
                 if (small(4)) {
-                    pipelined(OpVPsv<FD, kTileY, ring_stages<FD, 3, NP, 0, kTileY, vblocks(FD)>(), Q, SW, P1, false, true>{
+                    pipelined(OpVPsv<FD, kTileY, ring_stages<FD, 3, NP, kTileY, vblocks(FD)>(), Q, SW, P1, false, true>{
                         g, S, M, t, snap_out(hin)});
                     return;
                 }
             }
-            pipelined(OpVPsv<FD, kTileY, ring_stages<FD, 3, NP, 0, kTileY, vblocks(FD)>(), Q, SW, P1, false>{g, S, M, t, snap_out(hin)});
+            pipelined(OpVPsv<FD, kTileY, ring_stages<FD, 3, NP, kTileY, vblocks(FD)>(), Q, SW, P1, false>{g, S, M, t, snap_out(hin)});
         }
     }
     template <int FD>
@@ -407,12 +406,12 @@ struct Launcher {
             else if (want_p1) v_one<FD, false, 0, true>(hin);
             else v_one<FD, false, 0, false>(-1);
         }
-        if (c->sh) pipelined(OpVSh<FD, kTileY, ring_stages<FD, 2, 2, 0, kTileY, vblocks(FD)>()>{c->g, S, M, c->ktma, snap_out(hin)});
+        if (c->sh) pipelined(OpVSh<FD, kTileY, ring_stages<FD, 2, 2, kTileY, vblocks(FD)>()>{c->g, S, M, c->ktma, snap_out(hin)});
     }
     template <int FD, int LL, bool DIRECT>
     void s_visc_psv(int hin) {
         const KGrid &g = c->g;
-        constexpr int NST = ring_stages<FD, 2, 3 + 3 * LL + (DIRECT ? 0 : 6), 0, kTileY, visc_blocks(LL)>();
+        constexpr int NST = ring_stages<FD, 2, 3 + 3 * LL + (DIRECT ? 0 : 6), kTileY, visc_blocks(LL)>();
         if constexpr (FD >= 5) {
             if (g.quirk_hi) {
                 pipelined(OpSVisc<FD, kTileY, LL, NST, true, DIRECT>{g, S, M, c->ktma, snap_out(hin)});
@@ -439,11 +438,11 @@ struct Launcher {
             }
             if (!(visc_direct(FD, LL) && large)) s_visc_psv<FD, LL, false>(hin);
         }
-        if (c->sh) pipelined(OpSSh<FD, kTileY, LL, ring_stages<FD, 1, 2 + 2 * LL + 4, 0, kTileY, 3>()>{c->g, S, M, c->ktma, snap_out(hin)});
+        if (c->sh) pipelined(OpSSh<FD, kTileY, LL, ring_stages<FD, 1, 2 + 2 * LL + 4, kTileY, 3>()>{c->g, S, M, c->ktma, snap_out(hin)});
     }
     template <int FD, int LL>
     void p_visc_pipe(int hin) {
-        pipelined(OpPVisc<FD, kTileY, LL, ring_stages<FD, 2, 3 + LL, 0, kTileY, 3>()>{c->g, S, M, c->ktma, snap_out(hin)});
+        pipelined(OpPVisc<FD, kTileY, LL, ring_stages<FD, 2, 3 + LL, kTileY, 3>()>{c->g, S, M, c->ktma, snap_out(hin)});
     }
     template <int FD>
     void s_pipe_(int hin) {
@@ -462,7 +461,7 @@ struct Launcher {
             return;
         }
         if (c->ac) {
-            constexpr int NST = ring_stages<FD, 2, 2, 0, kTileY, sblocks(FD)>();
+            constexpr int NST = ring_stages<FD, 2, 2, kTileY, sblocks(FD)>();
             if constexpr (FD >= 5) {
                 if (quirk) {
                     pipelined(OpPAc<FD, kTileY, NST, true>{g, S, M, t, snap_out(hin)});
@@ -475,7 +474,7 @@ struct Launcher {
         switch (g.L) {
             case 0:
                 if (c->psv) {
-                    constexpr int NST = ring_stages<FD, 2, 6, 0, kTileY, sblocks(FD)>();
+                    constexpr int NST = ring_stages<FD, 2, 6, kTileY, sblocks(FD)>();
                     bool done = false;
                     if constexpr (FD >= 5) {
                         if (quirk) {
@@ -490,7 +489,7 @@ struct Launcher {
                     }
                     if (!done) pipelined(OpSEl<FD, kTileY, NST, false>{g, S, M, t, snap_out(hin)});
                 }
-                if (c->sh) pipelined(OpSSh<FD, kTileY, 0, ring_stages<FD, 1, 4, 0, kTileY, sblocks(FD)>()>{g, S, M, t, snap_out(hin)});
+                if (c->sh) pipelined(OpSSh<FD, kTileY, 0, ring_stages<FD, 1, 4, kTileY, sblocks(FD)>()>{g, S, M, t, snap_out(hin)});
                 break;
             case 1: s_visc_pipe<FD, 1>(hin); break;
             case 2: s_visc_pipe<FD, 2>(hin); break;

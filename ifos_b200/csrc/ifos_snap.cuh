@@ -80,11 +80,11 @@ __global__ void k_snap_seg16(KGrid g, KState<T> S, KSnap sn, int hin) {
 // cells after the stress kernel stored them, so those segments are stored
 // again from the final state.  Grid (segs + max_src, 1, slots), one warp.
 template <typename T>
-__global__ void k_snap_fix16(KGrid g, KState<T> S, KSnap sn, int hin, KSrc src, int surf, int4 patched) {
+__global__ void k_snap_fix16(KGrid g, KState<T> S, KSnap sn, int hin, KSrc src, int surf, int3 patched) {
     pdl_wait();
     pdl_launch();
     const int slot = blockIdx.z;
-    const int comps[4] = {patched.x, patched.y, patched.z, patched.w};
+    const int comps[3] = {patched.x, patched.y, patched.z};
     int j, seg;
     if ((int)blockIdx.x < sn.segs) {
         if (!surf) return;
@@ -99,7 +99,7 @@ __global__ void k_snap_fix16(KGrid g, KState<T> S, KSnap sn, int hin, KSrc src, 
         if (i < 1 || i > g.nx || j < 1 || j > g.ny) return;
         seg = (i - 1) / kSegCells;
     }
-    quant_seg<T>(g, S, sn, slot, hin, j, seg, comps, 4);
+    quant_seg<T>(g, S, sn, slot, hin, j, seg, comps, 3);
 }
 
 // fp32/fp64 snapshot copy (one thread per cell, all components)

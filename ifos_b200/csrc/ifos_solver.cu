@@ -306,8 +306,6 @@ static void setup_pipeline(ifos_ctx *c, const Layout &L) {
             (d <= 6 && !encode_planes(&c->tmaps[MAP_MODEL][d], c->models.p, L.pitch, L.rows, md_planes, kTileX, kTileY, d)))
             return;
     // fp32 snapshots are written by the stencil kernels themselves
-    t.snap_ntd = c->p.nt / c->p.dtinv;
-    t.snap_ncomp = c->ncomp;
     for (int k = 0; k < NP_FIELD; k++) t.snap_comp[k] = -1;
     for (int k = 0; k < c->ncomp; k++) t.snap_comp[c->comp_plane[k]] = k;
     // int16 segments are stored by k_snap_seg16 after the step, which keeps
@@ -950,7 +948,6 @@ static int forward_t(ifos_ctx *c, int nshots, int store, int nsteps) {
     };
     pt.c_sxx = comp_of(P_SXX);
     pt.c_syy = comp_of(P_SYY);
-    pt.c_sp = comp_of(P_SP);
     pt.c_syz = comp_of(P_SYZ);
     CK(cudaEventRecord(c->ev0, c->st));
     auto enqueue = [&]() {
@@ -981,7 +978,7 @@ static int forward_t(ifos_ctx *c, int nshots, int store, int nsteps) {
         Lr.post_fwd(nt, c->psv != 0, pt);
         if (snap_now && fused) {
             if (f16s && !in_stress && (p.free_surf || c->psv)) {
-                const int4 patched = make_int4(pt.c_sxx, pt.c_syy, pt.c_sp, pt.c_syz);
+                const int3 patched = make_int3(pt.c_sxx, pt.c_syy, pt.c_syz);
                 launch_dep(c->st, c->pdl, k_snap_fix16<T>, dim3(segs + std::max(1, p.max_src), 1, nshots), dim3(32),
                            0, c->g, Lr.S, sn, hin, Lr.src, p.free_surf ? 1 : 0, patched);
                 c->launches++;

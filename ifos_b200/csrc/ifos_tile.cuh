@@ -95,7 +95,6 @@ struct KTma {
     int mem_pid[N_MEM];
     int model_planes;
     int mid[NM_PLANE];
-    int snap_ntd, snap_ncomp;
     int snap_comp[NP_FIELD];  // component index of a state plane (-1: not stored)
 };
 
@@ -108,9 +107,6 @@ struct KMaps {
     CUtensorMap grp[kMaxGroups];  // state or model planes, box 64 x TY x GD[k]
 };
 
-// fp32 snapshot written by a launch: snapshot of slot 0 being stored (NULL:
-// none), floats between slots, NX*NY, and whether rows start 8-byte aligned
-// (NX even) for pair stores.
 // the snapshot a stencil launch stores (base NULL: none)
 struct KSnapOut {
     char *base;            // this snapshot of slot 0
@@ -122,9 +118,10 @@ struct KSnapOut {
     int segs;              // fp16: segments per row
 };
 
-// NH halo boxes, NP loaded plain boxes, NO output-only plain boxes, NST stages
-// V cells per thread: 4 (a compute warp takes two tile rows) or 2 (one row)
-template <int FDOH, int TY, int NH, int NP, int NO, int NST, int BCAP = 3, int V = 4>
+// The shared-memory ring of an op: NH halo planes and NP plain planes a stage,
+// NST stages; V cells per thread: 4 (a compute warp takes two tile rows) or 2
+// (one row); BCAP resident blocks per SM that the launch bounds aim for.
+template <int FDOH, int TY, int NH, int NP, int NST, int BCAP = 3, int V = 4>
 struct Pipe {
     static constexpr int ROWS = V / 2;                // tile rows of a compute warp
     static constexpr int NCW = TY / ROWS;             // compute warps; the block adds one producer warp
@@ -135,12 +132,12 @@ struct Pipe {
     static constexpr int BOXS = BW * BH;                        // a plane of the halo box
     static constexpr int HALO = (NH * BOXS + 31) / 32 * 32;     // the halo box, 128-byte aligned
     static constexpr int PLS = TX * TY;
-    static constexpr int NHALO = NH, NLOAD = NP, NPL = NP + NO, STAGES = NST;
-    static constexpr int STAGE = HALO + NPL * PLS;
+    static constexpr int STAGES = NST;
+    static constexpr int STAGE = HALO + NP * PLS;
     static constexpr int TILE_Y = TY;
     static constexpr uint32_t TXB = (uint32_t)((NH * BW * BH + NP * PLS) * 4);
     static constexpr size_t bytes() { return (size_t)NST * STAGE * 4; }
-    static constexpr int BLOCK_CAP = BCAP;  // resident blocks per SM the launch bounds aim for
+    static constexpr int BLOCK_CAP = BCAP;
     static_assert((V == 4 || V == 2) && TY % ROWS == 0 && NCW <= 8, "tile rows and compute warps");
 };
 
@@ -492,12 +489,12 @@ __device__ __forceinline__ void run_pipeline(const KGrid &g, const KMaps &mp, co
 }
 
 // ---------------------------------------------------------------------------
-// A thread owns four adjacent cells of one row (16-byte shared-memory reads
-// and global stores): 16 lanes cover a tile row, a warp two rows.  Against a
-// column pair per thread this halves the loads, the address arithmetic and
-// the per-row bookkeeping of a cell; the stencils were bound by instruction
-// issue, not by HBM (400 x 160, 64 shots, FDORDER 4: 263 instructions a cell
-// in the velocity update with DRAM at 25 % of its peak).
+// A thread owns V = 4 adjacent cells of one row (16-byte shared-memory reads
+// and global stores): 16 lanes cover a tile row, a warp two rows; or 2, and a
+// warp one row (kCells).  Against two cells, four halve the loads, the address
+// arithmetic and the per-row bookkeeping of a cell; the stencils were bound by
+// instruction issue, not by HBM (400 x 160, 64 shots, FDORDER 4: 263
+// instructions a cell in the velocity update with DRAM at 25 % of its peak).
 
 // FD weights of one launch
 template <int FDOH>
@@ -547,7 +544,7 @@ __device__ __forceinline__ void stv(float *p, const float (&v)[V]) {
     else *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
 }
 
-// Difference stencils of a thread's four cells.  The m=1 term starts each sum
+// Difference stencils of a thread's cells.  The m=1 term starts each sum
 // and the others are added in order, as in the reference's written-out
 // expressions (src/update_v_PML.c:164-175); Z0: the sum is accumulated from
 // zero, as in its generic loops (the FDORDER 10/12 default branches, e.g.
@@ -626,7 +623,7 @@ __device__ __forceinline__ void ydiff_fs(const Hc<FDOH> &hc, const float *t, int
 }
 
 // A thread's place in its tile: row jj, staged column c0, cell (j, i) of its
-// first column, and the number of its cells inside the grid (nv; 4 on tiles
+// first column, and the number of its cells inside the grid (nv; V on tiles
 // that are not EDGE).
 struct Lane {
     int jj, c, i, j, nv;
@@ -643,7 +640,7 @@ struct Lane {
 };
 
 // CPML of the thread's cells (src/update_v_PML.c:177-226).  The strip rows are
-// laid out so that a group of four cells is one aligned 16-byte access
+// laid out so that a thread's group of cells is one aligned access
 // (KGrid::psx, psy); cells of the group outside the strip have zero factors
 // and keep their difference.  The memory values are loaded before the wait
 // for the stage (Op::prefetch) and used after the differences.
@@ -1093,7 +1090,7 @@ struct OpSVisc {
     static constexpr int DEP_TILES = INT_MAX;
     static constexpr int NH_ = 2, NP_ = 3 + 3 * LL + (DIRECT ? 0 : 6);
     static constexpr bool CPML = !QUIRK, MIRROR = false;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, visc_blocks(LL), V>;
+    using P = Pipe<FDOH, TY, NH_, NP_, NST, visc_blocks(LL), V>;
     IFOS_OP_MEMBERS
     // boxes of consecutive planes: their number, planes of box k, whether they are model planes
     static constexpr int NG = DIRECT ? 2 : 3;
@@ -1275,7 +1272,7 @@ struct OpSEl {
     static constexpr int DEP_TILES = FDOH <= 2 ? kDepTiles : INT_MAX;
     static constexpr int NH_ = 2, NP_ = 6;
     static constexpr bool CPML = !QUIRK, MIRROR = false;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, SMALL ? 2 : sblocks(FDOH), V>;
+    using P = Pipe<FDOH, TY, NH_, NP_, NST, SMALL ? 2 : sblocks(FDOH), V>;
     IFOS_OP_MEMBERS
     // boxes of consecutive planes: their number, planes of box k, whether they are model planes
     static constexpr int NG = QUIRK ? 4 : 2;
@@ -1401,7 +1398,7 @@ struct OpVPsv {
     static constexpr int NH_ = AC ? 1 : 3;
     static constexpr int NP_ = (SW == 1 && !QUIRK) ? 6 : 4;
     static constexpr bool CPML = !QUIRK, MIRROR = true;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, SMALL ? 2 : vblocks(FDOH), V>;
+    using P = Pipe<FDOH, TY, NH_, NP_, NST, SMALL ? 2 : vblocks(FDOH), V>;
     IFOS_OP_MEMBERS
     // boxes of consecutive planes: their number, planes of box k, whether they are model planes
     static constexpr int NG = NP_ / 2;
@@ -1560,7 +1557,7 @@ struct OpVSh {
     static constexpr int DEP_TILES = INT_MAX;
     static constexpr int NH_ = 2, NP_ = 2;
     static constexpr bool CPML = true, MIRROR = true;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, vblocks(FDOH), V>;
+    using P = Pipe<FDOH, TY, NH_, NP_, NST, vblocks(FDOH), V>;
     IFOS_OP_MEMBERS
     // boxes of consecutive planes: their number, planes of box k, whether they are model planes
     static constexpr int NG = 2;
@@ -1645,7 +1642,7 @@ struct OpSSh {
     static constexpr int DEP_TILES = INT_MAX;
     static constexpr int NH_ = 1, NP_ = LL ? 2 + 2 * LL + 4 : 4, L1 = LL > 0 ? LL : 1;
     static constexpr bool CPML = true, MIRROR = false;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, LL ? 3 : sblocks(FDOH), V>;
+    using P = Pipe<FDOH, TY, NH_, NP_, NST, LL ? 3 : sblocks(FDOH), V>;
     IFOS_OP_MEMBERS
     // boxes of consecutive planes: their number, planes of box k, whether they are model planes
     static constexpr int NG = LL ? 5 : 2;
@@ -1771,7 +1768,7 @@ struct OpPAc {
     static constexpr int DEP_TILES = INT_MAX;
     static constexpr int NH_ = 2, NP_ = 2;
     static constexpr bool CPML = !QUIRK, MIRROR = false;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, sblocks(FDOH), V>;
+    using P = Pipe<FDOH, TY, NH_, NP_, NST, sblocks(FDOH), V>;
     IFOS_OP_MEMBERS
     // boxes of consecutive planes: their number, planes of box k, whether they are model planes
     static constexpr int NG = 2;
@@ -1860,7 +1857,7 @@ struct OpPVisc {
     static constexpr int DEP_TILES = INT_MAX;
     static constexpr bool Z0 = FDOH != 1, CPML = !Z0, MIRROR = false;
     static constexpr int NH_ = 2, NP_ = 3 + LL;
-    using P = Pipe<FDOH, TY, NH_, NP_, 0, NST, 3, V>;
+    using P = Pipe<FDOH, TY, NH_, NP_, NST, 3, V>;
     IFOS_OP_MEMBERS
     // boxes of consecutive planes: their number, planes of box k, whether they are model planes
     static constexpr int NG = 3;
