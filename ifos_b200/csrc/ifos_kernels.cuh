@@ -644,8 +644,6 @@ struct KSrc {
     const float *sig;    // slot * max_src * NT
     const int *nsrc;     // per slot
     int max_src, nt_total;
-    const unsigned char *rows;  // per slot row_bytes bytes: bit r of byte b is set when row 8 b + r + 1 holds a source
-    int row_bytes;
 };
 struct KRec {
     const int *pos;      // slot * 2 * max_rec
@@ -657,10 +655,12 @@ struct KRec {
     // receivers in place: per slot map_stride ints, first NY row entries
     // (-1: no receiver in the row, else the row's index among the slot's
     // receiver rows), then kRecMapRows rows of NX cell entries (-1 or the index of
-    // the receiver in the cell)
+    // the receiver in the cell), then two row tables of row_bytes bytes, of the
+    // slot's receivers and of its sources: bit r of byte b is set when row 8 b + r
+    // + 1 holds one
     const int *map;
     long long map_stride;
-    const unsigned char *rows;  // rows that hold receivers, as KSrc::rows
+    const unsigned char *rows;  // the row tables of slot 0
     int row_bytes;
 };
 

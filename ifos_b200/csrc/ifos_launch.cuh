@@ -67,6 +67,10 @@ static constexpr int kPipeMaxL = 5;
 // receiver rows a slot's cell map holds: slots whose receivers lie on more
 // rows are sampled and injected by the separate receiver kernels
 constexpr int kRecMapRows = 8;
+// ints of a slot's receiver map (KRec::map)
+inline long long rec_map_stride(const ifos_params &p) {
+    return (long long)p.ny + (long long)kRecMapRows * p.nx + (2 * ((p.ny + 7) / 8) + 3) / 4;
+}
 
 struct DevBuf {
     void *p = nullptr;
@@ -106,7 +110,7 @@ struct ifos_ctx {
     KGrid g{};
     int psv = 0, sh = 0, ac = 0;
     // state
-    DevBuf state, psi, models, prof, srf, slot_model, src_pos, src_sig, src_n, rec_pos, rec_n, rec_map, src_rows, rec_rows, adj, sec,
+    DevBuf state, psi, models, prof, srf, slot_model, src_pos, src_sig, src_n, rec_pos, rec_n, rec_map, adj, sec,
         snap, snap_scale, gacc, gacc64, gout, bad, dot_partial, dot_out, res_tr;
     long long proftab_off = 0;  // elements from prof to the table the stencil blocks stage (0: none)
     long long profx_off = 0;  // elements from prof to the x profiles by grid column
@@ -201,8 +205,6 @@ inline KSrc ksrc(const ifos_ctx *c) {
     s.pos = (const float *)c->src_pos.p;
     s.sig = (const float *)c->src_sig.p;
     s.nsrc = (const int *)c->src_n.p;
-    s.rows = (const unsigned char *)c->src_rows.p;
-    s.row_bytes = (c->p.ny + 7) / 8;
     s.max_src = std::max(1, c->p.max_src);
     s.nt_total = c->p.nt;
     return s;
@@ -214,10 +216,10 @@ inline KRec krec(const ifos_ctx *c) {
     r.max_rec = std::max(1, c->p.max_rec);
     r.adj = (const float *)c->adj.p;
     r.sec = (float *)c->sec.p;
-    r.rows = (const unsigned char *)c->rec_rows.p;
-    r.row_bytes = (c->p.ny + 7) / 8;
     r.map = (const int *)c->rec_map.p;
-    r.map_stride = (long long)c->p.ny + (long long)kRecMapRows * c->p.nx;
+    r.rows = (const unsigned char *)(r.map + c->p.ny + (long long)kRecMapRows * c->p.nx);
+    r.row_bytes = (c->p.ny + 7) / 8;
+    r.map_stride = rec_map_stride(c->p);
     return r;
 }
 inline KSnap ksnap(const ifos_ctx *c) {

@@ -238,7 +238,7 @@ extern "C" int ifos_ctx_destroy(ifos_ctx *c) {
     if (c->st) cudaStreamSynchronize(c->st);
     if (c->cp_st) cudaStreamSynchronize(c->cp_st);  // asynchronous fetches still reading the buffers
     DevBuf *bufs[] = {&c->state, &c->psi, &c->models, &c->prof, &c->srf, &c->slot_model, &c->src_pos, &c->src_sig,
-                      &c->src_n, &c->rec_pos, &c->rec_n, &c->rec_map, &c->src_rows, &c->rec_rows, &c->adj, &c->sec, &c->snap, &c->snap_scale,
+                      &c->src_n, &c->rec_pos, &c->rec_n, &c->rec_map, &c->adj, &c->sec, &c->snap, &c->snap_scale,
                       &c->gacc, &c->gacc64, &c->gout, &c->bad, &c->dot_partial, &c->dot_out, &c->res_tr};
     for (DevBuf *b : bufs) dev_free(*b);
     for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
@@ -471,13 +471,8 @@ extern "C" int ifos_ctx_create(const ifos_params *pp, int device, int with_snaps
     if ((rc = dev_alloc(c, c->src_n, (size_t)S * sizeof(int)))) return bail(rc);
     if ((rc = dev_alloc(c, c->rec_pos, (size_t)S * 2 * mr * 4))) return bail(rc);
     if ((rc = dev_alloc(c, c->rec_n, (size_t)S * sizeof(int)))) return bail(rc);
-    if ((rc = dev_alloc(c, c->rec_map, (size_t)S * ((size_t)p.ny + (size_t)kRecMapRows * p.nx) * sizeof(int))))
+    if ((rc = dev_alloc(c, c->rec_map, (size_t)S * rec_map_stride(p) * sizeof(int))))
         return bail(rc);
-    for (DevBuf *b : {&c->src_rows, &c->rec_rows}) {
-        if ((rc = dev_alloc(c, *b, (size_t)S * ((p.ny + 7) / 8)))) return bail(rc);
-        if (cudaMemsetAsync(b->p, 0, b->bytes, c->st) != cudaSuccess)
-            return bail(fail(c, IFOS_ERR_CUDA, "row table clear failed"));
-    }
     if (cudaMemsetAsync(c->rec_map.p, 0xff, c->rec_map.bytes, c->st) != cudaSuccess)  // -1: no receiver
         return bail(fail(c, IFOS_ERR_CUDA, "receiver map clear failed"));
     if ((rc = dev_alloc(c, c->adj, (size_t)S * 3 * mr * p.nt * 4))) return bail(rc);
@@ -717,7 +712,7 @@ extern "C" int ifos_shot_setup(ifos_ctx *c, int slot, int model, int nsrc, const
     CK(cudaMemcpyAsync((char *)c->rec_pos.p + (size_t)slot * 2 * mr * 4, rp.data(), rp.size() * 4,
                        cudaMemcpyHostToDevice, c->st));
     // the slot's cell -> receiver map for the in-stencil sampling and injection
-    const size_t mstride = (size_t)p.ny + (size_t)kRecMapRows * p.nx;
+    const size_t mstride = (size_t)rec_map_stride(p);
     std::vector<int> rm(mstride, -1);
     int lo = p.ny + 1, hi = 0, nrows = 0;
     bool mapped = true;
@@ -734,21 +729,17 @@ extern "C" int ifos_shot_setup(ifos_ctx *c, int slot, int model, int nsrc, const
         }
         rm[(size_t)p.ny + (size_t)rm[j - 1] * p.nx + (i - 1)] = l;
     }
-    CK(cudaMemcpyAsync((char *)c->rec_map.p + (size_t)slot * mstride * 4, rm.data(), rm.size() * 4,
-                       cudaMemcpyHostToDevice, c->st));
-    // the rows that hold the slot's sources and receivers
-    const size_t nb = ((size_t)p.ny + 7) / 8;
-    std::vector<unsigned char> srows(nb, 0), rrows(nb, 0);
+    // the row tables behind it
+    const size_t nb = ((size_t)p.ny + 7) / 8, maps = (size_t)p.ny + (size_t)kRecMapRows * p.nx;
+    std::fill(rm.begin() + maps, rm.end(), 0);
+    unsigned char *rrows = reinterpret_cast<unsigned char *>(rm.data() + maps), *srows = rrows + nb;
+    for (int l = 0; l < ntr; l++) rrows[(recpos[ntr + l] - 1) / 8] |= (unsigned char)(1 << (recpos[ntr + l] - 1) % 8);
     for (int l = 0; l < nsrc; l++) {
         const int j = (int)srcpos[nsrc + l];
         srows[(j - 1) / 8] |= (unsigned char)(1 << (j - 1) % 8);
     }
-    for (int l = 0; l < ntr; l++) {
-        const int j = recpos[ntr + l];
-        rrows[(j - 1) / 8] |= (unsigned char)(1 << (j - 1) % 8);
-    }
-    CK(cudaMemcpyAsync((char *)c->src_rows.p + (size_t)slot * nb, srows.data(), nb, cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync((char *)c->rec_rows.p + (size_t)slot * nb, rrows.data(), nb, cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync((char *)c->rec_map.p + (size_t)slot * mstride * 4, rm.data(), rm.size() * 4,
+                       cudaMemcpyHostToDevice, c->st));
     c->rec_mapped[slot] = mapped;
     c->rec_row_lo[slot] = lo;
     c->rec_row_hi[slot] = hi;

@@ -201,15 +201,15 @@ struct TileWalk {
     int px0, px1, top;
     int lo[NR], hi[NR];
     // The receiver and source ranges span all slots.  Where one holds more than
-    // one row, the slot's own rows are looked up (KRec::rows, KSrc::rows; NULL:
-    // the range says it all), so that shots at several depths, or receivers in
+    // one row, the slot's own rows are looked up (KRec::rows; NULL: the range says
+    // it all), so that shots at several depths, or receivers in
     // a shallow and a deep row, do not put all rows between on the longer path.
     // A forward step with the ranges alone, with the lookup, and with one row
     // (us): six viscoelastic shots of 2000 x 600 at six depths 261, 217 and 215;
     // four acoustic shots of 1500 x 500 at four depths 47.2, 34.9 and 32.2; a
     // P-SV shot of 4000 x 1200 with two receiver rows 88.5, 73.9 and 71.9.
     const unsigned char *own[2];
-    int own_stride;
+    long long own_stride;
     // TMA z coordinates: planes of a slot and of a model, the halo box's first plane, the groups'
     int slot_planes, model_planes, zh, zg[kMaxGroups];
 
@@ -252,8 +252,8 @@ struct TileWalk {
         range(R_SRC, op.fps || op.fvs, op.src_j0, op.src_j1);
         static_assert(TY == 8, "a tile's rows are one byte of the row tables");
         w.own[0] = w.hi[R_REC] > w.lo[R_REC] ? op.rec.rows : nullptr;
-        w.own[1] = w.hi[R_SRC] > w.lo[R_SRC] ? op.src.rows : nullptr;
-        w.own_stride = op.rec.row_bytes;
+        w.own[1] = w.hi[R_SRC] > w.lo[R_SRC] ? op.rec.rows + op.rec.row_bytes : nullptr;
+        w.own_stride = op.rec.map_stride * 4;
 
         int z[Op::NG];
         op.planes(w.zh, z);
@@ -280,15 +280,17 @@ struct TileWalk {
         tx = cl + c;
         return rt + r;
     }
-    // Tile t of the launch: slot, first cell, and the bits of the compute warps
-    // of ROWS rows each that need more than the plain update
+    // Tile t of the launch: slot, first cell, the slot's model (models NULL: 0),
+    // and the bits of the compute warps of ROWS rows each that need more than the
+    // plain update
     template <int TY, int ROWS>
-    __device__ __forceinline__ TileInfo tile(int t) const {
+    __device__ __forceinline__ TileInfo tile(int t, const int *models) const {
         TileInfo r;
         int rem, tx;
         if (nshots == 1) r.slot = 0, rem = t;
         else if (minor) rem = div_small(t, nshots, r_shots, r.slot);
         else r.slot = div_small(t, per, r_per, rem);
+        const int model = models ? models[r.slot] : 0;  // requested before the rest is worked out
         const int ty = cpml ? first(rem, tx) : div_small(rem, ntx, r_ntx, tx);
         r.i0 = tx * kTileX + 1;
         r.j0 = ty * TY + 1;
@@ -298,9 +300,9 @@ struct TileWalk {
             const int a = max(lo[k] - r.j0, 0), b = min(hi[k] - r.j0, TY - 1);
             if (a > b) continue;
             const unsigned char *p = k >= R_REC ? own[k - R_REC] : nullptr;
-            rows |= p ? p[(long long)r.slot * own_stride + ty] : (2u << b) - (1u << a);
+            rows |= p ? p[r.slot * own_stride + ty] : (2u << b) - (1u << a);
         }
-        r.bits = warps_of_rows<ROWS>(rows);
+        r.bits = model * 256 + warps_of_rows<ROWS>(rows);
         return r;
     }
     // bit w: one of the rows of compute warp w
@@ -375,9 +377,7 @@ __device__ __forceinline__ void run_pipeline(const KGrid &g, const KMaps &mp, co
         auto fill = [&](int k0) {
             const int k = k0 + lane, t = blockIdx.x + k * gridDim.x;
             if (t < ntiles) {
-                TileInfo ti = walk.tile<TY, P::ROWS>(t);
-                if (!op.M.one_model) ti.bits += op.M.slot_model[ti.slot] * 256;
-                tq[k % (2 * kTileBatch)] = ti;
+                tq[k % (2 * kTileBatch)] = walk.tile<TY, P::ROWS>(t, op.M.one_model ? nullptr : op.M.slot_model);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&filled);
