@@ -208,6 +208,9 @@ struct TileWalk {
     // (us): six viscoelastic shots of 2000 x 600 at six depths 261, 217 and 215;
     // four acoustic shots of 1500 x 500 at four depths 47.2, 34.9 and 32.2; a
     // P-SV shot of 4000 x 1200 with two receiver rows 88.5, 73.9 and 71.9.
+    // The lookup is out of line: a block works out its first tiles in code that
+    // comes cold from the instruction cache, and this part is rarely needed.
+    int lookup;
     const unsigned char *own[2];
     long long own_stride;
     // TMA z coordinates: planes of a slot and of a model, the halo box's first plane, the groups'
@@ -254,6 +257,7 @@ struct TileWalk {
         w.own[0] = w.hi[R_REC] > w.lo[R_REC] ? op.rec.rows : nullptr;
         w.own[1] = w.hi[R_SRC] > w.lo[R_SRC] ? op.rec.rows + op.rec.row_bytes : nullptr;
         w.own_stride = op.rec.map_stride * 4;
+        w.lookup = w.own[0] || w.own[1];
 
         int z[Op::NG];
         op.planes(w.zh, z);
@@ -296,14 +300,31 @@ struct TileWalk {
         r.j0 = ty * TY + 1;
         unsigned rows = tx < px0 || tx >= px1 || (top && ty == 0) ? (1u << TY) - 1 : 0u;
 #pragma unroll
-        for (int k = 0; k < NR; k++) {
-            const int a = max(lo[k] - r.j0, 0), b = min(hi[k] - r.j0, TY - 1);
-            if (a > b) continue;
-            const unsigned char *p = k >= R_REC ? own[k - R_REC] : nullptr;
-            rows |= p ? p[r.slot * own_stride + ty] : (2u << b) - (1u << a);
+        for (int k = 0; k < R_REC; k++) rows |= range<TY>(k, r.j0);
+        if (lookup) {
+            rows |= own_rows<TY>(r.slot, ty, r.j0);
+        } else {
+            rows |= range<TY>(R_REC, r.j0) | range<TY>(R_SRC, r.j0);
         }
         r.bits = model * 256 + warps_of_rows<ROWS>(rows);
         return r;
+    }
+    // rows of range k in the tile that starts at row j0
+    template <int TY>
+    __device__ __forceinline__ unsigned range(int k, int j0) const {
+        const int a = max(lo[k] - j0, 0), b = min(hi[k] - j0, TY - 1);
+        return a <= b ? (2u << b) - (1u << a) : 0u;
+    }
+    // the slot's receiver and source rows in tile row ty
+    template <int TY>
+    __device__ __noinline__ unsigned own_rows(int slot, int ty, int j0) const {
+        unsigned m = 0;
+        for (int k = R_REC; k <= R_SRC; k++) {
+            const unsigned r = range<TY>(k, j0);
+            const unsigned char *p = own[k - R_REC];
+            if (r) m |= p ? p[slot * own_stride + ty] : r;
+        }
+        return m;
     }
     // bit w: one of the rows of compute warp w
     template <int ROWS>
